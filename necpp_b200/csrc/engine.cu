@@ -2798,9 +2798,8 @@ int necgpu_set_sommerfeld(necgpu_engine* e, double eps_re, double eps_im) {
   CUDA_TRY(cudaSetDevice(e->device));
   if (!e->d_somm) TRY(dalloc(e, e->d_somm, (size_t)kSommPoints));
   CUDA_TRY(cudaMemsetAsync(e->d_status, 0, 4 * sizeof(int), e->stream));
-  const unsigned blocks = (unsigned)((kSommEvalPoints + 31) / 32);
   KLAUNCH(NECGPU_K_FILL, 0.0,
-          somm_table_kernel<<<blocks, 32, 0, e->stream>>>(mk(eps_re, eps_im), e->P.eta, e->d_somm, e->d_status));
+          somm_table_kernel<<<kSommEvalPoints + 1, kSommThreads, 0, e->stream>>>(mk(eps_re, eps_im), e->P.eta, e->d_somm, e->d_status));
   int st = 0;
   TRY(sync_status(e, &st));
   if (st & kStatIterCap) return fail(e, NECGPU_ERR_NONFINITE, "set_sommerfeld: a Sommerfeld integral did not converge");

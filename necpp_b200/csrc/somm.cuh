@@ -12,7 +12,8 @@
 // elevation: 11 x 10 points from R = 0 in steps of 0.02 wavelength, 17 x 5
 // and 9 x 8 points from R = 0.2 (theta below / above 20 degrees); four
 // functions per point (erv, ezv, erh, eph), scaled by the image spherical
-// wave.  One thread evaluates the Sommerfeld integrals of one grid point.
+// wave.  One CTA evaluates the Sommerfeld integrals of one grid point
+// (somm_table_kernel).
 //
 // The interpolation keeps the reference's cache: the last 4 x 4 patch and
 // its cell, reused for a point that lies below the start of the patch's
@@ -52,12 +53,22 @@ struct BesselTables {
   double bes_a1[25], bes_a2[25], han_a1[25], han_a2[25], han_a3[25], han_a4[25];
 };
 
+// (all threads of the CTA, ends with a barrier)
 __device__ void build_bessel_tables(BesselTables& t) {
-  for (int k = 1; k <= 25; k++) {
-    t.bes_a1[k - 1] = -0.25 / (k * k);
-    t.bes_a2[k - 1] = 1.0 / (k + 1.0);
+  const int tid = threadIdx.x;
+  if (tid < 25) {
+    const int k = tid + 1;
+    double psi = -.5772156649;
+    for (int q = 1; q <= k; q++) psi += 1.0 / q;
+    t.bes_a1[tid] = -0.25 / (k * k);
+    t.bes_a2[tid] = 1.0 / (k + 1.0);
+    t.han_a1[tid] = -.25 / (k * k);
+    t.han_a2[tid] = 1.0 / (k + 1.0);
+    t.han_a3[tid] = psi + psi;
+    t.han_a4[tid] = (psi + psi + 1.0 / (k + 1.0)) / (k + 1.0);
   }
-  for (int i = 1; i <= 101; i++) {
+  __syncthreads();
+  for (int i = tid + 1; i <= 101; i += blockDim.x) {
     double tst = 1.0;
     int init = 0;
     for (int k = 0; k < 24; k++) {
@@ -66,19 +77,8 @@ __device__ void build_bessel_tables(BesselTables& t) {
       if (tst < 1.0e-6) break;
     }
     t.bes_m[i - 1] = init + 1;
-  }
-  double psi = -.5772156649;
-  for (int k = 1; k <= 25; k++) {
-    int i = k - 1;
-    t.han_a1[i] = -.25 / (k * k);
-    t.han_a2[i] = 1.0 / (k + 1.0);
-    psi += 1.0 / k;
-    t.han_a3[i] = psi + psi;
-    t.han_a4[i] = (psi + psi + 1.0 / (k + 1.0)) / (k + 1.0);
-  }
-  for (int i = 1; i <= 101; i++) {
     double tt = 1.0;
-    int init = 0;
+    init = 0;
     for (int k = 0; k < 24; k++) {
       init = k;
       tt *= -i * t.han_a1[k];
@@ -86,6 +86,7 @@ __device__ void build_bessel_tables(BesselTables& t) {
     }
     t.han_m[i - 1] = init + 1;
   }
+  __syncthreads();
 }
 
 // asymptotic-series constants, c_evlcom.cpp:627-637
@@ -181,24 +182,36 @@ __device__ bool hankel_h0(const BesselTables& T, cplx z, cplx* h0, cplx* h0p) {
   return true;
 }
 
-// State of the contour integration of one grid point (c_evlcom members).
+// Constants of the contour integration of one grid point (c_evlcom members).
 struct Evl {
   double ck2, ck2sq, tkmag, tsmag, ck1r, zph, rho;
   cplx ct1, ct2, ct3, ck1, ck1sq, cksm;
-  cplx a, b;  // contour segment
-  bool bessel_form;
-  int fail;
 };
 
 constexpr int kSommNM = 131072, kSommMaxH = 20;
 constexpr double kSommCrit = 1.0E-4, kSommPTP = .6283185308;
+constexpr int kSommWarps = 8;         // contour intervals in flight per grid point
+constexpr int kSommWin = 32;          // cells of an interval's window of evaluated points
+constexpr int kSommThreads = 32 * kSommWarps;
 
-// integrands of the six Sommerfeld integrals at contour parameter t
-__device__ void saoa(const BesselTables& T, Evl& E, double t, cplx ans[6]) {
-  cplx dxl = E.b - E.a;
-  cplx xl = E.a + dxl * t;
+// Work area of the CTA of one grid point.
+struct SommShared {
+  BesselTables T;
+  Evl E;
+  cplx vals[kSommWarps][kSommWin + 1][6];  // the warps' windows of integrand values
+  cplx ival[kSommWarps][6];                // the warps' interval integrals
+  cplx q1[6][kSommMaxH], q2[6][kSommMaxH];
+  cplx sum[6], ans[6];
+  int done, fail;
+};
+
+// integrands of the six Sommerfeld integrals at parameter t of the contour
+// segment from a along dxl
+__device__ bool saoa(const BesselTables& T, const Evl& E, bool bessel_form, cplx a, cplx dxl, double t, cplx* ans) {
+  cplx xl = a + dxl * t;
   cplx b0 = mk(0, 0), b0p = mk(0, 0), cgam1, cgam2, com, dgam;
-  if (E.bessel_form) {
+  bool ok = true;
+  if (bessel_form) {
     bessel_j0(T, xl * E.rho, &b0, &b0p);
     b0 = b0 * 2.;
     b0p = b0p * 2.;
@@ -207,7 +220,7 @@ __device__ void saoa(const BesselTables& T, Evl& E, double t, cplx ans[6]) {
     if (cgam1.re == 0.0) cgam1 = mk(0.0, -fabs(cgam1.im));
     if (cgam2.re == 0.) cgam2 = mk(0.0, -fabs(cgam2.im));
   } else {
-    if (!hankel_h0(T, xl * E.rho, &b0, &b0p)) E.fail = 1;
+    ok = hankel_h0(T, xl * E.rho, &b0, &b0p);
     com = xl - E.ck1;
     cgam1 = csqrt_(xl + E.ck1) * csqrt_(com);
     if (com.re < 0. && com.im >= 0.) cgam1 = -cgam1;
@@ -238,227 +251,283 @@ __device__ void saoa(const BesselTables& T, Evl& E, double t, cplx ans[6]) {
   com = dxl * xl * cexp_(-cgam2 * E.zph);
   ans[5] = com * b0 * den1 / E.ck1;
   com = com * den2;
+  cplx a0, a3;
   if (E.rho != 0.) {
     b0p = b0p / E.rho;
-    ans[0] = -com * xl * (b0p + b0 * xl);
-    ans[3] = com * xl * b0p;
+    a0 = -com * xl * (b0p + b0 * xl);
+    a3 = com * xl * b0p;
   } else {
-    ans[0] = -com * xl * xl * .5;
-    ans[3] = ans[0];
+    a0 = -com * xl * xl * .5;
+    a3 = a0;
   }
+  ans[0] = a0;
+  ans[3] = a3;
   ans[1] = com * cgam2 * cgam2 * b0;
-  ans[2] = -ans[3] * cgam2 * E.rho;
+  ans[2] = -a3 * cgam2 * E.rho;
   ans[4] = com * b0;
+  return ok;
 }
 
-// variable-interval Romberg integration of the six integrands over [a, b]
-__device__ void rom1(const BesselTables& T, Evl& E, cplx sum[6], int nx) {
+// Variable-interval Romberg integration of the six integrands over the
+// contour segment [a, b] by one warp: the reference's decision sequence, the
+// six integrals on lanes 0-5 (the other lanes copy lane 5).  Every point the
+// sequence can ask for is a dyadic fraction of the interval, so the lanes
+// evaluate a window of points at once (cells 0..30 and 32 of `h` each from
+// z0; the first window spans the interval at 1/32, enough for steps down to
+// 1/8) and the sequence reads them; a step that needs a point outside the
+// window opens a finer one at its own start.  A serial evaluation spends one
+// integrand latency (several microseconds of dependent FP64) per point, this
+// one per window.
+__device__ void rom1_warp(SommShared& S, bool bessel_form, cplx a, cplx b, int nx) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int c = lane < 5 ? lane : 5;
+  cplx(*vals)[6] = S.vals[w];
+  const cplx dxl = b - a;
   const double s = 1.0, ze = 1.0, ep = s / (1.0e4 * kSommNM), zend = ze - ep;
   double z = 0.0, dz = 0.0, dzot = 0.0, tr, ti;
-  cplx g1[6], g2[6], g3[6], g4[6], g5[6], t01[6], t10[6], t20[6];
-  for (int i = 0; i < 6; i++) sum[i] = mk(0, 0);
+  double z0 = 0.0, h = 1.0 / kSommWin;
+  cplx sum = mk(0, 0), g1, g2, g3, g4, g5;
   int ns = nx, nt = 0;
-  saoa(T, E, z, g1);
-  bool jump = false;
-  for (int guard = 0; guard < (1 << 20); guard++) {
+  bool ok = true;
+  auto evaluate = [&]() {
+    const int k = lane < kSommWin - 1 ? lane : kSommWin;
+    const double t = z0 + k * h;
+    __syncwarp();
+    if (t <= ze) ok = saoa(S.T, S.E, bessel_form, a, dxl, t, vals[k]) && ok;
+    __syncwarp();
+  };
+  // cell of point t, or -1 when the window does not hold it (every t, z0
+  // and h is a dyadic fraction: the quotient is exact when it is whole)
+  auto cell = [&](double t) {
+    const double q = (t - z0) / h;
+    return q >= 0.0 && q <= kSommWin && q == floor(q) && q != kSommWin - 1 ? (int)q : -1;
+  };
+  auto have = [&](double t) { return cell(t) >= 0; };
+  auto open = [&]() {
+    z0 = z;
+    h = dz / 8.0;
+    evaluate();
+  };
+  auto at = [&](double t) { return vals[cell(t)][c]; };
+  evaluate();
+  g1 = at(0.0);
+  g3 = g5 = g1;
+  bool jump = false, finished = false;
+  for (int guard = 0; guard < (1 << 20) && !finished; guard++) {
     if (!jump) {
       dz = s / ns;
       if ((z + dz) > ze) {
         dz = ze - z;
-        if (dz <= ep) return;
+        if (dz <= ep) {
+          finished = true;
+          continue;
+        }
       }
       dzot = dz * .5;
-      saoa(T, E, z + dzot, g3);
-      saoa(T, E, z + dz, g5);
+      if (!have(z + dzot) || !have(z + dz)) open();
+      g3 = at(z + dzot);
+      g5 = at(z + dz);
     }
-    bool nogo = false;
-    for (int i = 0; i < 6; i++) {
-      cplx t00 = (g1[i] + g5[i]) * dzot;
-      t01[i] = (t00 + dz * g3[i]) * .5;
-      t10[i] = (4. * t01[i] - t00) / 3.;
-      conv_test(t01[i].re, t10[i].re, &tr, t01[i].im, t10[i].im, &ti);
-      if ((tr > kSommCrit) || (ti > kSommCrit)) nogo = true;
-    }
-    bool accept5 = false;
+    const cplx t00 = (g1 + g5) * dzot;
+    const cplx t01 = (t00 + dz * g3) * .5;
+    const cplx t10 = (4. * t01 - t00) / 3.;
+    conv_test(t01.re, t10.re, &tr, t01.im, t10.im, &ti);
+    bool nogo = __any_sync(0xffffffffu, (tr > kSommCrit) || (ti > kSommCrit));
     if (!nogo) {
-      for (int i = 0; i < 6; i++) sum[i] += t10[i];
+      sum += t10;
       nt += 2;
     } else {
-      saoa(T, E, z + dz * .25, g2);
-      saoa(T, E, z + dz * .75, g4);
-      nogo = false;
-      for (int i = 0; i < 6; i++) {
-        cplx t02 = (t01[i] + dzot * (g2[i] + g4[i])) * .5;
-        cplx t11 = (4. * t02 - t01[i]) / 3.;
-        t20[i] = (16. * t11 - t10[i]) / 15.;
-        conv_test(t11.re, t20[i].re, &tr, t11.im, t20[i].im, &ti);
-        if ((tr > kSommCrit) || (ti > kSommCrit)) nogo = true;
-      }
+      if (!have(z + dz * .25) || !have(z + dz * .75)) open();
+      g2 = at(z + dz * .25);
+      g4 = at(z + dz * .75);
+      const cplx t02 = (t01 + dzot * (g2 + g4)) * .5;
+      const cplx t11 = (4. * t02 - t01) / 3.;
+      const cplx t20 = (16. * t11 - t10) / 15.;
+      conv_test(t11.re, t20.re, &tr, t11.im, t20.im, &ti);
+      nogo = __any_sync(0xffffffffu, (tr > kSommCrit) || (ti > kSommCrit));
       if (nogo) {
         nt = 0;
         if (ns < kSommNM) {
           ns *= 2;
           dz = s / ns;
           dzot = dz * .5;
-          for (int i = 0; i < 6; i++) {
-            g5[i] = g3[i];
-            g3[i] = g2[i];
-          }
+          // as the reference: after a last step cut short at the end of the
+          // interval these are not the points of the halved step
+          g5 = g3;
+          g3 = g2;
           jump = true;
           continue;
         }
       }
-      accept5 = true;
-    }
-    if (accept5) {
-      for (int i = 0; i < 6; i++) sum[i] += t20[i];
+      sum += t20;
       nt++;
     }
     z += dz;
-    if (z > zend) return;
-    for (int i = 0; i < 6; i++) g1[i] = g5[i];
+    finished = z > zend;
+    g1 = g5;
     if ((nt >= 4) && (ns > nx)) {
       ns = ns / 2;
       nt = 1;
     }
     jump = false;
   }
-  E.fail = 1;
+  if (lane < 6) S.ival[w][lane] = sum;
+  if (!ok || !finished) S.fail = 1;
 }
 
-// integration from `start` to infinity with Shanks' transformation; at the
-// break point bk (when ibk != 0) the step changes from dela to delb
-__device__ void gshank(const BesselTables& T, Evl& E, cplx start, cplx dela, cplx sum[6], const cplx seed[6],
-                       int ibk, cplx bk, cplx delb) {
-  cplx q1[6][kSommMaxH], q2[6][kSommMaxH], ans1[6], ans2[6];
-  const double rbk = bk.re;
-  cplx del = dela;
-  int ibx = (ibk == 0) ? 1 : 0;
-  for (int i = 0; i < 6; i++) ans2[i] = seed[i];
-  E.b = start;
-  int restarts = 0;
-  for (int intx = 1; intx <= kSommMaxH; intx++) {
-    const int inx = intx - 1;
-    E.a = E.b;
-    E.b = E.b + del;
-    if ((ibx == 0) && (E.b.re >= rbk)) {
-      ibx = 1;
-      E.b = bk;
-      del = delb;
-      rom1(T, E, sum, 2);
-      for (int i = 0; i < 6; i++) ans2[i] += sum[i];
-      intx = 0;
-      if (++restarts > 2) break;
-      continue;
+// One Shanks step of gshank (warp 0; component c of lane): the new pair of
+// partial sums as1, as2 of iteration intx; true once all six have converged.
+__device__ bool shanks_step(SommShared& S, int c, cplx as1, cplx as2, int intx) {
+  for (int j = 1; j < intx; j++) {
+    const int jm = j - 1;
+    const cplx aa = S.q2[c][jm], q1 = S.q1[c][jm];
+    cplx a1 = q1 + as1 - 2. * aa;
+    if ((a1.re != 0.) || (a1.im != 0.)) {
+      cplx a2 = aa - q1;
+      a1 = q1 - a2 * a2 / a1;
+    } else {
+      a1 = q1;
     }
-    rom1(T, E, sum, 2);
-    for (int i = 0; i < 6; i++) ans1[i] = ans2[i] + sum[i];
-    E.a = E.b;
-    E.b = E.b + del;
-    if ((ibx == 0) && (E.b.re >= rbk)) {
-      ibx = 2;
-      E.b = bk;
-      del = delb;
-      rom1(T, E, sum, 2);
-      for (int i = 0; i < 6; i++) ans2[i] = ans1[i] + sum[i];
-      intx = 0;
-      if (++restarts > 2) break;
-      continue;
-    }
-    rom1(T, E, sum, 2);
-    for (int i = 0; i < 6; i++) ans2[i] = ans1[i] + sum[i];
-    double den = 0.;
-    for (int i = 0; i < 6; i++) {
-      cplx as1 = ans1[i], as2 = ans2[i];
-      for (int j = 1; j < intx; j++) {
-        const int jm = j - 1;
-        cplx aa = q2[i][jm];
-        cplx a1 = q1[i][jm] + as1 - 2. * aa;
-        if ((a1.re != 0.) || (a1.im != 0.)) {
-          cplx a2 = aa - q1[i][jm];
-          a1 = q1[i][jm] - a2 * a2 / a1;
-        } else {
-          a1 = q1[i][jm];
-        }
-        cplx a2 = aa + as2 - 2. * as1;
-        if ((a2.re != 0.) || (a2.im != 0.))
-          a2 = aa - (as1 - aa) * (as1 - aa) / a2;
-        else
-          a2 = aa;
-        q1[i][jm] = as1;
-        q2[i][jm] = as2;
-        as1 = a1;
-        as2 = a2;
-      }
-      q1[i][intx - 1] = as1;
-      q2[i][intx - 1] = as2;
-      double amg = fabs(as2.re) + fabs(as2.im);
-      if (amg > den) den = amg;
-    }
-    const double denm = 1.e-3 * den * kSommCrit;
-    int jm = intx - 3;
-    if (jm < 1) jm = 1;
-    bool brk = false;
-    for (int j = jm - 1; j < intx && !brk; j++) {
-      for (int i = 0; i < 6; i++) {
-        cplx a1 = q2[i][j];
-        double d = (fabs(a1.re) + fabs(a1.im)) * kSommCrit;
-        if (d < denm) d = denm;
-        a1 = q1[i][j] - a1;
-        if (fabs(a1.re) + fabs(a1.im) > d) {
-          brk = true;
-          break;
-        }
-      }
-    }
-    if (!brk) {
-      for (int i = 0; i < 6; i++) sum[i] = .5 * (q1[i][inx] + q2[i][inx]);
-      return;
-    }
+    cplx a2 = aa + as2 - 2. * as1;
+    if ((a2.re != 0.) || (a2.im != 0.))
+      a2 = aa - (as1 - aa) * (as1 - aa) / a2;
+    else
+      a2 = aa;
+    __syncwarp();
+    S.q1[c][jm] = as1;
+    S.q2[c][jm] = as2;
+    __syncwarp();
+    as1 = a1;
+    as2 = a2;
   }
-  E.fail = 1;
+  S.q1[c][intx - 1] = as1;
+  S.q2[c][intx - 1] = as2;
+  __syncwarp();
+  double den = fabs(as2.re) + fabs(as2.im);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) den = fmax(den, __shfl_xor_sync(0xffffffffu, den, off));
+  const double denm = 1.e-3 * den * kSommCrit;
+  int jm = intx - 3;
+  if (jm < 1) jm = 1;
+  bool brk = false;
+  for (int j = jm - 1; j < intx; j++) {
+    cplx a1 = S.q2[c][j];
+    double d = (fabs(a1.re) + fabs(a1.im)) * kSommCrit;
+    if (d < denm) d = denm;
+    a1 = S.q1[c][j] - a1;
+    brk = brk || fabs(a1.re) + fabs(a1.im) > d;
+  }
+  return !__any_sync(0xffffffffu, brk);
 }
 
-// The four field functions at the current (rho, zph): contour choice of evlua
-__device__ void evlua(const BesselTables& T, Evl& E, cplx* erv, cplx* ezv, cplx* erh, cplx* eph) {
-  cplx sum[6], ans[6];
+// Integration from `start` to infinity with Shanks' transformation; at the
+// break point bk (when ibk != 0) the step changes from dela to delb.  The
+// intervals follow from the geometry alone, so the CTA integrates the next
+// kSommWarps of them at once, a warp each, and warp 0 then takes them in
+// order through the transformation; intervals beyond the one that converged
+// are dropped.  seed -> sum (shared, six each; may be the same array).
+__device__ void gshank(SommShared& S, bool bessel_form, cplx start, cplx dela, cplx* sum, const cplx* seed, int ibk,
+                       cplx bk, cplx delb) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int c = lane < 5 ? lane : 5;
+  const double rbk = bk.re;
+  cplx del = dela, b = start;
+  int ibx = (ibk == 0) ? 1 : 0, half = 0;
+  cplx ans1 = mk(0, 0), ans2 = seed[c];
+  int intx = 1, restarts = 0;
+  // an iteration takes two intervals and there are at most three starts of
+  // at most kSommMaxH iterations
+  for (int round = 0; round < 2 * 3 * kSommMaxH / kSommWarps + 1; round++) {
+    cplx ma = b, mb = b;
+    unsigned kinds = 0;  // per interval: 0 / 1 first / second of an iteration, +2 when it ends at the break point
+    for (int k = 0; k < kSommWarps; k++) {
+      const cplx a = b;
+      b = b + del;
+      int kind = half;
+      if ((ibx == 0) && (b.re >= rbk)) {
+        ibx = half == 0 ? 1 : 2;
+        b = bk;
+        del = delb;
+        kind += 2;
+        half = 0;
+      } else {
+        half ^= 1;
+      }
+      kinds |= (unsigned)kind << (2 * k);
+      if (k == w) {
+        ma = a;
+        mb = b;
+      }
+    }
+    rom1_warp(S, bessel_form, ma, mb, 2);
+    __syncthreads();
+    if (w == 0) {
+      int done = 0;
+      for (int k = 0; k < kSommWarps && !done; k++) {
+        const int kind = (kinds >> (2 * k)) & 3;
+        const cplx v = S.ival[k][c];
+        if (kind == 0) {
+          ans1 = ans2 + v;
+          continue;
+        }
+        ans2 = kind == 2 ? ans2 + v : ans1 + v;
+        if (kind >= 2) {
+          intx = 1;
+          if (++restarts > 2) done = 2;
+          continue;
+        }
+        if (shanks_step(S, c, ans1, ans2, intx)) {
+          if (lane < 6) sum[c] = .5 * (S.q1[c][intx - 1] + S.q2[c][intx - 1]);
+          done = 1;
+        } else if (++intx > kSommMaxH) {
+          done = 2;
+        }
+      }
+      if (lane == 0) {
+        S.done = done;
+        if (done == 2) S.fail = 1;
+      }
+    }
+    __syncthreads();
+    if (S.done) return;
+  }
+  if (threadIdx.x == 0) S.fail = 1;
+  __syncthreads();
+}
+
+// The four field functions at the current (rho, zph): contour choice of
+// evlua (all threads of the CTA; the results are valid on every thread).
+__device__ void evlua(SommShared& S, cplx* erv, cplx* ezv, cplx* erh, cplx* eph) {
+  const Evl& E = S.E;
+  const int w = threadIdx.x >> 5, tid = threadIdx.x;
+  const bool six = tid < 6;
   double del = E.zph;
   if (E.rho > del) del = E.rho;
   if (E.zph >= 2. * E.rho) {
     // Bessel-function form
-    E.bessel_form = true;
-    E.a = mk(0.0, 0.0);
     del = 1.0 / del;
-    if (del > E.tkmag) {
-      E.b = mk(0.1 * E.tkmag, -0.1 * E.tkmag);
-      rom1(T, E, sum, 2);
-      E.a = E.b;
-      E.b = mk(del, -del);
-      rom1(T, E, ans, 2);
-      for (int i = 0; i < 6; i++) sum[i] += ans[i];
-    } else {
-      E.b = mk(del, -del);
-      rom1(T, E, sum, 2);
-    }
-    const cplx delta = mk(kSommPTP * del, 0.0);
-    gshank(T, E, E.b, delta, ans, sum, 0, E.b, E.b);
+    const bool two = del > E.tkmag;
+    const cplx mid = mk(0.1 * E.tkmag, -0.1 * E.tkmag), end = mk(del, -del);
+    if (w == 0) rom1_warp(S, true, mk(0.0, 0.0), two ? mid : end, 2);
+    if (w == 1 && two) rom1_warp(S, true, mid, end, 2);
+    __syncthreads();
+    if (six) S.sum[tid] = two ? S.ival[0][tid] + S.ival[1][tid] : S.ival[0][tid];
+    __syncthreads();
+    gshank(S, true, end, mk(kSommPTP * del, 0.0), S.ans, S.sum, 0, end, end);
   } else {
     // Hankel-function form
-    E.bessel_form = false;
     cplx cp1 = mk(0.0, .4 * E.ck2), cp2 = mk(.6 * E.ck2, -.2 * E.ck2), cp3 = mk(1.02 * E.ck2, -.2 * E.ck2);
-    E.a = cp1;
-    E.b = cp2;
-    rom1(T, E, sum, 2);
-    E.a = cp2;
-    E.b = cp3;
-    rom1(T, E, ans, 2);
-    for (int i = 0; i < 6; i++) sum[i] = -(sum[i] + ans[i]);
+    if (w == 0) rom1_warp(S, false, cp1, cp2, 2);
+    if (w == 1) rom1_warp(S, false, cp2, cp3, 2);
+    __syncthreads();
+    if (six) S.sum[tid] = -(S.ival[0][tid] + S.ival[1][tid]);
+    __syncthreads();
     const double slope = (E.zph > .001 * E.rho) ? E.rho / E.zph : 1000.;
     del = kSommPTP / del;
     cplx delta = mk(-1.0, slope) * del / sqrt(1. + slope * slope);
     const cplx delta2 = -conj_(delta);
     cplx bk = mk(0, 0);
-    gshank(T, E, cp1, delta, ans, sum, 0, bk, bk);
+    gshank(S, false, cp1, delta, S.ans, S.sum, 0, bk, bk);
     double rmis = E.rho * (E.ck1.re - E.ck2);
     bool below;
     if ((rmis < 2. * E.ck2) || (E.rho < 1.e-10)) {
@@ -475,56 +544,48 @@ __device__ void evlua(const BesselTables& T, Evl& E, cplx* erv, cplx* ezv, cplx*
       cp1 = E.ck1 - mk(0.1, +0.2);
       cp2 = cp1 + .2;
       bk = mk(0., del);
-      gshank(T, E, cp1, bk, sum, ans, 0, bk, bk);
-      E.a = cp1;
-      E.b = cp2;
-      rom1(T, E, ans, 1);
-      for (int i = 0; i < 6; i++) ans[i] -= sum[i];
-      gshank(T, E, cp3, bk, sum, ans, 0, bk, bk);
-      gshank(T, E, cp2, delta2, ans, sum, 0, bk, bk);
+      gshank(S, false, cp1, bk, S.sum, S.ans, 0, bk, bk);
+      if (w == 0) rom1_warp(S, false, cp1, cp2, 1);
+      __syncthreads();
+      if (six) S.ans[tid] = S.ival[0][tid] - S.sum[tid];
+      __syncthreads();
+      gshank(S, false, cp3, bk, S.sum, S.ans, 0, bk, bk);
+      gshank(S, false, cp2, delta2, S.ans, S.sum, 0, bk, bk);
     } else {
       // below the branch points, then to +infinity
-      for (int i = 0; i < 6; i++) sum[i] = -ans[i];
+      if (six) S.sum[tid] = -S.ans[tid];
+      __syncthreads();
       rmis = E.ck1.re * 1.01;
       if ((E.ck2 + 1.) > rmis) rmis = E.ck2 + 1.;
       bk = mk(rmis, .99 * E.ck1.im);
       delta = bk - cp3;
       delta = delta * (del / cabs_(delta));
-      gshank(T, E, cp3, delta, ans, sum, 1, bk, delta2);
+      gshank(S, false, cp3, delta, S.ans, S.sum, 1, bk, delta2);
     }
   }
-  ans[5] = ans[5] * E.ck1;
+  const cplx a5 = S.ans[5] * E.ck1;
   // conjugates: the integrals use exp(-jwt)
-  *erv = conj_(E.ck1sq * ans[2]);
-  *ezv = conj_(E.ck1sq * (ans[1] + E.ck2sq * ans[4]));
-  *erh = conj_(E.ck2sq * (ans[0] + ans[5]));
-  *eph = -conj_(E.ck2sq * (ans[3] + ans[5]));
+  *erv = conj_(E.ck1sq * S.ans[2]);
+  *ezv = conj_(E.ck1sq * (S.ans[1] + E.ck2sq * S.ans[4]));
+  *erh = conj_(E.ck2sq * (S.ans[0] + a5));
+  *eph = -conj_(E.ck2sq * (S.ans[3] + a5));
 }
 
-// One thread per grid point (257), plus the R = 0 column of the first grid
-// from the closed form (thread 0).  eps: complex permittivity (the reference's epscf).
-__global__ void __launch_bounds__(32) somm_table_kernel(cplx eps, double eta, cplx* tables, int* status) {
-  __shared__ BesselTables T;
-  if (threadIdx.x == 0) build_bessel_tables(T);
-  __syncthreads();
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// The tables: one CTA per grid point with integrals (257), and the R = 0
+// column of the first grid from its closed form (the last CTA).  eps:
+// complex permittivity (the reference's epscf).
+//
+// The integration is a chain of dependent decisions of about 3,000 integrand
+// evaluations at the slowest point; with a thread per point the kernel took
+// the latency of that chain (12.2 ms per frequency, 257 threads on 9 SMs).
+// Eight warps per point integrate eight contour intervals at once and 32
+// lanes the points of one: 0.235 ms.  Two CTAs fit an SM, so all 257 points
+// run in one wave.
+__global__ void __launch_bounds__(kSommThreads, 2) somm_table_kernel(cplx eps, double eta, cplx* tables, int* status) {
+  __shared__ SommShared S;
+  const int p = blockIdx.x;
   if (p < kSommEvalPoints) {
-    Evl E;
-    E.fail = 0;
-    E.ck2 = kTwoPiD;
-    E.ck2sq = E.ck2 * E.ck2;
-    E.ck1sq = E.ck2sq * conj_(eps);
-    E.ck1 = csqrt_(E.ck1sq);
-    E.ck1r = E.ck1.re;
-    E.tkmag = 100.0 * cabs_(E.ck1);
-    E.tsmag = 100.0 * cnorm(E.ck1);
-    E.cksm = E.ck2sq / (E.ck1sq + E.ck2sq);
-    E.ct1 = .5 * (E.ck1sq - E.ck2sq);
-    cplx erv = E.ck1sq * E.ck1sq, ezv = mk(E.ck2sq * E.ck2sq, 0.0), erh, eph;
-    E.ct2 = .125 * (erv - ezv);
-    erv = erv * E.ck1sq;
-    ezv = ezv * E.ck2sq;
-    E.ct3 = .0625 * (erv - ezv);
+    build_bessel_tables(S.T);
     // grid, radius and angle index of this point (grid 1 starts at R index 1)
     int g = 0, q = p;
     if (q >= 100) {
@@ -545,24 +606,45 @@ __global__ void __launch_bounds__(32) somm_table_kernel(cplx eps, double eta, cp
     for (int k = irs; k <= ir; k++) r += dr;
     double thet = somm_ys(g) - dth;
     for (int k = 0; k <= ith; k++) thet += dth;
-    E.rho = r * cos(thet);
-    E.zph = r * sin(thet);
-    if (E.rho < 1.e-7) E.rho = 1.e-8;
-    if (E.zph < 1.e-7) E.zph = 0.;
-    evlua(T, E, &erv, &ezv, &erh, &eph);
-    const double rk = E.ck2 * r;
-    double sr, cr;
-    sincos(rk, &sr, &cr);
-    const cplx con = (-mk(0.0, 4.771341189)) * r / mk(cr, -sr);
-    const int nd = nr * nth;
-    cplx* o = tables + somm_off(g) + ir + ith * nr;
-    o[0] = erv * con;
-    o[nd] = ezv * con;
-    o[2 * nd] = erh * con;
-    o[3 * nd] = eph * con;
-    if (E.fail) atomicOr(status, kStatIterCap);
-  }
-  if (p == 0) {
+    if (threadIdx.x == 0) {
+      Evl& E = S.E;
+      S.fail = 0;
+      E.ck2 = kTwoPiD;
+      E.ck2sq = E.ck2 * E.ck2;
+      E.ck1sq = E.ck2sq * conj_(eps);
+      E.ck1 = csqrt_(E.ck1sq);
+      E.ck1r = E.ck1.re;
+      E.tkmag = 100.0 * cabs_(E.ck1);
+      E.tsmag = 100.0 * cnorm(E.ck1);
+      E.cksm = E.ck2sq / (E.ck1sq + E.ck2sq);
+      E.ct1 = .5 * (E.ck1sq - E.ck2sq);
+      cplx e1 = E.ck1sq * E.ck1sq, e2 = mk(E.ck2sq * E.ck2sq, 0.0);
+      E.ct2 = .125 * (e1 - e2);
+      e1 = e1 * E.ck1sq;
+      e2 = e2 * E.ck2sq;
+      E.ct3 = .0625 * (e1 - e2);
+      E.rho = r * cos(thet);
+      E.zph = r * sin(thet);
+      if (E.rho < 1.e-7) E.rho = 1.e-8;
+      if (E.zph < 1.e-7) E.zph = 0.;
+    }
+    __syncthreads();
+    cplx erv, ezv, erh, eph;
+    evlua(S, &erv, &ezv, &erh, &eph);
+    if (threadIdx.x == 0) {
+      const double rk = S.E.ck2 * r;
+      double sr, cr;
+      sincos(rk, &sr, &cr);
+      const cplx con = (-mk(0.0, 4.771341189)) * r / mk(cr, -sr);
+      const int nd = nr * nth;
+      cplx* o = tables + somm_off(g) + ir + ith * nr;
+      o[0] = erv * con;
+      o[nd] = ezv * con;
+      o[2 * nd] = erh * con;
+      o[3 * nd] = eph * con;
+      if (S.fail) atomicOr(status, kStatIterCap);
+    }
+  } else if (threadIdx.x == 0) {
     // R = 0 of grid 1 from the static limit, c_ggrid.cpp:262-287
     const cplx c4 = mk(0.0, eta / 2.0);
     const cplx cl2 = -c4 * (eps - 1.) / (eps + 1.);
