@@ -3,8 +3,8 @@
 // fill, LU, refined solve, current coefficients and far field are the
 // single-problem path's, but the work of all problems shares each launch:
 //
-//   batch_fill_kernel     one CTA per (problem, 64-row tile, 32-column tile)
-//                         work item, through the single-problem fill tile
+//   batch_fill_kernel     one CTA per few rows of a problem, through the
+//                         single-problem fill_rows
 //   batch_lu_solve_kernel persistent: a CTA takes the next problem (largest
 //                         first) from a counter and does its complex64 LU
 //                         with partial pivoting (32-wide panels in shared
@@ -37,11 +37,13 @@ constexpr size_t kBatchPanelBytes = (size_t)kBatchMaxN * (kBatchNB + 1) * sizeof
 constexpr size_t kBatchUtBytes = (size_t)kBatchNB * (64 + 1) * sizeof(float2);
 constexpr size_t kBatchSmem = kBatchPanelBytes + kBatchUtBytes + 2 * kBatchMaxN * sizeof(double2) + 256;
 
+// One CTA per item: x problem, y first row, z rows and column block (in the
+// low and high halves), w sources staged at once.
 template <int GROUND, bool EXK>
-__global__ void __launch_bounds__(kFillTI) batch_fill_kernel(const FillArgs* __restrict__ As,
-                                                             const int4* __restrict__ items) {
-  const int4 it = items[blockIdx.x];  // x problem, y row tile, z column tile
-  fill_tile<GROUND, EXK, false>(As[it.x], ContractArgs{}, it.z, (int64_t)it.y * kFillTI);
+__global__ void __launch_bounds__(kFillThreads, GROUND == kGroundNone && !EXK ? 4 : 2)
+    batch_fill_kernel(const FillArgs* __restrict__ As, const int4* __restrict__ items) {
+  const int4 it = items[blockIdx.x];
+  fill_rows<GROUND, EXK, false>(As[it.x], ContractArgs{}, it.z >> 16, it.y, it.z & 0xffff, it.w);
 }
 
 // CTA-wide argmax of key (>= 0 candidates; -1 none), lowest row on ties.

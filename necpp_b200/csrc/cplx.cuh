@@ -87,4 +87,89 @@ __host__ __device__ __forceinline__ cplx cexp_(cplx z) {
   return {e * c, e * s};
 }
 
+#ifdef __CUDACC__
+// 1 / sqrt(x) of a positive normal x: the hardware approximation and one step
+// of Halley's iteration (y (1 + e/2 + 3 e^2/8), e = 1 - x y^2), which triples
+// its bits.  For the field kernels, whose squared distances are far from the
+// ends of the range; zero, infinity and NaN give NaN.
+__device__ __forceinline__ double rsqrt_pos(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// sqrt(x) and its reciprocal to half an ulp (one Newton step on each from
+// rsqrt_pos, the residuals exact by fused multiply-add)
+__device__ __forceinline__ double sqrt_pos(double x, double* inv) {
+  const double y = rsqrt_pos(x);
+  double r = x * y;
+  r = fma(fma(-r, r, x), 0.5 * y, r);
+  *inv = fma(fma(-r, y, 1.0), y, y);
+  return r;
+}
+
+// sin(pi x) and cos(pi x): exact reduction to |f| <= 1/4 (x = k/2 + f) and the
+// Taylor polynomials of sin(pi f)/f and cos(pi f) in f^2 (remainders below
+// 1e-18), swapped and signed by k mod 4.
+__device__ __forceinline__ void sincospi_poly(double x, double* s, double* c) {
+  const double k = rint(2.0 * x);
+  const double f = fma(-0.5, k, x), t = f * f;
+  double a = 7.952054001475513e-07;
+  a = fma(a, t, -2.1915353447830217e-05);
+  a = fma(a, t, 0.00046630280576761255);
+  a = fma(a, t, -0.0073704309457143504);
+  a = fma(a, t, 0.08214588661112823);
+  a = fma(a, t, -0.5992645293207921);
+  a = fma(a, t, 2.5501640398773455);
+  a = fma(a, t, -5.16771278004997);
+  a = fma(a, t, 3.141592653589793) * f;
+  double b = 4.303069587032947e-06;
+  b = fma(b, t, -0.0001046381049248457);
+  b = fma(b, t, 0.0019295743094039231);
+  b = fma(b, t, -0.02580689139001406);
+  b = fma(b, t, 0.2353306303588932);
+  b = fma(b, t, -1.3352627688545895);
+  b = fma(b, t, 4.0587121264167685);
+  b = fma(b, t, -4.934802200544679);
+  b = fma(b, t, 1.0);
+  const int q = __double2loint(k + 6755399441055744.0);  // k mod 2^32 (|k| < 2^51)
+  const double u = (q & 1) ? b : a, v = (q & 1) ? a : b;
+  *s = (q & 2) ? -u : u;
+  *c = ((q + 1) & 2) ? -v : v;
+}
+
+// sin and cos of x radians for angles of some thousands of periods at most:
+// Cody and Waite's reduction by pi/2 in two parts (the first of 33 bits, so
+// that its multiples are exact) and the Taylor polynomials on |f| <= pi/4.
+__device__ __forceinline__ void sincos_poly(double x, double* s, double* c) {
+  const double k = rint(x * 0.6366197723675814);
+  double f = fma(-k, 1.5707963267341256, x);  // exact
+  f = fma(-k, 6.077100506506192e-11, f);
+  const double t = f * f;
+  double a = 2.8114572543455206e-15;
+  a = fma(a, t, -7.647163731819816e-13);
+  a = fma(a, t, 1.6059043836821613e-10);
+  a = fma(a, t, -2.505210838544172e-08);
+  a = fma(a, t, 2.7557319223985893e-06);
+  a = fma(a, t, -0.0001984126984126984);
+  a = fma(a, t, 0.008333333333333333);
+  a = fma(a, t, -0.16666666666666666);
+  a = fma(a * t, f, f);
+  double b = 4.779477332387385e-14;
+  b = fma(b, t, -1.1470745597729725e-11);
+  b = fma(b, t, 2.08767569878681e-09);
+  b = fma(b, t, -2.755731922398589e-07);
+  b = fma(b, t, 2.48015873015873e-05);
+  b = fma(b, t, -0.001388888888888889);
+  b = fma(b, t, 0.041666666666666664);
+  b = fma(b, t, -0.5);
+  b = fma(b, t, 1.0);
+  const int q = __double2loint(k + 6755399441055744.0);
+  const double u = (q & 1) ? b : a, v = (q & 1) ? a : b;
+  *s = (q & 2) ? -u : u;
+  *c = ((q + 1) & 2) ? -v : v;
+}
+#endif
+
 }  // namespace necb

@@ -66,11 +66,12 @@ struct necgpu_engine {
   int ground = 0, use_exk = 0;
   double* d_seg = nullptr;  // 8n: x y z s b cab sab salp
   int32_t* d_ind = nullptr; // 2n
-  int32_t *d_tile_ptr = nullptr, *d_tsrc = nullptr, *d_tsrc_eptr = nullptr;
-  uint8_t* d_ecol = nullptr;
+  // the fill's column blocks (FillLists) and its cut into CTAs
+  int32_t *d_blk_ptr = nullptr, *d_fsrc = nullptr, *d_col_ptr = nullptr, *d_eloc = nullptr;
   double* d_ecoef = nullptr;  // 3*ne
   int64_t ne = 0;
-  int ntiles = 0;
+  int nblocks = 0;
+  FillPlan fplan{};
   int32_t *d_cptr = nullptr, *d_cbasis = nullptr;
   double* d_ccoef = nullptr;
   int64_t nc = 0;
@@ -417,10 +418,10 @@ void free_all(necgpu_engine* e) {
   e->lu_key = LuGraphKey{};
   dfree(e, e->d_seg);
   dfree(e, e->d_ind);
-  dfree(e, e->d_tile_ptr);
-  dfree(e, e->d_tsrc);
-  dfree(e, e->d_tsrc_eptr);
-  dfree(e, e->d_ecol);
+  dfree(e, e->d_blk_ptr);
+  dfree(e, e->d_fsrc);
+  dfree(e, e->d_col_ptr);
+  dfree(e, e->d_eloc);
   dfree(e, e->d_ecoef);
   dfree(e, e->d_cptr);
   dfree(e, e->d_cbasis);
@@ -528,12 +529,54 @@ double tock(necgpu_engine* e) {
 }
 
 // ---------------- fill ----------------
+// A structure's cut into the fill's CTAs.  Column blocks of at most 124
+// columns: a source that reaches columns of two blocks is evaluated in both,
+// which on plain wires is two sources per block, and 126 sources occupy the
+// 128 threads of a CTA once.  Junctions repeat more (a wire mesh needs 52
+// sources for 16 columns and still twice its columns at 1,000): with more
+// than four basis entries per segment one block is kept as long as a CTA with
+// an SM of its own can stage its sources.
+int fill_block_cols(int64_t n, int64_t ne) {
+  if (n <= kFillPairsBig && ne > 4 * n) return (int)n;
+  const int64_t nb = (n + kFillBlock - 1) / kFillBlock;
+  return (int)std::min(n, ((n + nb - 1) / nb + 3) / 4 * 4);
+}
+
+// Rows per CTA: as many as the staged pairs allow, so that a block's sources
+// and entries are read once for them, but no fewer than 600 CTAs (four per
+// SM) while a row each gives that many.  smax: most sources of a block.
+int fill_rows_per_cta(int64_t n, int nblocks, int smax) {
+  const int64_t by_grid = std::max<int64_t>(1, n * nblocks / 600);
+  return (int)std::max<int64_t>(1, std::min<int64_t>({kFillMaxRows, kFillPairs / std::max(smax, 1), by_grid}));
+}
+FillPlan fill_plan(int64_t n, int nblocks, int cols, int smax) {
+  FillPlan p{};
+  p.cols = cols;
+  p.rows = fill_rows_per_cta(n, nblocks, smax);
+  p.chunk = smax <= kFillPairsBig ? std::max(smax, 1) : kFillPairs;
+  const int most = p.chunk <= kFillPairs ? kFillThreads : p.chunk <= 1600 ? 2 * kFillThreads : kFillThreadsBig;
+  p.threads = std::max(64, std::min(most, (p.chunk + 31) / 32 * 32));
+  return p;
+}
+
+template <typename K>
+int fill_attr(necgpu_engine* e, K kernel, size_t smem) {
+  // the default limit of 48 KB counts the kernel's static arrays too
+  if (smem > 40 * 1024)
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  return 0;
+}
+
 template <int G, bool X>
 int launch_fill_t(necgpu_engine* e, const FillArgs& a) {
-  dim3 grid((unsigned)((e->n + kFillTI - 1) / kFillTI), (unsigned)e->ntiles);
+  const FillPlan& p = e->fplan;
+  const int threads = std::min(p.threads, fill_max_threads<G, X>());
+  const size_t smem = fill_smem(p.rows, p.chunk);
+  TRY(fill_attr(e, fill_kernel<G, X>, smem));
+  dim3 grid((unsigned)((e->n + p.rows - 1) / p.rows), (unsigned)e->nblocks);
   // work units of the fill: one per (observation, source) pair
   KLAUNCH(NECGPU_K_FILL, (double)e->n * (double)e->n,
-          fill_kernel<G, X><<<grid, kFillTI, 0, e->stream>>>(a));
+          fill_kernel<G, X><<<grid, threads, smem, e->stream>>>(a, p.rows, p.chunk));
   return 0;
 }
 
@@ -649,10 +692,11 @@ int run_fill(necgpu_engine* e, bool want64, bool want32) {
   a.salp = e->d_seg + 7 * n;
   a.ind1 = e->d_ind;
   a.ind2 = e->d_ind + n;
-  a.tile_src_ptr = e->d_tile_ptr;
-  a.tsrc = e->d_tsrc;
-  a.tsrc_eptr = e->d_tsrc_eptr;
-  a.ecol = e->d_ecol;
+  a.cols = e->fplan.cols;
+  a.blk_ptr = e->d_blk_ptr;
+  a.src = e->d_fsrc;
+  a.col_ptr = e->d_col_ptr;
+  a.eloc = e->d_eloc;
   a.ea = e->d_ecoef;
   a.eb = e->d_ecoef + e->ne;
   a.ec = e->d_ecoef + 2 * e->ne;
@@ -1956,56 +2000,57 @@ int fill_checked(necgpu_engine* e, bool want32) {
 
 namespace {
 
-// Column-tile source lists of a structure's basis tables (fill.cuh): for
-// every tile of kFillTB basis columns, the distinct contributing source
-// segments (ascending) and their (column, a, b, c) entries.  ecoef = a | b | c.
-// Built by a counting sort of the trio entries over tiles: each tile's
-// entries keep the (source, entry) order of the trio tables.
-struct TileLists {
-  std::vector<int32_t> tile_ptr, tsrc, tsrc_eptr;
-  std::vector<uint8_t> ecol;
+// Column blocks of a structure's basis tables (fill.cuh): for every block of
+// `cols` basis columns the distinct contributing source segments (ascending),
+// and for every column its entries by ascending source, an entry's source
+// given by its place in the block's list.  ecoef = a | b | c.
+struct FillLists {
+  std::vector<int32_t> blk_ptr, src, col_ptr, eloc;
   std::vector<double> ecoef;
+  int smax = 0;  // most sources of a block
 };
-void build_tile_lists(const necgpu_structure* s, int64_t n, int ntiles, TileLists& L) {
+void build_fill_lists(const necgpu_structure* s, int64_t n, int cols, FillLists& L) {
   const int32_t* tp = s->trio_ptr;
   const int64_t ne = tp[n];
-  // entry k of the trio tables goes to position at[tile] of the tile-sorted order
-  std::vector<int64_t> at(ntiles + 1, 0);
-  for (int64_t k = 0; k < ne; k++) at[s->trio_basis[k] / kFillTB + 1]++;
-  for (int t = 0; t < ntiles; t++) at[t + 1] += at[t];
-  std::vector<int32_t> src(ne), ent(ne);  // per sorted position: source segment, trio entry
-  {
-    std::vector<int64_t> next(at.begin(), at.end() - 1);
-    for (int64_t j = 0; j < n; j++)
-      for (int32_t k = tp[j]; k < tp[j + 1]; k++) {
-        const int64_t q = next[s->trio_basis[k] / kFillTB]++;
-        src[q] = (int32_t)j;
-        ent[q] = k;
+  const int nblk = (int)((n + cols - 1) / cols);
+  L.col_ptr.assign(n + 1, 0);
+  for (int64_t k = 0; k < ne; k++) L.col_ptr[s->trio_basis[k] + 1]++;
+  for (int64_t c = 0; c < n; c++) L.col_ptr[c + 1] += L.col_ptr[c];
+  // distinct sources per block, then their places
+  std::vector<int32_t> last(nblk, -1), count(nblk + 1, 0);
+  for (int64_t j = 0; j < n; j++)
+    for (int32_t k = tp[j]; k < tp[j + 1]; k++) {
+      const int b = s->trio_basis[k] / cols;
+      if (last[b] != (int32_t)j) {
+        last[b] = (int32_t)j;
+        count[b + 1]++;
       }
+    }
+  L.smax = 0;
+  for (int b = 0; b < nblk; b++) {
+    L.smax = std::max(L.smax, count[b + 1]);
+    count[b + 1] += count[b];
   }
-  L.tile_ptr.assign(ntiles + 1, 0);
-  L.tsrc.clear();
-  L.tsrc_eptr.clear();
-  L.tsrc.reserve(ne);
-  L.tsrc_eptr.reserve(ne + 1);
-  L.ecol.resize(ne);
+  L.blk_ptr = count;
+  L.src.assign(std::max<int32_t>(count[nblk], 1), 0);
+  L.eloc.assign(std::max<int64_t>(ne, 1), 0);
   L.ecoef.assign(3 * std::max<int64_t>(ne, 1), 0.0);
-  for (int t = 0; t < ntiles; t++) {
-    L.tile_ptr[t] = (int32_t)L.tsrc.size();
-    for (int64_t q = at[t]; q < at[t + 1]; q++) {
-      if (q == at[t] || src[q] != src[q - 1]) {
-        L.tsrc.push_back(src[q]);
-        L.tsrc_eptr.push_back((int32_t)q);
+  std::vector<int32_t> next(L.col_ptr.begin(), L.col_ptr.end() - 1), at(count.begin(), count.end() - 1);
+  std::fill(last.begin(), last.end(), -1);
+  for (int64_t j = 0; j < n; j++)
+    for (int32_t k = tp[j]; k < tp[j + 1]; k++) {
+      const int32_t c = s->trio_basis[k];
+      const int b = c / cols;
+      if (last[b] != (int32_t)j) {
+        last[b] = (int32_t)j;
+        L.src[at[b]++] = (int32_t)j;
       }
-      const int32_t k = ent[q];
-      L.ecol[q] = (uint8_t)(s->trio_basis[k] % kFillTB);
+      const int32_t q = next[c]++;
+      L.eloc[q] = at[b] - 1 - count[b];
       L.ecoef[q] = s->trio_a[k];
       L.ecoef[ne + q] = s->trio_b[k];
       L.ecoef[2 * ne + q] = s->trio_c[k];
     }
-  }
-  L.tile_ptr[ntiles] = (int32_t)L.tsrc.size();
-  L.tsrc_eptr.push_back((int32_t)ne);
 }
 
 // Per segment: the basis functions with support on it, ascending basis (the
@@ -2371,16 +2416,12 @@ int necgpu_set_structure(necgpu_engine* e, const necgpu_structure* s) {
     if (s->trio_basis[k] < 0 || s->trio_basis[k] >= n)
       return fail(e, NECGPU_ERR_ARG, "set_structure: basis index out of range");
 
-  const int ntiles = (int)((n + kFillTB - 1) / kFillTB);
-  e->ntiles = ntiles;
-  TileLists TL;
-  build_tile_lists(s, n, ntiles, TL);
-  const std::vector<int32_t>& tile_ptr = TL.tile_ptr;
-  const std::vector<int32_t>& tsrc = TL.tsrc;
-  const std::vector<int32_t>& tsrc_eptr = TL.tsrc_eptr;
-  const std::vector<uint8_t>& ecol = TL.ecol;
-  e->ne = (int64_t)ecol.size();
-  const std::vector<double>& ecoef = TL.ecoef;
+  FillLists FL;
+  const int cols = fill_block_cols(n, ntrio);
+  build_fill_lists(s, n, cols, FL);
+  e->nblocks = (int)((n + cols - 1) / cols);
+  e->fplan = fill_plan(n, e->nblocks, cols, FL.smax);
+  e->ne = ntrio;
   CoefLists CL;
   build_coef_lists(s, n, CL);
   e->nc = ntrio;
@@ -2394,11 +2435,11 @@ int necgpu_set_structure(necgpu_engine* e, const necgpu_structure* s) {
 
   TRY(upload(e, e->d_seg, seg.data(), seg.size()));
   TRY(upload(e, e->d_ind, ind.data(), ind.size()));
-  TRY(upload(e, e->d_tile_ptr, tile_ptr.data(), tile_ptr.size()));
-  TRY(upload(e, e->d_tsrc, tsrc.data(), std::max<size_t>(tsrc.size(), 1)));
-  TRY(upload(e, e->d_tsrc_eptr, tsrc_eptr.data(), tsrc_eptr.size()));
-  TRY(upload(e, e->d_ecol, ecol.data(), std::max<size_t>(ecol.size(), 1)));
-  TRY(upload(e, e->d_ecoef, ecoef.data(), ecoef.size()));
+  TRY(upload(e, e->d_blk_ptr, FL.blk_ptr.data(), FL.blk_ptr.size()));
+  TRY(upload(e, e->d_fsrc, FL.src.data(), FL.src.size()));
+  TRY(upload(e, e->d_col_ptr, FL.col_ptr.data(), FL.col_ptr.size()));
+  TRY(upload(e, e->d_eloc, FL.eloc.data(), FL.eloc.size()));
+  TRY(upload(e, e->d_ecoef, FL.ecoef.data(), FL.ecoef.size()));
   TRY(upload(e, e->d_cptr, cptr.data(), cptr.size()));
   TRY(upload(e, e->d_cbasis, cbasis.data(), cbasis.size()));
   TRY(upload(e, e->d_ccoef, ccoef.data(), ccoef.size()));
@@ -3019,10 +3060,9 @@ int necgpu_perturbed_terms(necgpu_engine* e, int nstruct, const necgpu_structure
     double* g = seg.data() + (size_t)q * 8 * n;
     const double* src[8] = {s->x, s->y, s->z, s->length, s->radius, s->cab, s->sab, s->salp};
     for (int a = 0; a < 8; a++) std::copy(src[a], src[a] + n, g + (size_t)a * n);
-    TileLists TL;
-    build_tile_lists(s, n, e->ntiles, TL);
-    if ((int64_t)TL.ecol.size() != ne) return fail(e, NECGPU_ERR_ARG, "perturbed_terms: tile layout differs");
-    std::copy(TL.ecoef.begin(), TL.ecoef.end(), pe.begin() + (size_t)q * 3 * std::max<int64_t>(ne, 1));
+    FillLists FL;
+    build_fill_lists(s, n, e->fplan.cols, FL);
+    std::copy(FL.ecoef.begin(), FL.ecoef.end(), pe.begin() + (size_t)q * 3 * std::max<int64_t>(ne, 1));
     CoefLists CL;
     build_coef_lists(s, n, CL);
     std::copy(CL.ccoef.begin(), CL.ccoef.end(), pc.begin() + (size_t)q * 3 * std::max<int64_t>(nc, 1));
@@ -3065,10 +3105,11 @@ int necgpu_perturbed_terms(necgpu_engine* e, int nstruct, const necgpu_structure
     a.salp = g + 7 * n;
     a.ind1 = e->d_ind;
     a.ind2 = e->d_ind + n;
-    a.tile_src_ptr = e->d_tile_ptr;
-    a.tsrc = e->d_tsrc;
-    a.tsrc_eptr = e->d_tsrc_eptr;
-    a.ecol = e->d_ecol;
+    a.cols = e->fplan.cols;
+    a.blk_ptr = e->d_blk_ptr;
+    a.src = e->d_fsrc;
+    a.col_ptr = e->d_col_ptr;
+    a.eloc = e->d_eloc;
     const double* c = e->d_pecoef + (size_t)q * pes;
     a.ea = c;
     a.eb = c + ne;
@@ -3089,20 +3130,31 @@ int necgpu_perturbed_terms(necgpu_engine* e, int nstruct, const necgpu_structure
   CUDA_TRY(cudaMemsetAsync(e->d_pout, 0, (size_t)nstruct * 2 * kMaxContract * sizeof(double), e->stream));
   CUDA_TRY(cudaMemsetAsync(e->d_status, 0, 4 * sizeof(int), e->stream));
   if (nw > 0) {
-    const dim3 grid((unsigned)((n + kFillTI - 1) / kFillTI), (unsigned)e->ntiles, (unsigned)nstruct);
+    const FillPlan& p = e->fplan;
+    const dim3 grid((unsigned)((n + p.rows - 1) / p.rows), (unsigned)e->nblocks, (unsigned)nstruct);
+    const size_t smem = fill_smem(p.rows, p.chunk);
     const bool xk = e->use_exk != 0;
-#define NECB_CONTRACT(G)                                                                                      \
-  (xk ? (fill_contract_kernel<G, true><<<grid, kFillTI, 0, e->stream>>>(e->d_pargs, e->d_pcargs), 0)           \
-      : (fill_contract_kernel<G, false><<<grid, kFillTI, 0, e->stream>>>(e->d_pargs, e->d_pcargs), 0))
+#define NECB_CONTRACT1(G, X)                                                                        \
+  do {                                                                                              \
+    TRY(fill_attr(e, fill_contract_kernel<G, X>, smem));                                            \
+    const int threads = std::min(p.threads, fill_max_threads<G, X>());                              \
+    KLAUNCH(NECGPU_K_FILL, (double)nstruct * n * n,                                                 \
+            fill_contract_kernel<G, X><<<grid, threads, smem, e->stream>>>(e->d_pargs, e->d_pcargs, \
+                                                                           p.rows, p.chunk));       \
+  } while (0)
+#define NECB_CONTRACT(G)    \
+  if (xk)                   \
+    NECB_CONTRACT1(G, true); \
+  else                      \
+    NECB_CONTRACT1(G, false)
     switch (e->ground) {
-      case kGroundNone: KLAUNCH(NECGPU_K_FILL, (double)nstruct * n * n, NECB_CONTRACT(kGroundNone)); break;
-      case kGroundPerfect: KLAUNCH(NECGPU_K_FILL, (double)nstruct * n * n, NECB_CONTRACT(kGroundPerfect)); break;
-      case kGroundReflection:
-        KLAUNCH(NECGPU_K_FILL, (double)nstruct * n * n, NECB_CONTRACT(kGroundReflection));
-        break;
-      default: KLAUNCH(NECGPU_K_FILL, (double)nstruct * n * n, NECB_CONTRACT(kGroundSommerfeld)); break;
+      case kGroundNone: NECB_CONTRACT(kGroundNone); break;
+      case kGroundPerfect: NECB_CONTRACT(kGroundPerfect); break;
+      case kGroundReflection: NECB_CONTRACT(kGroundReflection); break;
+      default: NECB_CONTRACT(kGroundSommerfeld); break;
     }
 #undef NECB_CONTRACT
+#undef NECB_CONTRACT1
   }
   const FarDir d = engine_far_dir(e, theta, phi);
   KLAUNCH(NECGPU_K_PATTERN, (double)nstruct * n * d.ksymp,
@@ -3160,13 +3212,12 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
   const int64_t T = seg_off[nprob], Zt = z_off[nprob];
   std::vector<double> seg(8 * T);
   std::vector<int32_t> ind(2 * T, 0);
-  std::vector<int32_t> tp_pool, ts_pool, te_pool, cptr_g(T + 1, 0), cbasis_pool;
-  std::vector<uint8_t> ecol_pool;
+  std::vector<int32_t> bp_pool, src_pool, cp_pool, eloc_pool, cptr_g(T + 1, 0), cbasis_pool;
   std::vector<double> ecoef_pool, ca_pool, cb_pool, cc_pool;
-  std::vector<int64_t> tp_off(nprob), ts_off(nprob), te_off(nprob), ec_off(nprob), ecf_off(nprob), ne_p(nprob);
-  std::vector<int> ntiles_p(nprob), seg_prob(T);
-  // per-problem tile and coefficient lists on all host cores, then concatenated
-  std::vector<TileLists> TLs(nprob);
+  std::vector<int64_t> bp_off(nprob), src_off(nprob), cp_off(nprob), el_off(nprob), ecf_off(nprob), ne_p(nprob);
+  std::vector<int> seg_prob(T);
+  // per-problem fill and coefficient lists on all host cores, then concatenated
+  std::vector<FillLists> FLs(nprob);
   std::vector<CoefLists> CLs(nprob);
   std::vector<int> bad(nprob, 0);
   {
@@ -3184,7 +3235,7 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
           bad[p] = 1;
           continue;
         }
-        build_tile_lists(&s, n, (int)((n + kFillTB - 1) / kFillTB), TLs[p]);
+        build_fill_lists(&s, n, fill_block_cols(n, tp[n]), FLs[p]);
         build_coef_lists(&s, n, CLs[p]);
       }
     };
@@ -3206,19 +3257,18 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     }
     for (int64_t j = 0; j < n; j++) seg_prob[o + j] = p;
     const int32_t* tp = s.trio_ptr;
-    ntiles_p[p] = (int)((n + kFillTB - 1) / kFillTB);
-    const TileLists& TL = TLs[p];
-    tp_off[p] = (int64_t)tp_pool.size();
-    ts_off[p] = (int64_t)ts_pool.size();
-    te_off[p] = (int64_t)te_pool.size();
-    ec_off[p] = (int64_t)ecol_pool.size();
+    const FillLists& FL = FLs[p];
+    bp_off[p] = (int64_t)bp_pool.size();
+    src_off[p] = (int64_t)src_pool.size();
+    cp_off[p] = (int64_t)cp_pool.size();
+    el_off[p] = (int64_t)eloc_pool.size();
     ecf_off[p] = (int64_t)ecoef_pool.size();
-    ne_p[p] = (int64_t)TL.ecol.size();
-    tp_pool.insert(tp_pool.end(), TL.tile_ptr.begin(), TL.tile_ptr.end());
-    ts_pool.insert(ts_pool.end(), TL.tsrc.begin(), TL.tsrc.end());
-    te_pool.insert(te_pool.end(), TL.tsrc_eptr.begin(), TL.tsrc_eptr.end());
-    ecol_pool.insert(ecol_pool.end(), TL.ecol.begin(), TL.ecol.end());
-    ecoef_pool.insert(ecoef_pool.end(), TL.ecoef.begin(), TL.ecoef.end());
+    ne_p[p] = tp[n];
+    bp_pool.insert(bp_pool.end(), FL.blk_ptr.begin(), FL.blk_ptr.end());
+    src_pool.insert(src_pool.end(), FL.src.begin(), FL.src.end());
+    cp_pool.insert(cp_pool.end(), FL.col_ptr.begin(), FL.col_ptr.end());
+    eloc_pool.insert(eloc_pool.end(), FL.eloc.begin(), FL.eloc.end());
+    ecoef_pool.insert(ecoef_pool.end(), FL.ecoef.begin(), FL.ecoef.end());
     const CoefLists& CL = CLs[p];
     const int64_t nt = tp[n], cbase = (int64_t)cbasis_pool.size();
     for (int64_t j = 0; j < n; j++) cptr_g[o + j] = (int32_t)(cbase + CL.cptr[j]);
@@ -3228,16 +3278,14 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     cc_pool.insert(cc_pool.end(), CL.ccoef.begin() + 2 * nt, CL.ccoef.begin() + 3 * nt);
   }
   cptr_g[T] = (int32_t)cbasis_pool.size();
-  for (auto* v : {&ts_pool, &te_pool, &cbasis_pool})
-    if (v->empty()) v->push_back(0);
-  if (ecol_pool.empty()) ecol_pool.push_back(0);
-  for (auto* v : {&ca_pool, &cb_pool, &cc_pool, &ecoef_pool})
+  if (cbasis_pool.empty()) cbasis_pool.push_back(0);
+  for (auto* v : {&ca_pool, &cb_pool, &cc_pool})
     if (v->empty()) v->push_back(0.0);
   // device pools (stream-ordered; freed at the end of the call)
   double *d_seg = nullptr, *d_ecoef = nullptr, *d_ca = nullptr, *d_cb = nullptr, *d_cc = nullptr, *d_abc = nullptr,
          *d_res = nullptr;
-  int32_t *d_ind = nullptr, *d_tp = nullptr, *d_ts = nullptr, *d_te = nullptr, *d_cptr = nullptr, *d_cbasis = nullptr;
-  uint8_t* d_ecol = nullptr;
+  int32_t *d_ind = nullptr, *d_bp = nullptr, *d_src = nullptr, *d_cp = nullptr, *d_el = nullptr, *d_cptr = nullptr,
+          *d_cbasis = nullptr;
   double2 *d_Z64 = nullptr, *d_b = nullptr, *d_x = nullptr, *d_cur = nullptr, *d_eth = nullptr, *d_eph = nullptr,
           *d_dirs = nullptr;
   float2* d_Z32 = nullptr;
@@ -3247,8 +3295,8 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
   int4* d_items = nullptr;
   auto release = [&]() {
     dfree(e, d_seg), dfree(e, d_ecoef), dfree(e, d_ca), dfree(e, d_cb), dfree(e, d_cc), dfree(e, d_abc);
-    dfree(e, d_res), dfree(e, d_ind), dfree(e, d_tp), dfree(e, d_ts), dfree(e, d_te), dfree(e, d_cptr);
-    dfree(e, d_cbasis), dfree(e, d_ecol), dfree(e, d_Z64), dfree(e, d_b), dfree(e, d_x), dfree(e, d_cur);
+    dfree(e, d_res), dfree(e, d_ind), dfree(e, d_bp), dfree(e, d_src), dfree(e, d_cp), dfree(e, d_cptr);
+    dfree(e, d_cbasis), dfree(e, d_el), dfree(e, d_Z64), dfree(e, d_b), dfree(e, d_x), dfree(e, d_cur);
     dfree(e, d_eth), dfree(e, d_eph), dfree(e, d_dirs), dfree(e, d_Z32), dfree(e, d_perm), dfree(e, d_segp);
     dfree(e, d_order), dfree(e, d_next), dfree(e, d_st), dfree(e, d_probs), dfree(e, d_args), dfree(e, d_items);
   };
@@ -3256,10 +3304,10 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
   do {
     if ((rc = upload(e, d_seg, seg.data(), seg.size()))) break;
     if ((rc = upload(e, d_ind, ind.data(), ind.size()))) break;
-    if ((rc = upload(e, d_tp, tp_pool.data(), tp_pool.size()))) break;
-    if ((rc = upload(e, d_ts, ts_pool.data(), ts_pool.size()))) break;
-    if ((rc = upload(e, d_te, te_pool.data(), te_pool.size()))) break;
-    if ((rc = upload(e, d_ecol, ecol_pool.data(), ecol_pool.size()))) break;
+    if ((rc = upload(e, d_bp, bp_pool.data(), bp_pool.size()))) break;
+    if ((rc = upload(e, d_src, src_pool.data(), src_pool.size()))) break;
+    if ((rc = upload(e, d_cp, cp_pool.data(), cp_pool.size()))) break;
+    if ((rc = upload(e, d_el, eloc_pool.data(), eloc_pool.size()))) break;
     if ((rc = upload(e, d_ecoef, ecoef_pool.data(), ecoef_pool.size()))) break;
     if ((rc = upload(e, d_cptr, cptr_g.data(), cptr_g.size()))) break;
     if ((rc = upload(e, d_cbasis, cbasis_pool.data(), cbasis_pool.size()))) break;
@@ -3277,10 +3325,11 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     if ((rc = dalloc(e, d_st, (size_t)nprob))) break;
     if ((rc = dalloc(e, d_res, (size_t)nprob))) break;
     if ((rc = dalloc(e, d_next, 1))) break;
-    // per-problem fill arguments and the fill work list
+    // per-problem fill arguments
     std::vector<FillArgs> fa(nprob);
     std::vector<BatchProblem> bp(nprob);
-    std::vector<int4> items;
+    std::vector<int4> items;  // the fill's CTAs: problem, first row, rows, sources
+    size_t fsmem = 0;
     for (int p = 0; p < nprob; p++) {
       const necgpu_structure& s = structs[p];
       const int64_t n = s.n, o = seg_off[p];
@@ -3297,10 +3346,11 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
       a.salp = d_seg + 7 * T + o;
       a.ind1 = d_ind + o;
       a.ind2 = d_ind + T + o;
-      a.tile_src_ptr = d_tp + tp_off[p];
-      a.tsrc = d_ts + ts_off[p];
-      a.tsrc_eptr = d_te + te_off[p];
-      a.ecol = d_ecol + ec_off[p];
+      a.cols = fill_block_cols(n, s.trio_ptr[n]);
+      a.blk_ptr = d_bp + bp_off[p];
+      a.src = d_src + src_off[p];
+      a.col_ptr = d_cp + cp_off[p];
+      a.eloc = d_el + el_off[p];
       a.ea = d_ecoef + ecf_off[p];
       a.eb = a.ea + ne_p[p];
       a.ec = a.ea + 2 * ne_p[p];
@@ -3314,9 +3364,11 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
       a.Z32 = d_Z32 + z_off[p];
       a.status = e->d_status;
       bp[p] = BatchProblem{(int)n, z_off[p], o};
-      const int rt = (int)((n + kFillTI - 1) / kFillTI);
-      for (int r = 0; r < rt; r++)
-        for (int c = 0; c < ntiles_p[p]; c++) items.push_back(make_int4(p, r, c, 0));
+      const int S = std::max(FLs[p].smax, 1), rows = std::max(1, std::min(kFillMaxRows, kFillPairs / S));
+      const int nblk = (int)FLs[p].blk_ptr.size() - 1;
+      fsmem = std::max(fsmem, fill_smem(rows, S));
+      for (int b = 0; b < nblk; b++)
+        for (int64_t r = 0; r < n; r += rows) items.push_back(make_int4(p, (int)r, rows | b << 16, S));
     }
     std::vector<int> order(nprob);
     std::iota(order.begin(), order.end(), 0);
@@ -3334,16 +3386,26 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
       for (int p = 0; p < nprob; p++) q += (double)structs[p].n * structs[p].n;
       return q;
     }();
-#define NECB_BFILL(G)                                                                                         \
-  (xk ? (batch_fill_kernel<G, true><<<(unsigned)items.size(), kFillTI, 0, e->stream>>>(d_args, d_items), 0)    \
-      : (batch_fill_kernel<G, false><<<(unsigned)items.size(), kFillTI, 0, e->stream>>>(d_args, d_items), 0))
+#define NECB_BFILL1(G, X)                                                                                     \
+  do {                                                                                                        \
+    if ((rc = fill_attr(e, batch_fill_kernel<G, X>, fsmem))) break;                                           \
+    KLAUNCH(NECGPU_K_FILL, pairs,                                                                             \
+            batch_fill_kernel<G, X><<<(unsigned)items.size(), kFillThreads, fsmem, e->stream>>>(d_args, d_items)); \
+  } while (0)
+#define NECB_BFILL(G)     \
+  if (xk)                 \
+    NECB_BFILL1(G, true); \
+  else                    \
+    NECB_BFILL1(G, false)
     switch (s0.ground) {
-      case kGroundNone: KLAUNCH(NECGPU_K_FILL, pairs, NECB_BFILL(kGroundNone)); break;
-      case kGroundPerfect: KLAUNCH(NECGPU_K_FILL, pairs, NECB_BFILL(kGroundPerfect)); break;
-      case kGroundReflection: KLAUNCH(NECGPU_K_FILL, pairs, NECB_BFILL(kGroundReflection)); break;
-      default: KLAUNCH(NECGPU_K_FILL, pairs, NECB_BFILL(kGroundSommerfeld)); break;
+      case kGroundNone: NECB_BFILL(kGroundNone); break;
+      case kGroundPerfect: NECB_BFILL(kGroundPerfect); break;
+      case kGroundReflection: NECB_BFILL(kGroundReflection); break;
+      default: NECB_BFILL(kGroundSommerfeld); break;
     }
 #undef NECB_BFILL
+#undef NECB_BFILL1
+    if (rc) break;
     // LU and refined solve, one problem per CTA at a time
     CUDA_TRY(cudaFuncSetAttribute(batch_lu_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kBatchSmem));

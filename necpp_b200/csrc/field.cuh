@@ -23,16 +23,18 @@ enum : int {
   kStatRombergCap = 1,     // intx hit the step-size limit ("STEP SIZE LIMITED")
   kStatIterCap = 2,        // a quadrature exceeded its iteration bound
   kStatSommerfeldTab = 4,  // a pair needs the Sommerfeld table path (r <= 0.95)
+  kStatDefer = 256,        // first-try evaluation (FIRST): the pair needs interval halvings (never reported)
 };
 
 struct SrcSeg {
   double x, y, z, s, b, cab, sab, salp;
   int ind1, ind2;
-  double sfac;  // far_sfac(s): set by whoever builds the SrcSeg
+  double ss, cs;  // sin and cos of pi s (half the electrical length)
 };
 
-// sin(pi s) / pi of efld_compute's far branch (2815), once per source
-__device__ __forceinline__ double far_sfac(double s) { return sin(kPiD * s) / kPiD; }
+// Set by whoever builds a SrcSeg, once per source: eksc's ss and cs (shk = pi
+// s), the far branch's sin(pi s) / pi (2815).
+__device__ __forceinline__ void set_half_length(SrcSeg& J) { sincos_poly(kPiD * J.s, &J.ss, &J.cs); }
 
 struct FieldParams {
   double rkh;
@@ -69,31 +71,84 @@ __device__ __forceinline__ void conv_test(double f1r, double f2r, double* tr, do
   *ti = fabs((f1i - f2i) / den);
 }
 
-// exp(jkr)/(kr) integrand, nec_context.cpp:3553-3578
+// exp(jkr)/(kr) integrand, nec_context.cpp:3553-3578 (the quotients by one
+// reciprocal square root)
 __device__ __forceinline__ void gf(double zk, double zpk, double rkb2, bool ija, double* co,
                                    double* si) {
   double zdk = zk - zpk;
-  double rk = sqrt(rkb2 + zdk * zdk);
-  double s, c;
-  sincos(rk, &s, &c);
-  *si = s / rk;
+  const double rks = rkb2 + zdk * zdk;
+  double s, c, rinv;
+  const double rk = sqrt_pos(rks, &rinv);
+  sincos_poly(rk, &s, &c);
+  *si = s * rinv;
   if (ija) {
-    *co = c / rk;
+    *co = c * rinv;
     return;
   }
   if (rk >= .2) {
-    *co = (c - 1.0) / rk;
+    *co = (c - 1.0) * rinv;
     return;
   }
-  double rks = rk * rk;
   *co = ((-1.38888889e-3 * rks + 4.16666667e-2) * rks - 0.5) * rk;
+}
+
+constexpr double kIntxRx = 1.0e-4;  // intx's convergence test
+
+// The two tests of intx (conv_test without its quotients): whether the
+// three-point result is accepted, and whether the five-point result is
+// refused.  Both are false for a NaN, which the reference accepts as a
+// five-point result.
+__device__ __forceinline__ double intx_den(double f2r, double f2i) {
+  double den = fabs(f2r);
+  const double t = fabs(f2i);
+  if (den < t) den = t;
+  return den;
+}
+__device__ __forceinline__ bool intx_accepts(double f1r, double f2r, double f1i, double f2i) {
+  const double den = intx_den(f2r, f2i), tol = kIntxRx * den;
+  return den < 1.0e-37 || (fabs(f1i - f2i) <= tol && fabs(f1r - f2r) <= tol);
+}
+__device__ __forceinline__ bool intx_refuses(double f1r, double f2r, double f1i, double f2i) {
+  const double den = intx_den(f2r, f2i), tol = kIntxRx * den;
+  return !(den < 1.0e-37) && (fabs(f1i - f2i) > tol || fabs(f1r - f2r) > tol);
+}
+
+// The first step of intx, which covers the whole interval: three points,
+// then five.  Most pairs need no more; one that does reports kStatDefer and
+// is evaluated again by the full sequence (intx), so that the lanes of a warp
+// take the same straight path here.
+__device__ __forceinline__ void intx_first(double el1, double el2, double b, bool ij, double zpk, double rkb2,
+                                           double* sgr, double* sgi, int* status) {
+  const double z = el1, ze = ij ? el2 : 0., dz = ze - z, dzot = dz * .5;
+  double g1r, g1i, g3r, g3i, g5r, g5i;
+  gf(z, zpk, rkb2, ij, &g1r, &g1i);
+  gf(z + dzot, zpk, rkb2, ij, &g3r, &g3i);
+  gf(z + dz, zpk, rkb2, ij, &g5r, &g5i);
+  const double t00r = (g1r + g5r) * dzot, t00i = (g1i + g5i) * dzot;
+  const double t01r = (t00r + dz * g3r) * 0.5, t01i = (t00i + dz * g3i) * 0.5;
+  double sr = (4.0 * t01r - t00r) / 3.0, si = (4.0 * t01i - t00i) / 3.0;
+  if (!intx_accepts(t01r, sr, t01i, si)) {
+    double g2r, g2i, g4r, g4i;
+    gf(z + dz * 0.25, zpk, rkb2, ij, &g2r, &g2i);
+    gf(z + dz * 0.75, zpk, rkb2, ij, &g4r, &g4i);
+    const double t02r = (t01r + dzot * (g2r + g4r)) * 0.5, t02i = (t01i + dzot * (g2i + g4i)) * 0.5;
+    const double t11r = (4.0 * t02r - t01r) / 3.0, t11i = (4.0 * t02i - t01i) / 3.0;
+    sr = (16.0 * t11r - sr) / 15.0;
+    si = (16.0 * t11i - si) / 15.0;
+    if (intx_refuses(t11r, sr, t11i, si)) *status |= kStatDefer;
+  }
+  if (!ij) {
+    sr = 2. * (sr + log((sqrt(b * b + dz * dz) + dz) / b));
+    si = 2. * si;
+  }
+  *sgr = sr;
+  *sgi = si;
 }
 
 // Variable-interval Romberg integration of exp(jkr)/r, nec_context.cpp:4135-4300
 __device__ void intx(double el1, double el2, double b, bool ij, double zpk, double rkb2,
                      double* sgr, double* sgi, int* status) {
   const int nx = 1, nma = 65536, nts = 4;
-  const double rx = 1.0e-4;
   double z = el1, ze = el2;
   if (!ij) ze = 0.;
   const double s = ze - z;
@@ -130,9 +185,7 @@ __device__ void intx(double el1, double el2, double b, bool ij, double zpk, doub
       double t01i = (t00i + dz * g3i) * 0.5;
       double t10r = (4.0 * t01r - t00r) / 3.0;
       double t10i = (4.0 * t01i - t00i) / 3.0;
-      double te1r, te1i;
-      conv_test(t01r, t10r, &te1r, t01i, t10i, &te1i);
-      if (te1i <= rx && te1r <= rx) {
+      if (intx_accepts(t01r, t10r, t01i, t10i)) {
         sr = sr + t10r;
         si = si + t10i;
         nt += 2;
@@ -157,9 +210,7 @@ __device__ void intx(double el1, double el2, double b, bool ij, double zpk, doub
       double t11i = (4.0 * t02i - t01i) / 3.0;
       double t20r = (16.0 * t11r - t10r) / 15.0;
       double t20i = (16.0 * t11i - t10i) / 15.0;
-      double te2r, te2i;
-      conv_test(t11r, t20r, &te2r, t11i, t20i, &te2i);
-      if (te2i > rx || te2r > rx) {
+      if (intx_refuses(t11r, t20r, t11i, t20i)) {
         nt = 0;
         if (ns >= nma) {
           *status |= kStatRombergCap;
@@ -202,14 +253,13 @@ done:
 
 // segment-end terms, nec_context.cpp:3605-3620
 __device__ __forceinline__ void gx(double zz, double rh, double xk, cplx* gz, cplx* gzp) {
-  double r2 = zz * zz + rh * rh;
-  double r = sqrt(r2);
-  double rkz = xk * r;
-  double s, c;
-  sincos(rkz, &s, &c);
-  cplx temp = mk(c, -s) / r;
+  const double r2 = zz * zz + rh * rh;
+  double s, c, rinv;
+  const double rkz = xk * sqrt_pos(r2, &rinv);
+  sincos_poly(rkz, &s, &c);
+  const cplx temp = mk(c, -s) * rinv;
   *gz = temp;
-  *gzp = -mk(1.0, rkz) * temp / r2;
+  *gzp = -mk(1.0, rkz) * temp * (rinv * rinv);
 }
 
 // extended-kernel segment-end terms, nec_context.cpp:3623-3676
@@ -256,17 +306,26 @@ __device__ void gxx(double zz, double rh, double a, double a2, double xk, int ir
   *gzp = -zz * c1 * gz;
 }
 
-// thin-wire (reduced) kernel, nec_context.cpp:3051-3104
-__device__ void eksc(double s, double z, double rh, double xk, bool ij, cplx* ezs, cplx* ers,
-                     cplx* ezc, cplx* erc, cplx* ezk, cplx* erk, int* status) {
+template <bool FIRST>
+__device__ __forceinline__ void intx_t(double el1, double el2, double b, bool ij, double zpk, double rkb2,
+                                       double* sgr, double* sgi, int* status) {
+  if (FIRST)
+    intx_first(el1, el2, b, ij, zpk, rkb2, sgr, sgi, status);
+  else
+    intx(el1, el2, b, ij, zpk, rkb2, sgr, sgi, status);
+}
+
+// thin-wire (reduced) kernel, nec_context.cpp:3051-3104; rhinv = 1 / rh
+template <bool FIRST>
+__device__ __forceinline__ void eksc(const SrcSeg& J, double z, double rh, double rhinv, double xk, bool ij, cplx* ezs,
+                                     cplx* ers, cplx* ezc, cplx* erc, cplx* ezk, cplx* erk, int* status) {
   const cplx C1 = mk(0.0, kC1);
   double zpk = xk * z;
   double rhk = xk * rh;
   double rkb2 = rhk * rhk;
-  double sh = .5 * s;
+  double sh = .5 * J.s;
   double shk = xk * sh;
-  double ss, cs;
-  sincos(shk, &ss, &cs);
+  const double ss = J.ss, cs = J.cs;
   double z2a = sh - z;
   double z1a = -(sh + z);
   cplx gz1, gz2, gp1, gp2;
@@ -278,13 +337,13 @@ __device__ void eksc(double s, double z, double rh, double xk, bool ij, cplx* ez
   *ezc = -C1 * ((gz2 + gz1) * ss * xk + (gzp2 - gzp1) * cs);
   *erk = C1 * (gp2 - gp1) * rh;
   double cint, sint;
-  intx(-shk, shk, rhk, ij, zpk, rkb2, &cint, &sint, status);
+  intx_t<FIRST>(-shk, shk, rhk, ij, zpk, rkb2, &cint, &sint, status);
   *ezk = -C1 * (gzp2 - gzp1 + xk * xk * mk(cint, -sint));
   if (rh >= 1.0e-10) {
     gzp1 = gzp1 * z1a;
     gzp2 = gzp2 * z2a;
-    *ers = -C1 * ((gzp2 + gzp1 + gz2 + gz1) * ss - (z2a * gz2 - z1a * gz1) * cs * xk) / rh;
-    *erc = -C1 * ((gzp2 - gzp1 + gz2 - gz1) * cs + (z2a * gz2 + z1a * gz1) * ss * xk) / rh;
+    *ers = -C1 * ((gzp2 + gzp1 + gz2 + gz1) * ss - (z2a * gz2 - z1a * gz1) * cs * xk) * rhinv;
+    *erc = -C1 * ((gzp2 - gzp1 + gz2 - gz1) * cs + (z2a * gz2 + z1a * gz1) * ss * xk) * rhinv;
     return;
   }
   *ers = mk(0., 0.);
@@ -292,10 +351,12 @@ __device__ void eksc(double s, double z, double rh, double xk, bool ij, cplx* ez
 }
 
 // extended thin-wire kernel, nec_context.cpp:3108-3188
-__device__ void ekscx(double bx, double s, double z, double rhx, double xk, bool ij, int inx1,
-                      int inx2, cplx* ezs, cplx* ers, cplx* ezc, cplx* erc, cplx* ezk,
-                      cplx* erk, int* status) {
+template <bool FIRST>
+__device__ __forceinline__ void ekscx(const SrcSeg& J, double z, double rhx, double xk, bool ij, cplx* ezs, cplx* ers,
+                                      cplx* ezc, cplx* erc, cplx* ezk, cplx* erk, int* status) {
   const cplx C1 = mk(0.0, kC1);
+  const double bx = J.b, s = J.s, ss = J.ss, cs = J.cs;
+  const int inx1 = J.ind1, inx2 = J.ind2;
   double b, rh;
   int ira;
   if (rhx >= bx) {
@@ -312,8 +373,6 @@ __device__ void ekscx(double bx, double s, double z, double rhx, double xk, bool
   double rhk = xk * rh;
   double rkb2 = rhk * rhk;
   double shk = xk * sh;
-  double ss, cs;
-  sincos(shk, &ss, &cs);
   double z2a = sh - z;
   double z1a = -(sh + z);
   double a2 = b * b;
@@ -344,92 +403,130 @@ __device__ void ekscx(double bx, double s, double z, double rhx, double xk, bool
   *erc = -C1 * ((z2a * grp2 - z1a * grp1 + gr2 - gr1) * cs + (z2a * gr2 + z1a * gr1) * ss * xk);
   *erk = C1 * (grk2 - grk1);
   double cint, sint;
-  intx(-shk, shk, rhk, ij, zpk, rkb2, &cint, &sint, status);
+  intx_t<FIRST>(-shk, shk, rhk, ij, zpk, rkb2, &cint, &sint, status);
   double bk = b * xk;
   double bk2 = bk * bk * .25;
   *ezk = -C1 * (gzp2 - gzp1 + xk * xk * (1. - bk2) * mk(cint, -sint) - bk2 * (gzz2 - gzz1));
 }
 
+// Cylindrical displacement of an observation point from a source (direct or
+// image, salpr = +-salp) and the far-pair decision, 2777-2797.
+struct PairGeom {
+  double zp, rh, rhinv, r, rinv;      // rinv only for a far pair
+  double rhox, rhoy, rhoz;            // radial unit vector (0 on the axis)
+  bool far;
+};
+
+__device__ __forceinline__ PairGeom pair_geometry(const SrcSeg& J, double xij, double yij, double zij, double salpr,
+                                                  double ai, double rkh) {
+  PairGeom g;
+  g.zp = xij * J.cab + yij * J.sab + zij * salpr;
+  g.rhox = xij - J.cab * g.zp;
+  g.rhoy = yij - J.sab * g.zp;
+  g.rhoz = zij - salpr * g.zp;
+  // both distances and their reciprocals by a reciprocal square root each
+  const double rh2 = g.rhox * g.rhox + g.rhoy * g.rhoy + g.rhoz * g.rhoz + ai * ai;
+  const double r2 = g.zp * g.zp + rh2;
+  g.rh = sqrt_pos(rh2, &g.rhinv);
+  g.r = sqrt_pos(r2, &g.rinv);
+  if (rh2 == 0.0) g.rh = 0.0;
+  if (r2 == 0.0) g.r = 0.0;
+  // a pair at the threshold is decided by the reference's own rounding
+  if (fabs(g.r - rkh) <= 1e-12 * rkh) {
+    const double rh = sqrt(rh2);
+    g.r = sqrt(g.zp * g.zp + rh * rh);
+  }
+  g.far = g.r >= rkh;
+  const double u = g.rh <= 1.e-10 ? 0.0 : g.rhinv;
+  g.rhox *= u;
+  g.rhoy *= u;
+  g.rhoz *= u;
+  return g;
+}
+
+// Far pair: the source as a lumped current element, 2798-2819.  The fields of
+// its constant and cosine currents are one field times the length and
+// sin(pi s) / pi, the sine current has none.  Returns that field projected on
+// a direction with components dz along the source and dr along the radial
+// unit vector: the reference's e1 cth - e2 px and e1 px + e2 cth collected
+// over the common factor eta exp(-j 2 pi r) / (2 pi r^2).
+__device__ __forceinline__ cplx far_projected(const PairGeom& g, double dz, double dr, double eta) {
+  const double rmag = kTwoPiD * g.r, cth = g.zp * g.rinv, px = g.rh * g.rinv;
+  const double rminv = g.rinv * (1.0 / kTwoPiD);
+  // exp(-j rmag) as sincospi of r * 2 pi / pi_exact (exact reduction)
+  constexpr double kTwoPiOverPi = kTwoPiD / 3.141592653589793;
+  double sn, cs;
+  sincospi_poly(kTwoPiOverPi * g.r, &sn, &cs);
+  const double c2 = cth * cth, hp2 = .5 * px * px, pc = px * cth, q = .5 * (rmag - rminv);
+  const double f = eta * (rminv * g.rinv);
+  const double re = (dz * (c2 - hp2) + dr * (1.5 * pc)) * f;
+  const double im = (dr * (pc * (q - rminv)) - dz * (c2 * rminv + (2.0 * hp2) * q)) * f;
+  return mk(re * cs + im * sn, im * cs - re * sn);
+}
+
+// Near pair: fields of the constant, sine and cosine currents along the
+// source (z) and radially (r), 2820-2832.
+template <bool EXK, bool FIRST>
+__device__ __forceinline__ void near_components(const SrcSeg& J, const PairGeom& g, bool ijx, cplx* tezs, cplx* ters,
+                                                cplx* tezc, cplx* terc, cplx* tezk, cplx* terk, int* status) {
+  if (!EXK)
+    eksc<FIRST>(J, g.zp, g.rh, g.rhinv, kTwoPiD, ijx, tezs, ters, tezc, terc, tezk, terk, status);
+  else
+    ekscx<FIRST>(J, g.zp, g.rh, kTwoPiD, ijx, tezs, ters, tezc, terc, tezk, terk, status);
+}
+
 // Fields of one source segment (direct or image) at a displacement:
 // nec_context.cpp:2777-2843.  e[0..8] = (xk,yk,zk, xs,ys,zs, xc,yc,zc).
-// Returns r, the distance used for the far-pair decision.
-template <bool EXK>
-__device__ double efld_compute(const SrcSeg& J, double xij, double yij, double ai,
-                               double salpr, double zij, bool ijx, const FieldParams& P,
-                               cplx e[9], int* status) {
+// Returns r, the distance used for the far-pair decision.  FIRST: a near pair
+// takes the first step of its quadrature only (intx_first).
+template <bool EXK, bool FIRST>
+__device__ __forceinline__ double efld_compute(const SrcSeg& J, double xij, double yij, double ai,
+                                               double salpr, double zij, bool ijx, const FieldParams& P,
+                                               cplx e[9], int* status) {
   const double cabj = J.cab, sabj = J.sab;
   cplx tezs, ters, tezc, terc, tezk, terk;
-  double zp = xij * cabj + yij * sabj + zij * salpr;
-  double rhox = xij - cabj * zp;
-  double rhoy = yij - sabj * zp;
-  double rhoz = zij - salpr * zp;
-  double rh = sqrt(rhox * rhox + rhoy * rhoy + rhoz * rhoz + ai * ai);
-  double r = sqrt(zp * zp + rh * rh);
-  const bool far = r >= P.rkh;
-  // the FP64 divide is the costliest operation of a far pair: 1 / rh for
-  // the three components and, for a far pair, 1 / r come from one
-  // reciprocal of rh r
-  double rinv = 0.0;
-  if (rh <= 1.e-10) {
-    rhox = 0.0;
-    rhoy = 0.0;
-    rhoz = 0.0;
-    if (far) rinv = 1.0 / r;
-  } else {
-    double rhinv;
-    if (far) {
-      const double q = 1.0 / (rh * r);
-      rhinv = r * q;
-      rinv = rh * q;
-    } else {
-      rhinv = 1.0 / rh;
-    }
-    rhox *= rhinv;
-    rhoy *= rhinv;
-    rhoz *= rhinv;
-  }
-  if (far) {
-    // lumped current element, 2798-2819, with the divisions by r, rmag and
-    // py = 2 pi r^2 folded into that reciprocal
-    double rmag = kTwoPiD * r;
-    double cth = zp * rinv;
-    double px = rh * rinv;
-    // exp(-j rmag) as sincospi of r * 2 pi / pi_exact (exact reduction)
-    constexpr double kTwoPiOverPi = kTwoPiD / 3.141592653589793;
-    double sn, cs;
-    sincospi(kTwoPiOverPi * r, &sn, &cs);
-    cplx e0 = mk(cs, -sn);
-    const double rminv = rinv * (1.0 / kTwoPiD);
-    const double pyinv = rminv * rinv;  // 1 / py
-    cplx e1 = (P.eta * cth * pyinv) * e0 * mk(1.0, -rminv);
-    cplx e2 = (0.5 * P.eta * px * pyinv) * e0 * mk(1.0, rmag - rminv);
-    tezk = e1 * cth - e2 * px;
-    terk = e1 * px + e2 * cth;
-    const double sfac = J.sfac;
-    tezc = tezk * sfac;
-    terc = terk * sfac;
-    tezk = tezk * J.s;
-    terk = terk * J.s;
+  const PairGeom g = pair_geometry(J, xij, yij, zij, salpr, ai, P.rkh);
+  if (g.far) {
+    const cplx fz = far_projected(g, 1.0, 0.0, P.eta), fr = far_projected(g, 0.0, 1.0, P.eta);
+    const double sfac = J.ss * (1.0 / kPiD);
+    tezc = fz * sfac;
+    terc = fr * sfac;
+    tezk = fz * J.s;
+    terk = fr * J.s;
     e[3] = mk(0., 0.);
     e[4] = mk(0., 0.);
     e[5] = mk(0., 0.);
   } else {
-    if (!EXK)
-      eksc(J.s, zp, rh, kTwoPiD, ijx, &tezs, &ters, &tezc, &terc, &tezk, &terk, status);
-    else
-      ekscx(J.b, J.s, zp, rh, kTwoPiD, ijx, J.ind1, J.ind2, &tezs, &ters, &tezc, &terc, &tezk,
-            &terk, status);
-    e[3] = tezs * cabj + ters * rhox;
-    e[4] = tezs * sabj + ters * rhoy;
-    e[5] = tezs * salpr + ters * rhoz;
+    near_components<EXK, FIRST>(J, g, ijx, &tezs, &ters, &tezc, &terc, &tezk, &terk, status);
+    e[3] = tezs * cabj + ters * g.rhox;
+    e[4] = tezs * sabj + ters * g.rhoy;
+    e[5] = tezs * salpr + ters * g.rhoz;
   }
-  e[0] = tezk * cabj + terk * rhox;
-  e[1] = tezk * sabj + terk * rhoy;
-  e[2] = tezk * salpr + terk * rhoz;
-  e[6] = tezc * cabj + terc * rhox;
-  e[7] = tezc * sabj + terc * rhoy;
-  e[8] = tezc * salpr + terc * rhoz;
-  return r;
+  e[0] = tezk * cabj + terk * g.rhox;
+  e[1] = tezk * sabj + terk * g.rhoy;
+  e[2] = tezk * salpr + terk * g.rhoz;
+  e[6] = tezc * cabj + terc * g.rhox;
+  e[7] = tezc * sabj + terc * g.rhoy;
+  e[8] = tezc * salpr + terc * g.rhoz;
+  return g.r;
+}
+
+// Reciprocals of the small integers, rounded to nearest.
+struct SmallRecip {
+  double r[202];
+  constexpr SmallRecip() : r() {
+    for (int i = 1; i < 202; i++) r[i] = 1.0 / i;
+  }
+};
+__constant__ SmallRecip kSmallRecip{};
+// v / i for an integer 0 < i < 202: a product with the rounded reciprocal and
+// Markstein's correction, which rounds as the division does.
+__device__ __forceinline__ cplx div_small(cplx v, int i) {
+  const double y = kSmallRecip.r[i], d = i;
+  cplx q = v * y;
+  q.re = fma(fma(-q.re, d, v.re), y, q.re);
+  q.im = fma(fma(-q.im, d, v.im), y, q.im);
+  return q;
 }
 
 // Sommerfeld attenuation function, c_ggrid.cpp:291-350
@@ -438,13 +535,13 @@ __device__ cplx fbar(cplx p) {
   const double tosp = 2.0 / sqrt_pi;
   cplx z = mk(0.0, 1.0) * csqrt_(p);
   if (cabs_(z) <= 3.) {
-    cplx zs = z * z;
+    const cplx zs = z * z;
     cplx sum = z, pw = z;
     for (int i = 1; i <= 100; i++) {
-      pw = -pw * zs / static_cast<double>(i);
-      cplx term = pw / (2. * i + 1.);
+      pw = div_small(-pw * zs, i);
+      const cplx term = div_small(pw, 2 * i + 1);
       sum = sum + term;
-      if (cnorm(term) / cnorm(sum) < 1.E-12) break;
+      if (cnorm(term) < 1.E-12 * cnorm(sum)) break;
     }
     return 1. - (1. - sum * tosp) * z * cexp_(zs) * sqrt_pi;
   }
@@ -535,48 +632,56 @@ __device__ void gwave(double r2, double zph, cplx xx2, cplx u, cplx u2, double e
 
 enum { kGroundNone = 0, kGroundPerfect = 1, kGroundReflection = 2, kGroundSommerfeld = 3 };
 
+// Field of the source's image at observation point i, as efld (2845-2956)
+// subtracts it (before the factor frati).
+template <int GROUND, bool EXK, bool FIRST>
+__device__ __forceinline__ void image_fields9(const SrcSeg& J, double xij, double yij, double zi, double ai,
+                                              const FieldParams& P, cplx e[9], int* status) {
+  const double zij = zi + J.z;
+  double r = efld_compute<EXK, FIRST>(J, xij, yij, ai, -J.salp, zij, true, P, e, status);
+  if (GROUND == kGroundReflection) {
+    // reflection-coefficient approximation, 2893-2944
+    cplx zratx = P.zrati;
+    double xymag = sqrt(xij * xij + yij * yij);
+    double px, py, cth;
+    cplx zrsin;
+    if (xymag <= 1.0e-6) {
+      px = 0.;
+      py = 0.;
+      cth = 1.;
+      zrsin = mk(1., 0.);
+    } else {
+      px = -yij / xymag;
+      py = xij / xymag;
+      cth = zij / r;
+      zrsin = csqrt_(1.0 - zratx * zratx * (1.0 - cth * cth));
+    }
+    cplx refs = (cth - zratx * zrsin) / (cth + zratx * zrsin);
+    cplx refps = -(zratx * cth - zrsin) / (zratx * cth + zrsin);
+    refps = refps - refs;
+#pragma unroll
+    for (int k = 0; k < 9; k += 3) {
+      cplx epy = px * e[k] + py * e[k + 1];
+      cplx epx = px * epy;
+      epy = py * epy;
+      e[k] = refs * e[k] + refps * epx;
+      e[k + 1] = refs * e[k + 1] + refps * epy;
+      e[k + 2] = refs * e[k + 2];
+    }
+  }
+}
+
 // Fields of source J at observation point i, direct plus (for a ground)
 // image: efld (2845-2956) up to the Sommerfeld/Norton part.
 template <int GROUND, bool EXK>
 __device__ __forceinline__ void pair_fields9(const SrcSeg& J, double xi, double yi, double zi, double ai,
                                              bool ij, const FieldParams& P, cplx ex[9], int* status) {
-  cplx e[9];
   const double xij = xi - J.x;
   const double yij = yi - J.y;
-  efld_compute<EXK>(J, xij, yij, ai, J.salp, zi - J.z, ij, P, ex, status);
+  efld_compute<EXK, false>(J, xij, yij, ai, J.salp, zi - J.z, ij, P, ex, status);
   if (GROUND != kGroundNone) {
-    const double zij = zi + J.z;
-    double r = efld_compute<EXK>(J, xij, yij, ai, -J.salp, zij, true, P, e, status);
-    if (GROUND == kGroundReflection) {
-      // reflection-coefficient approximation, 2893-2944
-      cplx zratx = P.zrati;
-      double xymag = sqrt(xij * xij + yij * yij);
-      double px, py, cth;
-      cplx zrsin;
-      if (xymag <= 1.0e-6) {
-        px = 0.;
-        py = 0.;
-        cth = 1.;
-        zrsin = mk(1., 0.);
-      } else {
-        px = -yij / xymag;
-        py = xij / xymag;
-        cth = zij / r;
-        zrsin = csqrt_(1.0 - zratx * zratx * (1.0 - cth * cth));
-      }
-      cplx refs = (cth - zratx * zrsin) / (cth + zratx * zrsin);
-      cplx refps = -(zratx * cth - zrsin) / (zratx * cth + zrsin);
-      refps = refps - refs;
-#pragma unroll
-      for (int k = 0; k < 9; k += 3) {
-        cplx epy = px * e[k] + py * e[k + 1];
-        cplx epx = px * epy;
-        epy = py * epy;
-        e[k] = refs * e[k] + refps * epx;
-        e[k + 1] = refs * e[k + 1] + refps * epy;
-        e[k + 2] = refs * e[k + 2];
-      }
-    }
+    cplx e[9];
+    image_fields9<GROUND, EXK, false>(J, xij, yij, zi, ai, P, e, status);
 #pragma unroll
     for (int k = 0; k < 9; k++) ex[k] -= e[k] * P.frati;
   }
@@ -710,16 +815,41 @@ __device__ __forceinline__ void project_fields(const cplx ex[9], double cabi, do
   *etc = ex[6] * cabi + ex[7] * sabi + ex[8] * salpi;
 }
 
+// Projected fields (etk, ets, etc) of one source (direct, or its image in a
+// perfect ground with salpr = -salp) on an observation segment; false for a
+// far pair, whose one field is returned in *etk (see far_projected).
+template <bool EXK, bool FIRST>
+__device__ __forceinline__ bool projected_fields(const SrcSeg& J, double xij, double yij, double zij, double salpr,
+                                                 double ai, double cabi, double sabi, double salpi, bool ij,
+                                                 const FieldParams& P, cplx* etk, cplx* ets, cplx* etc, int* status) {
+  const PairGeom g = pair_geometry(J, xij, yij, zij, salpr, ai, P.rkh);
+  const double dz = J.cab * cabi + J.sab * sabi + salpr * salpi, dr = g.rhox * cabi + g.rhoy * sabi + g.rhoz * salpi;
+  if (g.far) {
+    *etk = far_projected(g, dz, dr, P.eta);
+    return false;
+  }
+  cplx tezs, ters, tezc, terc, tezk, terk;
+  near_components<EXK, FIRST>(J, g, ij, &tezs, &ters, &tezc, &terc, &tezk, &terk, status);
+  *etk = tezk * dz + terk * dr;
+  *ets = tezs * dz + ters * dr;
+  *etc = tezc * dz + terc * dr;
+  return true;
+}
+
 // Projected fields (etk, ets, etc) of source J on observation segment i:
-// efld (2845-3045) followed by the tangential projection of cmww (2617-2619).
-// For Sommerfeld ground, a pair within the table limit of its image is read
-// from P.near_g at pair_index (obs * n + src) when those fields exist, and
-// is reported (kStatSommerfeldTab) otherwise.
-template <int GROUND, bool EXK>
-__device__ void pair_field(const SrcSeg& J, double xi, double yi, double zi, double ai,
-                           double cabi, double sabi, double salpi, bool ij,
-                           const FieldParams& P, cplx* etk, cplx* ets, cplx* etc,
-                           int* status, int64_t pair_index = -1) {
+// efld (2845-3045) and the tangential projection of cmww (2617-2619).  In
+// free space a far pair returns false and its one field in *etk: etk = s
+// etk, ets = 0, etc = sin(pi s) / pi etk.  For Sommerfeld ground, a pair
+// within the table limit of its image is read from P.near_g at pair_index
+// (obs * n + src) when those fields exist, and is reported
+// (kStatSommerfeldTab) otherwise.  FIRST: a pair whose quadrature needs more
+// than its first step reports kStatDefer and nothing else; pair_field_full
+// evaluates it.
+template <int GROUND, bool EXK, bool FIRST>
+__device__ __forceinline__ bool pair_field(const SrcSeg& J, double xi, double yi, double zi, double ai,
+                                           double cabi, double sabi, double salpi, bool ij,
+                                           const FieldParams& P, cplx* etk, cplx* ets, cplx* etc,
+                                           int* status, int64_t pair_index = -1) {
   const double xij = xi - J.x, yij = yi - J.y;
   double r_img = 0.0;
   if (GROUND == kGroundSommerfeld) {
@@ -729,24 +859,59 @@ __device__ void pair_field(const SrcSeg& J, double xi, double yi, double zi, dou
       *etk = g[0];
       *ets = g[1];
       *etc = g[2];
-      return;
+      return true;
     }
   }
-  cplx ex[9];
-  pair_fields9<GROUND, EXK>(J, xi, yi, zi, ai, ij, P, ex, status);
-  if (GROUND == kGroundSommerfeld) {
+  const bool near =
+      projected_fields<EXK, FIRST>(J, xij, yij, zi - J.z, J.salp, ai, cabi, sabi, salpi, ij, P, etk, ets, etc, status);
+  if (GROUND == kGroundNone) return near;
+  const double sfac = J.ss * (1.0 / kPiD);
+  if (!near) {
+    *etc = *etk * sfac;
+    *ets = mk(0., 0.);
+    *etk = *etk * J.s;
+  }
+  if (FIRST && (*status & kStatDefer)) return true;
+  cplx ik, is, ic;
+  if (GROUND == kGroundPerfect) {
+    if (!projected_fields<EXK, FIRST>(J, xij, yij, zi + J.z, -J.salp, ai, cabi, sabi, salpi, true, P, &ik, &is, &ic,
+                                      status)) {
+      ic = ik * sfac;
+      is = mk(0., 0.);
+      ik = ik * J.s;
+    }
+  } else {
     cplx e[9];
+    image_fields9<GROUND, EXK, FIRST>(J, xij, yij, zi, ai, P, e, status);
+    project_fields(e, cabi, sabi, salpi, &ik, &is, &ic);
+  }
+  if (FIRST && (*status & kStatDefer)) return true;
+  *etk -= ik * P.frati;
+  *ets -= is * P.frati;
+  *etc -= ic * P.frati;
+  if (GROUND == kGroundSommerfeld) {
     if (r_img <= .95) {
       *status |= kStatSommerfeldTab;
-      for (int k = 0; k < 9; k++) e[k] = mk(0., 0.);
     } else {
+      cplx e[9];
       const SommGeom g = somm_geometry(J, xi, yi, zi, ai);
       norton_field(J, g, xij, yij, zi + J.z, r_img, ai, P, e);
+      project_fields(e, cabi, sabi, salpi, &ik, &is, &ic);
+      *etk += ik;
+      *ets += is;
+      *etc += ic;
     }
-#pragma unroll
-    for (int k = 0; k < 9; k++) ex[k] = ex[k] + e[k];
   }
-  project_fields(ex, cabi, sabi, salpi, etk, ets, etc);
+  return true;
+}
+
+// The pairs with interval halvings, a few per observation segment: kept out
+// of line so that they do not set the registers of the others.
+template <int GROUND, bool EXK>
+__device__ __noinline__ void pair_field_full(const SrcSeg& J, const double* obs, bool ij, const FieldParams& P,
+                                             cplx out[3], int* status, int64_t pair_index) {
+  pair_field<GROUND, EXK, false>(J, obs[0], obs[1], obs[2], obs[3], obs[4], obs[5], obs[6], ij, P, &out[0], &out[1],
+                                 &out[2], status, pair_index);
 }
 
 }  // namespace necb

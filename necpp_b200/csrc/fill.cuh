@@ -4,14 +4,26 @@
 // Z is row-major: Z[obs * ld + basis].  The reference fills the same layout
 // (cm[basis + obs*nrow]) by scattering, for each source segment j in turn,
 // etk*ax + ets*bx + etc*cx into the <= jsno basis columns that have support
-// on j.  Here the scatter is turned into a gather that needs no atomics:
-// one CTA owns a tile of TI observation rows x TB basis columns.  The host
-// lists, per column tile, the distinct source segments that contribute to
-// any of its columns (ascending), and for each such source the (column,
-// a, b, c) entries.  Each thread (one observation row) walks that list,
-// computes the source's fields once, and accumulates into its row of a
-// shared-memory tile.  Because sources are visited in ascending order, every
-// element is summed in exactly the reference's order.
+// on j.  Here the scatter is turned into a gather that needs no atomics.  A
+// CTA owns a few rows of a block of basis columns and works in two phases:
+// its threads evaluate the fields of the block's source segments on those
+// rows, a pair each, into shared memory; then a thread per column combines
+// the fields of the column's sources in ascending order, so every element is
+// summed in exactly the reference's order and written in whole rows.
+//
+// The pairs of a CTA are independent, and within a warp they take one path:
+// the closed form of a far pair, or the first step of a near pair's adaptive
+// quadrature.  The few near pairs whose quadrature goes on (neighbours on the
+// wire, dozens of points each) are queued in shared memory and evaluated
+// after the others, a thread each.  A far pair is stored as one field (its
+// constant and cosine currents differ by a factor of the source).
+//
+// Bound by instruction issue (FP64 a third of the instructions) and, below a
+// few hundred segments, by one pair's latency.  One thread per row walking
+// the sources of 16 columns, as the fill did before, made every warp wait for
+// each of its rows' neighbours in turn: 288 us for a dipole of 51 segments
+// (now 18), 4.2 ms for the wire mesh of 3,280 (2.1), 3.5 ms for the helix
+// array of 11,520 (2.45: 54 G pairs/s), 13.6 ms for 1,024 Yagis (5.9).
 #pragma once
 #include <cstdint>
 
@@ -19,24 +31,51 @@
 
 namespace necb {
 
-constexpr int kFillTI = 64;  // observation rows per CTA (= threads)
-constexpr int kFillTB = 16;  // basis columns per CTA
+constexpr int kFillMaxRows = 8;    // rows per CTA
+constexpr int kFillBlock = 124;    // most columns of a block (junctions apart, see fill_block_cols)
+constexpr int kFillPairs = 1050;   // pairs staged per CTA, four CTAs per SM
+constexpr int kFillPairsBig = 3360;  // one CTA per SM
+constexpr int kFillThreads = 128;
+constexpr int kFillThreadsBig = 512;
+// Dynamic shared memory of a CTA that stages `rows` x `chunk` pairs: the
+// projected fields (three complex, or a far pair's one) and the queue, and
+// per source its length and sin(pi s) / pi and its rows' kinds.
+constexpr size_t fill_smem(int rows, int chunk) {
+  return (size_t)rows * chunk * (3 * sizeof(double2) + sizeof(uint16_t)) + (size_t)chunk * (sizeof(double2) + 1);
+}
+// Free space with the thin-wire kernel runs in 128 registers (four CTAs of
+// 128 threads per SM, or one of 512); the ground and extended-kernel fields
+// take up to 255 (two of 128).
+template <int GROUND, bool EXK>
+constexpr int fill_max_threads() {
+  return GROUND == kGroundNone && !EXK ? kFillThreadsBig : kFillThreads;
+}
 
 struct FillArgs {
   int64_t n, ld;
   // segments (wavelengths)
   const double *x, *y, *z, *s, *b, *cab, *sab, *salp;
   const int32_t *ind1, *ind2;
-  // column-tile source lists
-  const int32_t* tile_src_ptr;  // [ntiles+1] into tsrc
-  const int32_t* tsrc;          // source segment (0-based)
-  const int32_t* tsrc_eptr;     // [len(tsrc)+1] into entries
-  const uint8_t* ecol;          // column within tile
-  const double *ea, *eb, *ec;   // basis coefficients
+  // column blocks of `cols` basis columns: the distinct sources of a block
+  // (ascending) and, per column, its entries by ascending source
+  int cols;
+  const int32_t* blk_ptr;  // [nblocks+1] into src
+  const int32_t* src;      // source segment (0-based)
+  const int32_t* col_ptr;  // [n+1] into the entries
+  const int32_t* eloc;     // an entry's source, as an index into its block's list
+  const double *ea, *eb, *ec;  // basis coefficients
   FieldParams P;
   double2* Z64;  // row-major FP64 output (may be null)
   float2* Z32;   // row-major FP32 copy (mixed precision; may be null)
   int* status;
+};
+
+// How a structure is cut into CTAs (fill_plan in engine.cu).
+struct FillPlan {
+  int cols;     // basis columns per block
+  int rows;     // rows per CTA
+  int chunk;    // sources staged at once
+  int threads;
 };
 
 // Contraction instead of storage (adjoint gradients): out[k] +=
@@ -49,129 +88,194 @@ struct ContractArgs {
 };
 constexpr int kMaxContract = 4;
 
-// One tile of Z: rows [row0, row0+64) x basis columns of column tile `tile`.
-// CONTRACT = false stores the tile (Z64 / Z32); true folds it into C.out.
-template <int GROUND, bool EXK, bool CONTRACT>
-__device__ __forceinline__ void fill_tile(const FillArgs& A, const ContractArgs& C, int tile, int64_t row0) {
-  __shared__ double2 acc[kFillTB][kFillTI + 1];
-  const int tid = threadIdx.x;
-  const int64_t i = row0 + tid;
-  const bool active = i < A.n;
-#pragma unroll
-  for (int c = 0; c < kFillTB; c++) acc[c][tid] = make_double2(0.0, 0.0);
+template <bool EXK>
+__device__ __forceinline__ SrcSeg fill_source(const FillArgs& A, int j) {
+  SrcSeg J;
+  J.x = __ldg(A.x + j);
+  J.y = __ldg(A.y + j);
+  J.z = __ldg(A.z + j);
+  J.s = __ldg(A.s + j);
+  J.b = __ldg(A.b + j);
+  J.cab = __ldg(A.cab + j);
+  J.sab = __ldg(A.sab + j);
+  J.salp = __ldg(A.salp + j);
+  J.ind1 = EXK ? __ldg(A.ind1 + j) : 0;
+  J.ind2 = EXK ? __ldg(A.ind2 + j) : 0;
+  set_half_length(J);
+  return J;
+}
 
-  double xi = 0, yi = 0, zi = 0, ai = 0, cabi = 0, sabi = 0, salpi = 0;
-  if (active) {
-    xi = A.x[i];
-    yi = A.y[i];
-    zi = A.z[i];
-    ai = A.b[i];
-    cabi = A.cab[i];
-    sabi = A.sab[i];
-    salpi = A.salp[i];
+// Rows [row0, row0 + rows) of column block `blk`, `chunk` sources at a time
+// (one chunk unless a block has more sources than shared memory holds; the
+// sums are then carried in Z64).  CONTRACT = false stores the rows (Z64 /
+// Z32); true folds them into C.out.
+template <int GROUND, bool EXK, bool CONTRACT>
+__device__ __forceinline__ void fill_rows(const FillArgs& A, const ContractArgs& C, int blk, int64_t row0, int rows,
+                                          int chunk) {
+  extern __shared__ double2 fill_fields[];
+  __shared__ double obs[kFillMaxRows][8];
+  __shared__ int nhard;
+  double2* F = fill_fields;
+  double2* len = F + 3 * rows * chunk;  // per source: s, sin(pi s) / pi
+  uint16_t* hard = reinterpret_cast<uint16_t*>(len + chunk);
+  uint8_t* near_rows = reinterpret_cast<uint8_t*>(hard + rows * chunk);  // per source: bit r set, row r is near
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int nr = (int)min((int64_t)rows, A.n - row0);
+  if (tid < 8 * nr) {
+    const int k = tid & 7;
+    const double* p = k == 0 ? A.x : k == 1 ? A.y : k == 2 ? A.z : k == 3 ? A.b : k == 4 ? A.cab : k == 5 ? A.sab : A.salp;
+    obs[tid >> 3][k] = p[row0 + (tid >> 3)];
   }
+  const int sbeg = A.blk_ptr[blk], send = A.blk_ptr[blk + 1];
+  const int64_t col0 = (int64_t)blk * A.cols;
+  const int ncols = (int)min((int64_t)A.cols, A.n - col0);
   int status = 0;
-  const int sbeg = A.tile_src_ptr[tile], send = A.tile_src_ptr[tile + 1];
-  // the far-pair factor sin(pi s)/pi of the tile's sources, computed once per
-  // source by the CTA in chunks of kFillTI instead of once per pair
-  __shared__ double sfac[kFillTI];
-  for (int sidx = sbeg; sidx < send; sidx++) {
-    if ((sidx - sbeg) % kFillTI == 0) {
-      __syncthreads();  // the previous chunk's factors are no longer read
-      const int q = sidx + tid;
-      if (q < send) sfac[tid] = far_sfac(__ldg(A.s + __ldg(A.tsrc + q)));
-      __syncthreads();
+  for (int s0 = sbeg; s0 < send || s0 == sbeg; s0 += chunk) {
+    const int cnt = max(0, min(chunk, send - s0));
+    if (s0 > sbeg) __syncthreads();  // the previous chunk's fields are no longer read
+    if (tid == 0) nhard = 0;
+    __syncthreads();
+    for (int q = tid; q < cnt; q += nt) {
+      const int j = __ldg(A.src + s0 + q);
+      const SrcSeg J = fill_source<EXK>(A, j);
+      if (GROUND == kGroundNone) len[q] = make_double2(J.s, J.ss * (1.0 / kPiD));
+      unsigned near = 0;
+      // one pair by the general path
+      auto general = [&](int r) {
+        const int64_t i = row0 + r;
+        cplx etk, ets, etc;
+        int st = 0;
+        if (pair_field<GROUND, EXK, true>(J, obs[r][0], obs[r][1], obs[r][2], obs[r][3], obs[r][4], obs[r][5],
+                                          obs[r][6], i != j, A.P, &etk, &ets, &etc, &st, i * A.n + j))
+          near |= 1u << r;
+        double2* f = F + 3 * (r * chunk + q);
+        if (st & kStatDefer) {
+          hard[atomicAdd(&nhard, 1)] = (uint16_t)(r * chunk + q);
+          return;
+        }
+        status |= st;
+        f[0] = make_double2(etk.re, etk.im);
+        if (near >> r & 1) {
+          f[1] = make_double2(ets.re, ets.im);
+          f[2] = make_double2(etc.re, etc.im);
+        }
+      };
+      int r = 0;
+      if (GROUND == kGroundNone) {
+        // far pairs two rows at a time, for their independent chains
+#pragma unroll 1
+        for (; r + 1 < nr; r += 2) {
+          const double *o = obs[r], *p = obs[r + 1];
+          const PairGeom g = pair_geometry(J, o[0] - J.x, o[1] - J.y, o[2] - J.z, J.salp, o[3], A.P.rkh);
+          const PairGeom h = pair_geometry(J, p[0] - J.x, p[1] - J.y, p[2] - J.z, J.salp, p[3], A.P.rkh);
+          if (!g.far || !h.far) break;
+          const cplx u = far_projected(g, J.cab * o[4] + J.sab * o[5] + J.salp * o[6],
+                                       g.rhox * o[4] + g.rhoy * o[5] + g.rhoz * o[6], A.P.eta);
+          const cplx v = far_projected(h, J.cab * p[4] + J.sab * p[5] + J.salp * p[6],
+                                       h.rhox * p[4] + h.rhoy * p[5] + h.rhoz * p[6], A.P.eta);
+          F[3 * (r * chunk + q)] = make_double2(u.re, u.im);
+          F[3 * ((r + 1) * chunk + q)] = make_double2(v.re, v.im);
+        }
+      }
+      // from the first near pair on (or every row): one at a time
+#pragma unroll 1
+      for (; r < nr; r++) general(r);
+      if (GROUND == kGroundNone) near_rows[q] = (uint8_t)near;
     }
-    const int j = __ldg(A.tsrc + sidx);
-    SrcSeg J;
-    J.sfac = sfac[(sidx - sbeg) % kFillTI];
-    J.x = __ldg(A.x + j);
-    J.y = __ldg(A.y + j);
-    J.z = __ldg(A.z + j);
-    J.s = __ldg(A.s + j);
-    J.b = __ldg(A.b + j);
-    J.cab = __ldg(A.cab + j);
-    J.sab = __ldg(A.sab + j);
-    J.salp = __ldg(A.salp + j);
-    J.ind1 = EXK ? __ldg(A.ind1 + j) : 0;
-    J.ind2 = EXK ? __ldg(A.ind2 + j) : 0;
-    if (!active) continue;
-    cplx etk, ets, etc;
-    pair_field<GROUND, EXK>(J, xi, yi, zi, ai, cabi, sabi, salpi, i != j, A.P, &etk, &ets, &etc,
-                            &status, i * A.n + j);
-    const int e0 = __ldg(A.tsrc_eptr + sidx), e1 = __ldg(A.tsrc_eptr + sidx + 1);
-    for (int e = e0; e < e1; e++) {
-      const int c = A.ecol[e];
-      const double a = __ldg(A.ea + e), bb = __ldg(A.eb + e), cc = __ldg(A.ec + e);
-      cplx v = etk * a + ets * bb + etc * cc;
-      double2 t = acc[c][tid];
-      t.x += v.re;
-      t.y += v.im;
-      acc[c][tid] = t;
+    __syncthreads();
+    for (int h = tid; h < nhard; h += nt) {
+      const int code = hard[h], r = code / chunk, q = code - r * chunk;
+      const int j = __ldg(A.src + s0 + q);
+      const int64_t i = row0 + r;
+      const SrcSeg J = fill_source<EXK>(A, j);
+      cplx out[3];
+      pair_field_full<GROUND, EXK>(J, obs[r], i != j, A.P, out, &status, i * A.n + j);
+      double2* f = F + 3 * code;
+      f[0] = make_double2(out[0].re, out[0].im);
+      f[1] = make_double2(out[1].re, out[1].im);
+      f[2] = make_double2(out[2].re, out[2].im);
+    }
+    __syncthreads();
+    double tr[kFillMaxRows], ti[kFillMaxRows];  // CONTRACT: the rows' sums over this thread's columns
+#pragma unroll
+    for (int r = 0; r < kFillMaxRows; r++) tr[r] = ti[r] = 0.0;
+    for (int c = tid; c < ncols; c += nt) {
+      const int64_t col = col0 + c;
+      const int e0 = __ldg(A.col_ptr + col), e1 = __ldg(A.col_ptr + col + 1);
+      cplx acc[kFillMaxRows];
+#pragma unroll
+      for (int r = 0; r < kFillMaxRows; r++) {
+        acc[r] = mk(0.0, 0.0);
+        if (!CONTRACT && s0 > sbeg && r < nr) {
+          const double2 z = A.Z64[(row0 + r) * A.ld + col];
+          acc[r] = mk(z.x, z.y);
+        }
+      }
+      for (int e = e0; e < e1; e++) {
+        const int q = __ldg(A.eloc + e) - (s0 - sbeg);
+        if ((unsigned)q >= (unsigned)cnt) continue;
+        const double a = __ldg(A.ea + e), bb = __ldg(A.eb + e), cc = __ldg(A.ec + e);
+        // a far pair's constant and cosine currents share one field
+        const double w = GROUND == kGroundNone ? a * len[q].x + cc * len[q].y : 0.0;
+        const unsigned near = GROUND == kGroundNone ? near_rows[q] : ~0u;
+#pragma unroll
+        for (int r = 0; r < kFillMaxRows; r++)
+          if (r < nr) {
+            const double2* f = F + 3 * (r * chunk + q);
+            if (near >> r & 1)
+              acc[r] += mk(f[0].x, f[0].y) * a + mk(f[1].x, f[1].y) * bb + mk(f[2].x, f[2].y) * cc;
+            else
+              acc[r] += mk(f[0].x, f[0].y) * w;
+          }
+      }
+#pragma unroll
+      for (int r = 0; r < kFillMaxRows; r++)
+        if (r < nr) {
+          if (CONTRACT) {
+            const double2 xv = C.x[col];
+            tr[r] += acc[r].re * xv.x - acc[r].im * xv.y;
+            ti[r] += acc[r].re * xv.y + acc[r].im * xv.x;
+          } else {
+            const int64_t at = (row0 + r) * A.ld + col;
+            if (A.Z64) A.Z64[at] = make_double2(acc[r].re, acc[r].im);
+            if (A.Z32 && s0 + chunk >= send) A.Z32[at] = make_float2((float)acc[r].re, (float)acc[r].im);
+          }
+        }
+    }
+    if (CONTRACT) {
+      // row i: t = sum_c Z[i][c] x[c]; out[k] += w_k[i] t, a warp at a time
+#pragma unroll
+      for (int r = 0; r < kFillMaxRows; r++)
+        if (r < nr) {
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) {
+            tr[r] += __shfl_down_sync(0xffffffffu, tr[r], off);
+            ti[r] += __shfl_down_sync(0xffffffffu, ti[r], off);
+          }
+          if ((tid & 31) == 0)
+            for (int k = 0; k < C.nw; k++) {
+              const double2 wv = C.w[(int64_t)k * A.n + row0 + r];
+              atomicAdd(C.out + 2 * k, wv.x * tr[r] - wv.y * ti[r]);
+              atomicAdd(C.out + 2 * k + 1, wv.x * ti[r] + wv.y * tr[r]);
+            }
+        }
     }
   }
   if (status) atomicOr(A.status, status);
-  __syncthreads();
-  const int lane = tid & 31, warp = tid >> 5;
-  if (CONTRACT) {
-    // row i: t = sum_c Z[i][col0+c] x[col0+c]; out[k] += w_k[i] t
-    double tr = 0, ti = 0;
-    if (active) {
-      const int64_t col0 = (int64_t)tile * kFillTB;
-      for (int c = 0; c < kFillTB && col0 + c < A.n; c++) {
-        const double2 z = acc[c][tid], xv = C.x[col0 + c];
-        tr += z.x * xv.x - z.y * xv.y;
-        ti += z.x * xv.y + z.y * xv.x;
-      }
-    }
-    for (int k = 0; k < C.nw; k++) {
-      double pr = 0, pi = 0;
-      if (active) {
-        const double2 wv = C.w[(int64_t)k * A.n + i];
-        pr = wv.x * tr - wv.y * ti;
-        pi = wv.x * ti + wv.y * tr;
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        pr += __shfl_down_sync(0xffffffffu, pr, off);
-        pi += __shfl_down_sync(0xffffffffu, pi, off);
-      }
-      if (lane == 0) {
-        atomicAdd(C.out + 2 * k, pr);
-        atomicAdd(C.out + 2 * k + 1, pi);
-      }
-    }
-    return;
-  }
-  // write out: consecutive threads along a row's (contiguous) columns
-  (void)lane;
-  (void)warp;
-  const int64_t col0 = (int64_t)tile * kFillTB;
-  for (int e = tid; e < kFillTI * kFillTB; e += kFillTI) {
-    const int r = e / kFillTB, c = e % kFillTB;
-    const int64_t row = row0 + r, col = col0 + c;
-    if (row < A.n && col < A.n) {
-      const double2 v = acc[c][r];
-      if (A.Z64) A.Z64[row * A.ld + col] = v;
-      if (A.Z32) A.Z32[row * A.ld + col] = make_float2((float)v.x, (float)v.y);
-    }
-  }
 }
 
-// Free space: registers capped so that eight 64-thread CTAs fit an SM (the
-// fill is latency-bound at six); the ground variants keep their registers
-// (their larger field code spills at the cap).
 template <int GROUND, bool EXK>
-__global__ void __launch_bounds__(kFillTI, GROUND == 0 ? 8 : 1) fill_kernel(FillArgs A) {
-  fill_tile<GROUND, EXK, false>(A, ContractArgs{}, blockIdx.y, (int64_t)blockIdx.x * kFillTI);
+__global__ void __launch_bounds__(fill_max_threads<GROUND, EXK>()) fill_kernel(const __grid_constant__ FillArgs A, int rows,
+                                                                                       int chunk) {
+  fill_rows<GROUND, EXK, false>(A, ContractArgs{}, blockIdx.y, (int64_t)blockIdx.x * rows, rows, chunk);
 }
 
 // Batched fill of perturbed structures (blockIdx.z), each contracted with
 // its own output slot: out_s[k] = w_k^T Z_s x.
 template <int GROUND, bool EXK>
-__global__ void __launch_bounds__(kFillTI) fill_contract_kernel(const FillArgs* __restrict__ As,
-                                                                const ContractArgs* __restrict__ Cs) {
-  fill_tile<GROUND, EXK, true>(As[blockIdx.z], Cs[blockIdx.z], blockIdx.y, (int64_t)blockIdx.x * kFillTI);
+__global__ void __launch_bounds__(fill_max_threads<GROUND, EXK>())
+    fill_contract_kernel(const FillArgs* __restrict__ As, const ContractArgs* __restrict__ Cs, int rows, int chunk) {
+  fill_rows<GROUND, EXK, true>(As[blockIdx.z], Cs[blockIdx.z], blockIdx.y, (int64_t)blockIdx.x * rows, rows, chunk);
 }
 
 }  // namespace necb

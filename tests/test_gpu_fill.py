@@ -1,0 +1,88 @@
+"""The fill's cut into CTAs (column blocks, rows per CTA, staged chunks) at
+the edges of its blocks, against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GROUNDS = {"free": None, "perfect": (1, 0, 0, 0, 0, 0, 0, 0), "reflection": (0, 0, 13.0, 0.005, 0, 0, 0, 0),
+           "sommerfeld": (2, 0, 13.0, 0.005, 0, 0, 0, 0)}
+
+
+@pytest.fixture(scope="module")
+def engine(nb):
+    from gpu_helpers import Engine
+    e = Engine(nb.lib)
+    yield e
+    e.close()
+
+
+def wire(nb, n, ground="free", extended=False, length=4.0):
+    """Structure tables of a straight wire of n segments and `length`
+    wavelengths: self, near and far pairs."""
+    ctx = nb.nec_create()
+    assert nb.nec_wire(ctx, 1, n, 0.3, -0.5 * length, 2.0, 0.1, 0.5 * length, 2.5, 1e-3, 1.0, 1.0) == 0
+    assert nb.nec_geometry_complete(ctx, 0) == 0
+    if extended:
+        assert nb.nec_ek_card(ctx, 0) == 0
+    if GROUNDS[ground]:
+        assert nb.nec_gn_card(ctx, *GROUNDS[ground]) == 0
+    st = nb.structure(ctx, 299.8)
+    nb.nec_delete(ctx)
+    return st
+
+
+# one block and two (124 columns), whole and partial; with 613 segments also
+# several rows per CTA, the last CTA's incomplete
+@pytest.mark.parametrize("n,ground,extended", [
+    (2, "free", False), (3, "free", True), (63, "free", False), (64, "perfect", False), (65, "reflection", False),
+    (124, "free", False), (125, "free", False), (125, "free", True), (125, "perfect", True),
+    (127, "sommerfeld", False), (129, "reflection", True), (248, "free", False), (249, "perfect", False),
+    (613, "free", False), (613, "perfect", False)])
+def test_fill_at_block_edges(nb, oracle, engine, n, ground, extended):
+    """Element-wise to 1e-12 of max|Z|, the fill's tolerance."""
+    st = wire(nb, n, ground, extended)
+    Zo, _ = oracle.fill(st)
+    engine.set_structure(st, tables=False)  # no pair is near its image
+    engine.fill()
+    assert np.max(np.abs(engine.copy_z() - Zo)) <= 1e-12 * np.max(np.abs(Zo))
+
+
+def test_fill_of_a_block_in_chunks(nb, engine):
+    """A column block whose sources exceed the shared memory is summed in
+    chunks carried through the matrix.  Tables with one entry per segment
+    give Z0; entries of every segment on basis 7 as well must add up Z0's
+    columns there (4 chunks of rounding each: 1e-13 of the largest sum) and
+    leave the rest as it was."""
+    n = 3400
+    ctx = nb.nec_create()
+    assert nb.nec_wire(ctx, 1, n, 0.0, 0.0, 0.0, 0.0, 0.0, 40.0, 1e-4, 1.0, 1.0) == 0
+    assert nb.nec_geometry_complete(ctx, 0) == 0
+    st = nb.structure(ctx, 299.8)
+    nb.nec_delete(ctx)
+    rng = np.random.default_rng(5)
+    abc = rng.uniform(0.5, 1.5, (n, 3))
+
+    def tables(extra):
+        ptr, basis, coef = [0], [], []
+        for j in range(n):
+            for c in ([j, 7] if extra and j != 7 else [j]):
+                basis.append(c)
+                coef.append(abc[j])
+            ptr.append(len(basis))
+        t = dict(st)
+        t["tptr"] = np.array(ptr, dtype=np.int32)
+        t["tbasis"] = np.array(basis, dtype=np.int32)
+        t["tabc"] = np.ascontiguousarray(np.array(coef).T.ravel())
+        return t
+
+    out = []
+    for extra in (False, True):
+        engine.set_structure(tables(extra))
+        engine.fill()
+        out.append(engine.copy_z())
+    z0, z1 = out
+    total = z0.sum(axis=1)
+    assert np.max(np.abs(z1[:, 7] - total)) <= 1e-13 * np.sum(np.abs(z0), axis=1).max()
+    z0[:, 7] = z1[:, 7] = 0
+    assert np.max(np.abs(z1 - z0)) <= 1e-15 * np.max(np.abs(z0))
