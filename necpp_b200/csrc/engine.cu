@@ -583,14 +583,14 @@ int launch_fill_t(necgpu_engine* e, const FillArgs& a) {
 // Sommerfeld ground: evaluations that read the tables through the
 // interpolation cache, in the reference's order over `nunits` units (source
 // columns of the fill, or field points).  Every unit is first evaluated from
-// a fresh cache, one thread per unit.  A unit's result depends on the cache
+// a fresh cache, all units at once.  A unit's result depends on the cache
 // it starts from only when its first table point falls below the cached
 // patch's grid and the cached cell passes the reuse test; a host scan over
 // the units in order finds those whose true starting cache (the one the
 // previous unit leaves, the first unit starting from the cache the engine
 // holds) differs from the one used, and only they are evaluated again from
 // it.  The scan repeats until every unit is consistent; after a bounded
-// number of rounds the rest is walked by one thread in order.  The cache
+// number of rounds the rest is walked by one CTA in order.  The cache
 // left at the end is kept, with its coefficients, for the next evaluation.
 // launch(entry, units, count, chain) runs the kernel; d_rec holds one
 // NearRecord per unit.
@@ -627,7 +627,7 @@ int resolve_cache_order(necgpu_engine* e, int64_t nunits, NearRecord* d_rec, Lau
     e->stats.near_passes = round + 1;
     if (ndirty == 0) {
       if (t.igrs != kInterpFresh && !t.carry)
-        KLAUNCH(NECGPU_K_FILL, 0.0, interp_store_kernel<<<1, 1, 0, e->stream>>>(t, e->d_somm, e->d_interp_carry));
+        KLAUNCH(NECGPU_K_FILL, 0.0, interp_store_kernel<<<1, 16, 0, e->stream>>>(t, e->d_somm, e->d_interp_carry));
       if (t.igrs != kInterpFresh) t.carry = 1;
       e->interp_key = t;
       return 0;
@@ -645,7 +645,9 @@ int resolve_cache_order(necgpu_engine* e, int64_t nunits, NearRecord* d_rec, Lau
 }
 
 // Near-ground pairs of the fill (pairs within the table limit of their
-// image), one unit per source column in the reference's order (cmset).
+// image) in the reference's order (cmset): a unit is one of `parts` runs of
+// `chunks` x 16 observation points of a source column (at most 16 per column,
+// so that the host's scan stays short against the pairs' work).
 template <bool X>
 int run_near_ground(necgpu_engine* e, const FillArgs& a) {
   const int64_t n = e->n;
@@ -656,22 +658,24 @@ int run_near_ground(necgpu_engine* e, const FillArgs& a) {
     TRY(dalloc(e, e->d_near_g, (size_t)n * n * 3));
     e->near_g_cap = n * n * 3;
   }
-  if (e->near_cap < n) {
-    TRY(dalloc(e, e->d_near_rec, (size_t)n));
-    e->near_cap = n;
+  const int64_t runs = (n + kNearGroundPairs - 1) / kNearGroundPairs;
+  const int chunks = (int)((runs + 15) / 16), parts = (int)((runs + chunks - 1) / chunks);
+  const int64_t nunits = n * parts;
+  if (e->near_cap < nunits) {
+    TRY(dalloc(e, e->d_near_rec, (size_t)nunits));
+    e->near_cap = nunits;
   }
-  auto launch = [&](const std::vector<InterpKey>& entry, const std::vector<int>& cols, int ncols,
+  auto launch = [&](const std::vector<InterpKey>& entry, const std::vector<int>& units, int count,
                     int chain) -> int {
-    TRY(upload(e, e->d_near_entry, entry.data(), (size_t)n));
-    TRY(upload(e, e->d_near_cols, cols.data(), (size_t)ncols));
-    const unsigned blocks = chain ? 1u : (unsigned)((ncols + 63) / 64);
+    TRY(upload(e, e->d_near_entry, entry.data(), (size_t)nunits));
+    TRY(upload(e, e->d_near_cols, units.data(), (size_t)count));
     KLAUNCH(NECGPU_K_FILL, 0.0,
-            near_ground_kernel<X><<<blocks, chain ? 1 : 64, 0, e->stream>>>(
-                a, e->d_somm, e->d_near_cols, ncols, e->d_near_entry, e->d_interp_carry, e->d_near_rec,
+            near_ground_kernel<X><<<chain ? 1u : (unsigned)count, kNearThreads, 0, e->stream>>>(
+                a, e->d_somm, e->d_near_cols, count, parts, chunks, e->d_near_entry, e->d_interp_carry, e->d_near_rec,
                 e->d_near_g, chain));
     return 0;
   };
-  return resolve_cache_order(e, n, e->d_near_rec, launch);
+  return resolve_cache_order(e, nunits, e->d_near_rec, launch);
 }
 
 int run_fill(necgpu_engine* e, bool want64, bool want32) {
@@ -2913,14 +2917,14 @@ int necgpu_near_field(necgpu_engine* e, int magnetic, int npts, const double* pt
                           int chain) -> int {
           TRY(upload(e, d_entry, entry.data(), (size_t)npts));
           TRY(upload(e, d_units, units.data(), (size_t)count));
-          const unsigned nb = chain ? 1u : (unsigned)((count + 63) / 64);
+          const unsigned nb = chain ? 1u : (unsigned)count;
           if (x)
             KLAUNCH(NECGPU_K_PATTERN, 0.0,
-                    near_field_chain_kernel<true><<<nb, chain ? 1 : 64, 0, e->stream>>>(
+                    near_field_chain_kernel<true><<<nb, kNearThreads, 0, e->stream>>>(
                         a, d_ax, e->d_somm, d_units, count, d_entry, e->d_interp_carry, d_rec, d_near, chain));
           else
             KLAUNCH(NECGPU_K_PATTERN, 0.0,
-                    near_field_chain_kernel<false><<<nb, chain ? 1 : 64, 0, e->stream>>>(
+                    near_field_chain_kernel<false><<<nb, kNearThreads, 0, e->stream>>>(
                         a, d_ax, e->d_somm, d_units, count, d_entry, e->d_interp_carry, d_rec, d_near, chain));
           return 0;
         };

@@ -128,59 +128,57 @@ __global__ void __launch_bounds__(32 * kNearWarps) near_e_kernel(NearFieldArgs A
 }
 
 // Sommerfeld ground: the (point, segment) pairs within the table limit, in
-// the reference's order (points in turn, segments ascending), one thread
-// per listed point from the cache `entry[p]`, or (chain) one thread over
-// all listed points in order.  Sums into near[3 * p].
+// the reference's order (points in turn, segments ascending), one CTA per
+// listed point from the cache `entry[p]`, or (chain) one CTA over all listed
+// points in order.  Sums into near[3 * p].  0.22 ms for 135 points and 31
+// segments (2.0 ms with a thread per point).
 template <bool EXK>
-__global__ void __launch_bounds__(64) near_field_chain_kernel(NearFieldArgs A, const double* __restrict__ axs,
-                                                              const cplx* __restrict__ tab,
-                                                              const int* __restrict__ units, int nunits,
-                                                              const InterpKey* __restrict__ entry,
-                                                              const InterpCache* __restrict__ carried,
-                                                              NearRecord* __restrict__ rec, double2* __restrict__ near,
-                                                              int chain) {
-  int k0, k1;
-  if (chain) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    k0 = 0;
-    k1 = nunits;
-  } else {
-    k0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k0 >= nunits) return;
-    k1 = k0 + 1;
-  }
-  InterpCache S;
+__global__ void __launch_bounds__(kNearThreads)
+    near_field_chain_kernel(const __grid_constant__ NearFieldArgs A, const double* __restrict__ axs,
+                            const cplx* __restrict__ tab, const int* __restrict__ units, int nunits,
+                            const InterpKey* __restrict__ entry, const InterpCache* __restrict__ carried,
+                            NearRecord* __restrict__ rec, double2* __restrict__ near, int chain) {
+  __shared__ NearShared<kNearFieldPairs> S;
+  const int k0 = chain ? 0 : blockIdx.x, k1 = chain ? nunits : k0 + 1;
   InterpKey key = entry[units[k0]];
-  interp_restore(S, key, tab, carried);
   int status = 0;
   for (int k = k0; k < k1; k++) {
-    const int p = units[k];
-    const double xob = A.pts[3 * p], yob = A.pts[3 * p + 1], zob = A.pts[3 * p + 2], ax = axs[p];
-    NearRecord r;
-    r.has_near = 0;
-    r.used = key;
-    r.x1 = r.y1 = 0.0;
-    cplx f[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};
-    for (int64_t i = 0; i < A.n; i++) {
-      const SrcSeg J = load_seg(A, i, EXK);
-      if (image_r2(xob - J.x, yob - J.y, zob + J.z) > .95) continue;
-      double2 s1;
-      cplx e[9];
-      near_efld9<EXK>(J, xob, yob, zob, ax, true, A.P, A.n, S, tab, r.has_near ? nullptr : &s1, e, &status);
-      if (!r.has_near) {
-        r.has_near = 1;
-        r.x1 = s1.x;
-        r.y1 = s1.y;
+    const int u = units[k];
+    const double xob = A.pts[3 * u], yob = A.pts[3 * u + 1], zob = A.pts[3 * u + 2], ax = axs[u];
+    NearUnit unit;
+    unit.start(key);
+    cplx f[3] = {mk(0, 0), mk(0, 0), mk(0, 0)};  // warp 0: segment i0 + lane of every chunk
+    for (int64_t i0 = 0; i0 < A.n; i0 += kNearFieldPairs) {
+      const int count = (int)min((int64_t)kNearFieldPairs, A.n - i0);
+      key = near_chunk<EXK>(
+          S, count, key, A.P, A.n, carried, tab,
+          [&](int p, SrcSeg& J, double* o, bool& ij) {
+            J = near_source<EXK>(A.x, A.y, A.z, A.s, A.b, A.cab, A.sab, A.salp, A.ind1, A.ind2, i0 + p);
+            o[0] = xob;
+            o[1] = yob;
+            o[2] = zob;
+            o[3] = ax;
+            ij = true;
+            return image_r2(xob - J.x, yob - J.y, zob + J.z) <= .95;
+          },
+          &status);
+      const int p = threadIdx.x;
+      if (p < count && S.near[p]) {
+        const int64_t i = i0 + p;
+        const cplx ac = coef(A.abc, A.n, i, 0), bc = coef(A.abc, A.n, i, 1), cc = coef(A.abc, A.n, i, 2);
+        for (int c = 0; c < 3; c++)
+          f[c] += (S.base[p][c] + S.rom[p][c]) * ac + (S.base[p][c + 3] + S.rom[p][c + 3]) * bc +
+                  (S.base[p][c + 6] + S.rom[p][c + 6]) * cc;
       }
-      const cplx ac = coef(A.abc, A.n, i, 0), bc = coef(A.abc, A.n, i, 1), cc = coef(A.abc, A.n, i, 2);
-      f[0] += e[0] * ac + e[3] * bc + e[6] * cc;
-      f[1] += e[1] * ac + e[4] * bc + e[7] * cc;
-      f[2] += e[2] * ac + e[5] * bc + e[8] * cc;
+      if (threadIdx.x == 0) unit.chunk(S, count);
     }
-    for (int c = 0; c < 3; c++) near[3 * p + c] = make_double2(f[c].re, f[c].im);
-    key = InterpKey{S.igrs, S.ix, S.iy, S.carry};
-    r.exit = key;
-    rec[p] = r;
+    if (threadIdx.x < 32) {
+      warp_sum3(f);
+      if (threadIdx.x == 0)
+        for (int c = 0; c < 3; c++) near[3 * u + c] = make_double2(f[c].re, f[c].im);
+    }
+    unit.r.exit = key;
+    if (threadIdx.x == 0) rec[u] = unit.r;
   }
   if (status) atomicOr(A.status, status);
 }

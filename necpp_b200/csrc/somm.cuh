@@ -689,10 +689,10 @@ struct InterpKey {
   int igrs, ix, iy, carry;
 };
 
+// Coefficients of a patch (the carried cache; within a fill they are formed
+// from the tables as a point is evaluated).
 struct InterpCache {
-  int igrs, ix, iy, ixs, iys, ixeg, iyeg, nxm2, nym2, nxms, nyms, nd, ndp;
-  int carry;  // coefficients come from a previous fill's tables
-  double dx, dy, xs, ys, xz, yz;
+  double dx, dy, xz, yz;
   cplx a[4][4], b[4][4], c[4][4], d[4][4];
 };
 
@@ -725,116 +725,78 @@ __host__ __device__ inline bool interp_reuses(InterpKey k, double x, double y) {
   return (k.ix >= ixeg && k.iy >= iyeg) && (abs(k.ix - ixs) < 2 && abs(k.iy - iys) < 2);
 }
 
-__device__ void interp_coefficients(InterpCache& s, const cplx* tables) {
-  const cplx* ar = tables + somm_off(s.igrs);
-  int iadz = s.ixs + (s.iys - 3) * s.nd - s.ndp;
-  for (int k = 0; k < 4; k++) {
-    iadz += s.ndp;
-    int iadd = iadz;
+// The cell a recomputation at (x, y) leaves.
+__device__ __forceinline__ InterpKey interp_point_key(double x, double y) {
+  InterpKey k;
+  k.igrs = x <= somm_xs(1) ? 0 : (y > somm_ys(2) ? 2 : 1);
+  k.ix = (int)((x - somm_xs(k.igrs)) / somm_dx(k.igrs)) + 1;
+  k.iy = (int)((y - somm_ys(k.igrs)) / somm_dy(k.igrs)) + 1;
+  k.carry = 0;
+  return k;
+}
+
+// The cache's cell after point (x, y) met it as `k`, from which the point is
+// read: unchanged when the cached patch serves it (c_ggrid::interpolate,
+// c_ggrid.cpp:44-98).
+__device__ InterpKey interp_next(InterpKey k, double x, double y) {
+  const bool fresh = k.igrs == kInterpFresh;
+  const int g = fresh ? 0 : k.igrs;
+  const double xs = fresh ? 0.0 : somm_xs(g), ys = fresh ? 0.0 : somm_ys(g);
+  if (x >= xs && y >= ys) {
+    k.ix = (int)((x - xs) / (fresh ? 1.0 : somm_dx(g))) + 1;
+    k.iy = (int)((y - ys) / (fresh ? 1.0 : somm_dy(g))) + 1;
+  } else {
+    int ixs = -10, iys = -10, ixeg = 0, iyeg = 0;  // c_ggrid::initialize
+    if (!fresh) interp_cell(g, k.ix, k.iy, &ixs, &iys, &ixeg, &iyeg);
+    if (k.ix >= ixeg && k.iy >= iyeg && abs(k.ix - ixs) < 2 && abs(k.iy - iys) < 2) return k;
+  }
+  const InterpKey p = interp_point_key(x, y);
+  if (p.igrs != k.igrs) k = p;
+  k.carry = 0;
+  return k;
+}
+
+// Cubic through four table values, as coefficients.
+__device__ __forceinline__ void interp_cubic(const cplx* t, cplx* a, cplx* b, cplx* c, cplx* d) {
+  const cplx p1 = t[0], p2 = t[1], p3 = t[2], p4 = t[3];
+  *a = (p4 - p1 + 3.0 * (p2 - p3)) * 0.1666666667;
+  *b = (p1 - 2.0 * p2 + p3) * 0.5;
+  *c = p3 - (2.0 * p1 + 3.0 * p2 + p4) * 0.1666666667;
+  *d = p2;
+}
+
+// The four functions at (x, y) from the patch of cell `k`: from the tables,
+// or (k.carry) from the carried cache's coefficients.
+__device__ void interp_value(InterpKey k, const cplx* tables, const InterpCache* carried, double x, double y,
+                             cplx f[4]) {
+  const int g = k.igrs, nd = somm_nx(g), ndp = nd * somm_ny(g);
+  int ixs, iys, ixeg, iyeg;
+  interp_cell(g, k.ix, k.iy, &ixs, &iys, &ixeg, &iyeg);
+  const double dx = k.carry ? carried->dx : somm_dx(g), dy = k.carry ? carried->dy : somm_dy(g);
+  const double xz = k.carry ? carried->xz : (ixs - 1) * dx + somm_xs(g);
+  const double yz = k.carry ? carried->yz : (iys - 1) * dy + somm_ys(g);
+  const double xx = (x - xz) / dx, yy = (y - yz) / dy;
+  const cplx* ar = tables + somm_off(g) + ixs + (iys - 2) * nd - 2;
+#pragma unroll 1
+  for (int q = 0; q < 4; q++) {
+    cplx fx[4];
+#pragma unroll
     for (int i = 0; i < 4; i++) {
-      iadd += s.nd;
-      const cplx p1 = ar[iadd - 2], p2 = ar[iadd - 1], p3 = ar[iadd], p4 = ar[iadd + 1];
-      s.a[i][k] = (p4 - p1 + 3.0 * (p2 - p3)) * 0.1666666667;
-      s.b[i][k] = (p1 - 2.0 * p2 + p3) * 0.5;
-      s.c[i][k] = p3 - (2.0 * p1 + 3.0 * p2 + p4) * 0.1666666667;
-      s.d[i][k] = p2;
+      cplx a, b, c, d;
+      if (k.carry) {
+        a = carried->a[i][q];
+        b = carried->b[i][q];
+        c = carried->c[i][q];
+        d = carried->d[i][q];
+      } else {
+        interp_cubic(ar + q * ndp + i * nd, &a, &b, &c, &d);
+      }
+      fx[i] = ((a * xx + b) * xx + c) * xx + d;
     }
-  }
-  s.xz = (s.ixs - 1) * s.dx + s.xs;
-  s.yz = (s.iys - 1) * s.dy + s.ys;
-}
-
-__device__ void interp_set_grid(InterpCache& s, int igr) {
-  s.igrs = igr;
-  s.dx = somm_dx(igr);
-  s.dy = somm_dy(igr);
-  s.xs = somm_xs(igr);
-  s.ys = somm_ys(igr);
-  s.nxm2 = somm_nx(igr) - 2;
-  s.nym2 = somm_ny(igr) - 2;
-  s.nxms = ((s.nxm2 + 1) / 3) * 3 + 1;
-  s.nyms = ((s.nym2 + 1) / 3) * 3 + 1;
-  s.nd = somm_nx(igr);
-  s.ndp = somm_nx(igr) * somm_ny(igr);
-}
-
-// Rebuild a cache from its key (c_ggrid::initialize for a fresh one) with
-// coefficients from `tables`, or take the carried cache.
-__device__ void interp_restore(InterpCache& s, InterpKey k, const cplx* tables, const InterpCache* carried) {
-  s.carry = 0;
-  if (k.igrs != kInterpFresh && k.carry) {
-    s = *carried;
-    s.carry = 1;
-    return;
-  }
-  if (k.igrs == kInterpFresh) {
-    s.ixs = -10;
-    s.iys = -10;
-    s.igrs = kInterpFresh;
-    s.ixeg = 0;
-    s.iyeg = 0;
-    s.dx = 1.0;
-    s.dy = 1.0;
-    s.xs = 0.0;
-    s.ys = 0.0;
-    s.ix = 0;
-    s.iy = 0;
-    return;
-  }
-  interp_set_grid(s, k.igrs);
-  s.ix = k.ix;
-  s.iy = k.iy;
-  interp_cell(k.igrs, k.ix, k.iy, &s.ixs, &s.iys, &s.ixeg, &s.iyeg);
-  interp_coefficients(s, tables);
-}
-
-// c_ggrid::interpolate: the four functions at R = x, theta = y
-__device__ void interp_eval(InterpCache& s, const cplx* tables, double x, double y, cplx f[4]) {
-  bool recalc = true;
-  if ((x >= s.xs) && (y >= s.ys)) {
-    s.ix = (int)((x - s.xs) / s.dx) + 1;
-    s.iy = (int)((y - s.ys) / s.dy) + 1;
-  } else if (((s.ix >= s.ixeg) && (s.iy >= s.iyeg)) && ((abs(s.ix - s.ixs) < 2) && (abs(s.iy - s.iys) < 2))) {
-    recalc = false;
-  }
-  if (recalc) {
-    int igr;
-    if (x <= somm_xs(1))
-      igr = 0;
-    else
-      igr = (y > somm_ys(2)) ? 2 : 1;
-    if (igr != s.igrs) {
-      interp_set_grid(s, igr);
-      s.ix = (int)((x - s.xs) / s.dx) + 1;
-      s.iy = (int)((y - s.ys) / s.dy) + 1;
-    }
-    s.ixs = ((s.ix - 1) / 3) * 3 + 2;
-    if (s.ixs < 2) s.ixs = 2;
-    s.ixeg = -10000;
-    if (s.ixs > s.nxm2) {
-      s.ixs = s.nxm2;
-      s.ixeg = s.nxms;
-    }
-    s.iys = ((s.iy - 1) / 3) * 3 + 2;
-    if (s.iys < 2) s.iys = 2;
-    s.iyeg = -10000;
-    if (s.iys > s.nym2) {
-      s.iys = s.nym2;
-      s.iyeg = s.nyms;
-    }
-    interp_coefficients(s, tables);
-    s.carry = 0;
-  }
-  const double xx = (x - s.xz) / s.dx, yy = (y - s.yz) / s.dy;
-  for (int k = 0; k < 4; k++) {
-    cplx fx1 = ((s.a[0][k] * xx + s.b[0][k]) * xx + s.c[0][k]) * xx + s.d[0][k];
-    cplx fx2 = ((s.a[1][k] * xx + s.b[1][k]) * xx + s.c[1][k]) * xx + s.d[1][k];
-    cplx fx3 = ((s.a[2][k] * xx + s.b[2][k]) * xx + s.c[2][k]) * xx + s.d[2][k];
-    cplx fx4 = ((s.a[3][k] * xx + s.b[3][k]) * xx + s.c[3][k]) * xx + s.d[3][k];
-    cplx p1 = fx4 - fx1 + 3.0 * (fx2 - fx3);
-    cplx p2 = 3.0 * (fx1 - 2.0 * fx2 + fx3);
-    cplx p3 = 6.0 * fx3 - 2.0 * fx1 - 3.0 * fx2 - fx4;
-    f[k] = ((p1 * yy + p2) * yy + p3) * yy * 0.1666666667 + fx2;
+    const cplx p1 = fx[3] - fx[0] + 3.0 * (fx[1] - fx[2]);
+    const cplx p2 = 3.0 * (fx[0] - 2.0 * fx[1] + fx[2]);
+    const cplx p3 = 6.0 * fx[2] - 2.0 * fx[0] - 3.0 * fx[1] - fx[3];
+    f[q] = ((p1 * yy + p2) * yy + p3) * yy * 0.1666666667 + fx[1];
   }
 }
 
@@ -845,12 +807,21 @@ struct NearSrc {
   SommGeom g;
 };
 
+// One point of the integration over the source: the table field of a current
+// element at t from the source's centre, sin and cos of 2 pi t, the table
+// point (R, theta) it reads and the cell it was read from.
+struct NearPt {
+  cplx e[3];
+  double st, ct, x, y;
+  InterpKey key;
+};
+
 // sflds, isnor = 1 (6024-6066, 6108-6137): field due to ground of a
 // current element at t from the source centre, from the tables.  The
 // positions that steer the interpolation are rounded as the reference
-// rounds them.  `first` (if set) receives the point (R, theta).
-__device__ void sflds_table(const NearSrc& N, double t, InterpCache& S, const cplx* tab, cplx e[9],
-                            double2* first) {
+// rounds them.  key: the cache the point meets.
+__device__ __noinline__ void sflds_table(const NearSrc& N, double t, InterpKey key, const InterpCache* carried,
+                                         const cplx* tab, NearPt& out) {
   const SommGeom& g = N.g;
   const double xt = __dadd_rn(N.xj, __dmul_rn(t, N.cabj));
   const double yt = __dadd_rn(N.yj, __dmul_rn(t, N.sabj));
@@ -881,25 +852,20 @@ __device__ void sflds_table(const NearSrc& N, double t, InterpCache& S, const cp
   double sr, cr;
   sincos(rk, &sr, &cr);
   const double thet = (rho >= 1.0e-12) ? atan(zph / rho) : kPiD / 2.0;
-  if (first) *first = make_double2(r2, thet);
+  out.x = r2;
+  out.y = thet;
+  out.key = interp_next(key, r2, thet);
   cplx f[4];
-  interp_eval(S, tab, r2, thet, f);
+  interp_value(out.key, tab, carried, r2, thet, f);
   const cplx xx2 = mk(cr, -sr) / r2;
   const double sfac = g.sn * cph;
   const cplx erh = xx2 * (N.salpj * f[0] + sfac * f[2]);
   const cplx ezh = xx2 * (N.salpj * f[1] - sfac * f[0]);
   const cplx eph = g.sn * sph * xx2 * f[3];
-  e[0] = erh * rhx + eph * phx;
-  e[1] = erh * rhy + eph * phy;
-  e[2] = ezh;
-  double st, ct;
-  sincos(kTwoPiD * t, &st, &ct);
-  e[3] = e[0] * st;
-  e[4] = e[1] * st;
-  e[5] = e[2] * st;
-  e[6] = e[0] * ct;
-  e[7] = e[1] * ct;
-  e[8] = e[2] * ct;
+  out.e[0] = erh * rhx + eph * phx;
+  out.e[1] = erh * rhy + eph * phy;
+  out.e[2] = ezh;
+  sincos(kTwoPiD * t, &out.st, &out.ct);
 }
 
 __device__ __forceinline__ double test_simple(double f1r, double f2r, double dmin) {
@@ -909,210 +875,414 @@ __device__ __forceinline__ double test_simple(double f1r, double f2r, double dmi
   return fabs((f1r - f2r) / den);
 }
 
-// rom2, 5589-5834: Romberg integration of the table field over [a, b]; the
-// finest step is (b - a) / nseg (nseg: segments of the structure).
-__device__ void rom2_table(const NearSrc& N, double a, double b, cplx sum[9], double dmin, int64_t nseg,
-                           InterpCache& S, const cplx* tab, double2* first, int* status) {
-  const int n = 9, nts = 4, nx = 1;
+// A CTA's work area: NP pairs at a time whose near-ground fields its warps
+// integrate.
+constexpr int kNearWarpsG = 8, kNearThreads = 32 * kNearWarpsG;
+constexpr int kNearGroundPairs = 16;  // per unit of the fill (CTAs of several units fill the device)
+constexpr int kNearFieldPairs = 32;   // of a field point, whose segments follow one another in one unit
+// window of points: halvings of the first step, steps that follow it as it
+// is, and steps that follow it halved once (2 + 2 x 5 + 4 x 2 + 4 x 3 = 32)
+constexpr int kNearLevels = 5, kNearMarch = 2, kNearMarchHalf = 3;
+template <int NP>
+struct NearShared {
+  NearPt win[kNearWarpsG][32];
+  cplx base[NP][9], rom[NP][9];  // direct and image fields; the table field's integrals
+  double dmin[NP], x1[NP], y1[NP];
+  InterpKey used[NP], exit[NP];
+  int near[NP], dirty[NP];
+  InterpKey last;
+  int ndirty;
+};
+
+// rom2, 5589-5834, by one warp: Romberg integration of the table field over
+// [a, b] through the cache `key` (left as the integration leaves it); the
+// finest step is (b - a) / nseg (nseg: segments of the structure).  Component
+// c (x, y, z of the constant, sine and cosine currents) of the integral on
+// lane c < 9.
+//
+// The points follow one another in the reference's order and rounding, but
+// which ones are needed depends on the convergence tests.  The lanes evaluate
+// a window ahead: the first step's points and those of its next halvings, and
+// the points of the next steps of its size, each from a recomputed patch
+// (which is what a point meets unless it lies below the grid of the cell
+// before it: interp_next decides as the points are taken in order, and such a
+// point is evaluated again from the cached patch).
+__device__ void rom2_warp(const NearSrc& N, double a, double b, double dmin, int64_t nseg, InterpKey& key,
+                          const InterpCache* carried, const cplx* tab, NearPt* win, cplx* sum_out, double* x1,
+                          double* y1, int* status) {
+  const int lane = threadIdx.x & 31, nts = 4, nx = 1;
+  const int c = lane < 9 ? lane : 8;
   const double rx = 1e-4;
-  double z = a, dz = 0.0, dzot = 0.0;
   const double ze = b, s = b - a;
-  cplx g1[9], g2[9], g3[9], g4[9], g5[9], t01[9], t10[9], t20[9];
-  const double ep = s / (1.0e4 * (double)nseg);
-  const double zend = ze - ep;
-  for (int i = 0; i < n; i++) sum[i] = mk(0, 0);
+  const double ep = s / (1.0e4 * (double)nseg), zend = ze - ep;
+  double z = a, dz = 0.0, dzot = 0.0;
+  cplx g1, g2, g3, g4, g5, sum = mk(0, 0);
   int64_t ns = nx;
   int nt = 0;
-  sflds_table(N, z, S, tab, g1, first);
+  // window: `at` the step that z stands at (0 the first, then the steps ahead,
+  // of size wdz), run: whether those steps follow the first one as it is (0)
+  // or halved (1); level: halvings of the first step so far
+  double wdz = 0.0;
+  int at = -1, run = 0, level = 0;
+  auto open = [&]() {
+    // lanes 0, 1: z + dz/2, z + dz; 2 q + 2, + 3: the quarter points of the
+    // first step halved q times; then four points for each of the steps that
+    // follow it, and of those that follow it halved once
+    double t = z;
+    if (lane < 2) {
+      t = __dadd_rn(z, lane == 0 ? dz * .5 : dz);
+    } else if (lane < 2 + 2 * kNearLevels) {
+      const int q = (lane - 2) >> 1;
+      const double d = q == 0 ? dz : s / (double)(ns << q);
+      t = __dadd_rn(z, __dmul_rn(d, (lane & 1) ? .75 : .25));
+    } else {
+      const int l = lane - 2 - 2 * kNearLevels, h = l >= 4 * kNearMarch, m = (l >> 2) - h * kNearMarch, p = l & 3;
+      const double d = h ? s / (double)(ns << 1) : dz;
+      double zm = z;
+      for (int k = 0; k <= m; k++) zm = __dadd_rn(zm, d);
+      t = __dadd_rn(zm, p == 0 ? d * .5 : p == 1 ? d : __dmul_rn(d, p == 2 ? .25 : .75));
+    }
+    __syncwarp();
+    sflds_table(N, t, key, carried, tab, win[lane]);
+    __syncwarp();
+    wdz = dz;
+    at = 0;
+    run = 0;
+    level = 0;
+  };
+  auto component = [&](const NearPt& p) {
+    const cplx e = p.e[c % 3];
+    return c < 3 ? e : e * (c < 6 ? p.st : p.ct);
+  };
+  // the window's point l taken in order through the cache
+  auto take = [&](int l, double t) {
+    const NearPt& w = win[l];
+    const InterpKey k = interp_next(key, w.x, w.y);
+    if (k.igrs == w.key.igrs && k.ix == w.key.ix && k.iy == w.key.iy && k.carry == w.key.carry) {
+      key = k;
+      return component(w);
+    }
+    NearPt p;
+    sflds_table(N, t, key, carried, tab, p);
+    key = p.key;
+    return component(p);
+  };
+  auto march = [&](int m, int p) { return 2 + 2 * kNearLevels + 4 * (m - 1 + (run ? kNearMarch : 0)) + p; };
+  // tmag of the first three components (test_simple's arguments)
+  auto magnitude = [&](cplx v) {
+    const double q = cnorm(v);
+    return sqrt(__shfl_sync(0xffffffffu, q, 0) + __shfl_sync(0xffffffffu, q, 1) + __shfl_sync(0xffffffffu, q, 2));
+  };
+  dz = s / (double)ns;
+  if (__dadd_rn(z, dz) >= ze) dz = ze - z;
+  {
+    // the first point by itself: its place in the order is before the window's
+    NearPt p;
+    sflds_table(N, z, key, carried, tab, p);
+    *x1 = p.x;
+    *y1 = p.y;
+    key = p.key;
+    g1 = component(p);
+  }
+  open();
   // every accepted step advances z by at least s / nseg
-  for (int64_t guard = 0; guard < 4 * nseg + 64; guard++) {
+  for (int64_t guard = 0;; guard++) {
+    if (guard >= 4 * nseg + 64) {
+      *status |= kStatIterCap;
+      break;
+    }
     dz = s / (double)ns;
     if (__dadd_rn(z, dz) >= ze) {
       dz = ze - z;
-      if (dz <= ep) return;
+      if (dz <= ep) break;
     }
     dzot = dz * .5;
-    sflds_table(N, __dadd_rn(z, dzot), S, tab, g3, nullptr);
-    sflds_table(N, __dadd_rn(z, dz), S, tab, g5, nullptr);
+    if (at < 0 || at > (run ? kNearMarchHalf : kNearMarch) || dz != wdz || level > 0) open();
+    g3 = take(at ? march(at, 0) : 0, __dadd_rn(z, dzot));
+    g5 = take(at ? march(at, 1) : 1, __dadd_rn(z, dz));
     bool five = false;
+    cplx t10, t20 = mk(0, 0);
     for (;;) {
-      for (int i = 0; i < n; i++) {
-        const cplx t00 = (g1[i] + g5[i]) * dzot;
-        t01[i] = (t00 + dz * g3[i]) * 0.5;
-        t10[i] = (4.0 * t01[i] - t00) / 3.;
+      const cplx t00 = (g1 + g5) * dzot;
+      const cplx t01 = (t00 + dz * g3) * 0.5;
+      t10 = (4.0 * t01 - t00) / 3.;
+      if (test_simple(magnitude(t01), magnitude(t10), dmin) <= rx) break;
+      const double ta = __dadd_rn(z, __dmul_rn(dz, .25)), tb = __dadd_rn(z, __dmul_rn(dz, .75));
+      int la, lb;
+      if (at == 0 && level < kNearLevels) {
+        la = 2 + 2 * level;
+        lb = la + 1;
+      } else if (at > 0 && level == 0) {
+        la = march(at, 2);
+        lb = march(at, 3);
+      } else {  // a step ahead, or one halved past the window: a new window at its size
+        open();
+        la = 2;
+        lb = 3;
       }
-      double tmag1 = sqrt(cnorm(t01[0]) + cnorm(t01[1]) + cnorm(t01[2]));
-      double tmag2 = sqrt(cnorm(t10[0]) + cnorm(t10[1]) + cnorm(t10[2]));
-      if (test_simple(tmag1, tmag2, dmin) <= rx) {
-        for (int i = 0; i < n; i++) sum[i] += t10[i];
-        nt += 2;
-        break;
-      }
-      sflds_table(N, __dadd_rn(z, __dmul_rn(dz, .25)), S, tab, g2, nullptr);
-      sflds_table(N, __dadd_rn(z, __dmul_rn(dz, .75)), S, tab, g4, nullptr);
-      cplx t11[9];
-      for (int i = 0; i < n; i++) {
-        const cplx t02 = (t01[i] + dzot * (g2[i] + g4[i])) * 0.5;
-        t11[i] = (4.0 * t02 - t01[i]) / 3.0;
-        t20[i] = (16. * t11[i] - t10[i]) / 15.0;
-      }
-      tmag1 = sqrt(cnorm(t11[0]) + cnorm(t11[1]) + cnorm(t11[2]));
-      tmag2 = sqrt(cnorm(t20[0]) + cnorm(t20[1]) + cnorm(t20[2]));
-      if (test_simple(tmag1, tmag2, dmin) <= rx) {
-        five = true;
-        break;
-      }
+      g2 = take(la, ta);
+      g4 = take(lb, tb);
+      const cplx t02 = (t01 + dzot * (g2 + g4)) * 0.5;
+      const cplx t11 = (4.0 * t02 - t01) / 3.0;
+      t20 = (16. * t11 - t10) / 15.0;
+      five = true;
+      if (test_simple(magnitude(t11), magnitude(t20), dmin) <= rx) break;
       nt = 0;
       if (ns >= nseg) {
         *status |= kStatRombergCap;
-        five = true;
         break;
       }
+      five = false;
       ns = ns * 2;
       dz = s / (double)ns;
       dzot = dz * .5;
-      for (int i = 0; i < n; i++) {
-        g5[i] = g3[i];
-        g3[i] = g2[i];
-      }
+      level++;
+      g5 = g3;
+      g3 = g2;
     }
     if (five) {
-      for (int i = 0; i < n; i++) sum[i] += t20[i];
+      sum += t20;
       nt = nt + 1;
+    } else {
+      sum += t10;
+      nt += 2;
     }
-    z = z + dz;
-    if (z > zend) return;
-    for (int i = 0; i < n; i++) g1[i] = g5[i];
+    z = __dadd_rn(z, dz);
+    if (z > zend) break;
+    // the window goes on with the steps of this size, if it has them
+    if (at == 0 && level == 1) {
+      run = 1;
+      wdz = dz;
+      at = 1;
+    } else {
+      at = level == 0 ? at + 1 : -1;
+    }
+    level = 0;
+    g1 = g5;
     if ((nt >= nts) && (ns > nx)) {
       ns = ns / 2;
       nt = 1;
     }
   }
-  *status |= kStatIterCap;
+  if (lane < 9) sum_out[lane] = sum;
 }
 
-// Fields of source J at a point within the table limit of J's image:
-// direct and image fields plus the table field integrated over the source
-// (efld, 2993-3001).
-template <bool EXK>
-__device__ void near_efld9(const SrcSeg& J, double xi, double yi, double zi, double ai, bool ij,
-                           const FieldParams& P, int64_t nseg, InterpCache& S, const cplx* tab, double2* first,
-                           cplx ex[9], int* status) {
-  pair_fields9<kGroundSommerfeld, EXK>(J, xi, yi, zi, ai, ij, P, ex, status);
-  double dmin = cnorm(ex[0]) + cnorm(ex[1]) + cnorm(ex[2]);
-  dmin = 0.01 * sqrt(dmin);
-  NearSrc N;
-  N.xj = J.x;
-  N.yj = J.y;
-  N.zj = J.z;
-  N.cabj = J.cab;
-  N.sabj = J.sab;
-  N.salpj = J.salp;
-  N.g = somm_geometry(J, xi, yi, zi, ai);
-  const double shaf = 0.5 * J.s;
-  cplx e[9];
-  rom2_table(N, -shaf, shaf, e, dmin, nseg, S, tab, first, status);
-#pragma unroll
-  for (int k = 0; k < 9; k++) ex[k] = ex[k] + e[k];
+// Fields (direct, image, and the table field integrated over the source) of
+// up to NP pairs in the reference's order, from the cache `t`: pair(p, ...)
+// gives the source, the observation point and radius, whether they are
+// distinct segments, and whether the pair is within the table limit of its
+// image (efld, 2993-3001).  Each pair's integration reads the tables through
+// the cache the previous one left; every pair is first integrated from a
+// fresh cache, a warp each, and those that turn out to start from another
+// cache that they would reuse are integrated again, until all are consistent
+// (the first of them is final after every round).  Results in S.base + S.rom
+// of the pairs with S.near; returns the cache left.
+template <bool EXK, int NP, class Pair>
+__device__ InterpKey near_chunk(NearShared<NP>& S, int count, InterpKey t, const FieldParams& P, int64_t nseg,
+                                const InterpCache* carried, const cplx* tab, Pair pair, int* status) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const InterpKey fresh{kInterpFresh, 0, 0, 0};
+  __syncthreads();  // the previous chunk's results have been read
+  {
+    const int p = w + kNearWarpsG * lane;
+    if (lane < NP / kNearWarpsG) {
+      bool near = false, ij = true;
+      SrcSeg J;
+      double o[4];
+      if (p < count) near = pair(p, J, o, ij);
+      S.near[p] = near;
+      S.dirty[p] = near;
+      S.used[p] = fresh;
+      if (near) {
+        cplx ex[9];
+        pair_fields9<kGroundSommerfeld, EXK>(J, o[0], o[1], o[2], o[3], ij, P, ex, status);
+        double dmin = cnorm(ex[0]) + cnorm(ex[1]) + cnorm(ex[2]);
+        S.dmin[p] = 0.01 * sqrt(dmin);
+        for (int k = 0; k < 9; k++) S.base[p][k] = ex[k];
+      }
+    }
+  }
+  __syncwarp();
+  for (int round = 0; round <= NP; round++) {
+    for (int p = w; p < count; p += kNearWarpsG) {
+      if (!S.dirty[p]) continue;
+      SrcSeg J;
+      double o[4];
+      bool ij;
+      pair(p, J, o, ij);
+      NearSrc N;
+      N.xj = J.x;
+      N.yj = J.y;
+      N.zj = J.z;
+      N.cabj = J.cab;
+      N.sabj = J.sab;
+      N.salpj = J.salp;
+      N.g = somm_geometry(J, o[0], o[1], o[2], o[3]);
+      const double shaf = 0.5 * J.s;
+      InterpKey key = S.used[p];
+      double x1, y1;
+      rom2_warp(N, -shaf, shaf, S.dmin[p], nseg, key, carried, tab, S.win[w], S.rom[p], &x1, &y1, status);
+      if (lane == 0) {
+        S.exit[p] = key;
+        S.x1[p] = x1;
+        S.y1[p] = y1;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      InterpKey k = t;
+      S.ndirty = 0;
+      for (int p = 0; p < count; p++) {
+        S.dirty[p] = 0;
+        if (!S.near[p]) continue;
+        const InterpKey need = interp_reuses(k, S.x1[p], S.y1[p]) ? k : fresh;
+        const InterpKey u = S.used[p];
+        const bool same = need.igrs == u.igrs &&
+                          (need.igrs == kInterpFresh || (need.ix == u.ix && need.iy == u.iy && need.carry == u.carry));
+        if (same) {
+          k = S.exit[p];
+        } else {
+          // most pairs that begin below a cached grid stay below it
+          S.used[p] = need;
+          S.dirty[p] = 1;
+          S.ndirty++;
+          k = need.igrs == kInterpFresh ? S.exit[p] : need;
+        }
+      }
+      S.last = k;
+    }
+    __syncthreads();
+    if (S.ndirty == 0) return S.last;
+  }
+  *status |= kStatIterCap;  // not reached: a round settles at least one pair
+  return t;
 }
 
-// One near-ground pair of the fill, projected (cmww 2617-2619).
-template <bool EXK>
-__device__ void near_pair(const SrcSeg& J, double xi, double yi, double zi, double ai, double cabi, double sabi,
-                          double salpi, bool ij, const FieldParams& P, int64_t nseg, InterpCache& S,
-                          const cplx* tab, double2* first, cplx out[3], int* status) {
-  cplx ex[9];
-  near_efld9<EXK>(J, xi, yi, zi, ai, ij, P, nseg, S, tab, first, ex, status);
-  project_fields(ex, cabi, sabi, salpi, &out[0], &out[1], &out[2]);
-}
-
-// Per source column j: whether it has near pairs, the cache it was
-// computed from, the cache it leaves, and the first table point it reads.
+// A unit of the near-ground evaluations: whether it has near pairs, the cache
+// it was computed from, the cache it leaves, and the first table point it
+// reads.
 struct NearRecord {
   int has_near;
   InterpKey used, exit;
   double x1, y1;
 };
 
-// The near-ground pairs of the listed source columns.  The reference fills
-// source by source (cmset, 2077-2204) and, per source, observation points in
-// order; each pair's integration reads the tables through the cache left by
-// the previous pair.  One thread follows that order down one column from
-// the cache `entry[j]`; with `chain` set a single thread walks all listed
-// columns in order, each starting from the cache the previous one left.
-// Writes the projected fields of every near pair to G[(i * n + j) * 3 + k].
-template <bool EXK>
-__global__ void __launch_bounds__(64) near_ground_kernel(FillArgs A, const cplx* __restrict__ tab,
-                                                         const int* __restrict__ cols, int ncols,
-                                                         const InterpKey* __restrict__ entry,
-                                                         const InterpCache* __restrict__ carried,
-                                                         NearRecord* __restrict__ rec, cplx* __restrict__ G,
-                                                         int chain) {
-  int k0, k1;
-  if (chain) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    k0 = 0;
-    k1 = ncols;
-  } else {
-    k0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k0 >= ncols) return;
-    k1 = k0 + 1;
-  }
-  const int64_t n = A.n;
-  InterpCache S;
-  InterpKey key = entry[cols[k0]];
-  interp_restore(S, key, tab, carried);
-  int status = 0;
-  for (int k = k0; k < k1; k++) {
-    const int j = cols[k];
-    NearRecord r;
+// One unit's record from its chunks (thread 0).
+struct NearUnit {
+  NearRecord r;
+  __device__ void start(InterpKey key) {
     r.has_near = 0;
     r.used = key;
     r.x1 = r.y1 = 0.0;
-    SrcSeg J;
-    J.x = A.x[j];
-    J.y = A.y[j];
-    J.z = A.z[j];
-    J.s = A.s[j];
-    J.b = A.b[j];
-    J.cab = A.cab[j];
-    J.sab = A.sab[j];
-    J.salp = A.salp[j];
-    J.ind1 = EXK ? A.ind1[j] : 0;
-    J.ind2 = EXK ? A.ind2[j] : 0;
-    set_half_length(J);
-    for (int64_t i = 0; i < n; i++) {
-      const double xi = A.x[i], yi = A.y[i], zi = A.z[i];
-      if (image_r2(xi - J.x, yi - J.y, zi + J.z) > .95) continue;
-      double2 s1;
-      cplx out[3];
-      near_pair<EXK>(J, xi, yi, zi, A.b[i], A.cab[i], A.sab[i], A.salp[i], i != j, A.P, n, S, tab,
-                     r.has_near ? nullptr : &s1, out, &status);
-      if (!r.has_near) {
+  }
+  template <int NP>
+  __device__ void chunk(const NearShared<NP>& S, int count) {
+    for (int p = 0; p < count && !r.has_near; p++)
+      if (S.near[p]) {
         r.has_near = 1;
-        r.x1 = s1.x;
-        r.y1 = s1.y;
+        r.x1 = S.x1[p];
+        r.y1 = S.y1[p];
       }
-      cplx* o = G + (i * n + j) * 3;
-      o[0] = out[0];
-      o[1] = out[1];
-      o[2] = out[2];
+  }
+};
+
+template <bool EXK>
+__device__ __forceinline__ SrcSeg near_source(const double* x, const double* y, const double* z, const double* s,
+                                              const double* b, const double* cab, const double* sab,
+                                              const double* salp, const int32_t* ind1, const int32_t* ind2, int64_t j) {
+  SrcSeg J;
+  J.x = x[j];
+  J.y = y[j];
+  J.z = z[j];
+  J.s = s[j];
+  J.b = b[j];
+  J.cab = cab[j];
+  J.sab = sab[j];
+  J.salp = salp[j];
+  J.ind1 = EXK ? ind1[j] : 0;
+  J.ind2 = EXK ? ind2[j] : 0;
+  set_half_length(J);
+  return J;
+}
+
+// The near-ground pairs of the listed units: unit u is the part u % parts of
+// the observation points (in 16s) of source column u / parts.  The reference
+// fills source by source (cmset, 2077-2204) and, per source, observation
+// points in order; each pair's integration reads the tables through the cache
+// left by the previous pair.  One CTA takes a unit from the cache `entry[u]`;
+// with `chain` set one CTA walks all listed units in order, each starting
+// from the cache the previous one left.  Writes the projected fields of every
+// near pair to G[(i * n + j) * 3 + k].
+//
+// Latency-bound: a pair is a chain of up to 150 table evaluations between
+// convergence tests.  With a thread per column walking its pairs one by one
+// the kernel took 2.4 ms for 31 segments; with a warp per pair and a window
+// of points ahead it takes 0.16 ms.
+template <bool EXK>
+__global__ void __launch_bounds__(kNearThreads)
+    near_ground_kernel(const __grid_constant__ FillArgs A, const cplx* __restrict__ tab, const int* __restrict__ units,
+                       int nunits, int parts, int chunks, const InterpKey* __restrict__ entry,
+                       const InterpCache* __restrict__ carried, NearRecord* __restrict__ rec, cplx* __restrict__ G,
+                       int chain) {
+  __shared__ NearShared<kNearGroundPairs> S;
+  const int k0 = chain ? 0 : blockIdx.x, k1 = chain ? nunits : k0 + 1;
+  const int64_t n = A.n;
+  InterpKey key = entry[units[k0]];
+  int status = 0;
+  for (int k = k0; k < k1; k++) {
+    const int u = units[k], j = u / parts;
+    NearUnit unit;
+    unit.start(key);
+    for (int q = 0; q < chunks; q++) {
+      const int64_t i0 = ((int64_t)(u % parts) * chunks + q) * kNearGroundPairs;
+      const int count = (int)max((int64_t)0, min((int64_t)kNearGroundPairs, n - i0));
+      if (count == 0) break;
+      key = near_chunk<EXK>(
+          S, count, key, A.P, n, carried, tab,
+          [&](int p, SrcSeg& J, double* o, bool& ij) {
+            const int64_t i = i0 + p;
+            J = near_source<EXK>(A.x, A.y, A.z, A.s, A.b, A.cab, A.sab, A.salp, A.ind1, A.ind2, j);
+            o[0] = A.x[i];
+            o[1] = A.y[i];
+            o[2] = A.z[i];
+            o[3] = A.b[i];
+            ij = i != j;
+            return image_r2(o[0] - J.x, o[1] - J.y, o[2] + J.z) <= .95;
+          },
+          &status);
+      const int p = threadIdx.x;
+      if (p < count && S.near[p]) {
+        const int64_t i = i0 + p;
+        cplx ex[9], out[3];
+        for (int c = 0; c < 9; c++) ex[c] = S.base[p][c] + S.rom[p][c];
+        project_fields(ex, A.cab[i], A.sab[i], A.salp[i], &out[0], &out[1], &out[2]);
+        cplx* o = G + (i * n + j) * 3;
+        o[0] = out[0];
+        o[1] = out[1];
+        o[2] = out[2];
+      }
+      if (threadIdx.x == 0) unit.chunk(S, count);
     }
-    key = InterpKey{S.igrs, S.ix, S.iy, S.carry};
-    r.exit = key;
-    rec[j] = r;
+    unit.r.exit = key;
+    if (threadIdx.x == 0) rec[u] = unit.r;
   }
   if (status) atomicOr(A.status, status);
 }
 
 // The cache a fill leaves, with coefficients of this fill's tables, kept
-// for the next fill (one thread).
+// for the next fill (one thread per function and row of the patch).
 __global__ void interp_store_kernel(InterpKey key, const cplx* __restrict__ tab, InterpCache* __restrict__ out) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  InterpCache S;
-  key.carry = 0;
-  interp_restore(S, key, tab, nullptr);
-  *out = S;
+  const int g = key.igrs, nd = somm_nx(g), ndp = nd * somm_ny(g), q = threadIdx.x >> 2, i = threadIdx.x & 3;
+  int ixs, iys, ixeg, iyeg;
+  interp_cell(g, key.ix, key.iy, &ixs, &iys, &ixeg, &iyeg);
+  interp_cubic(tab + somm_off(g) + ixs + (iys - 2) * nd - 2 + q * ndp + i * nd, &out->a[i][q], &out->b[i][q],
+               &out->c[i][q], &out->d[i][q]);
+  if (threadIdx.x == 0) {
+    out->dx = somm_dx(g);
+    out->dy = somm_dy(g);
+    out->xz = (ixs - 1) * out->dx + somm_xs(g);
+    out->yz = (iys - 1) * out->dy + somm_ys(g);
+  }
 }
 
 }  // namespace necb

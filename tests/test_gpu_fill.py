@@ -86,3 +86,26 @@ def test_fill_of_a_block_in_chunks(nb, engine):
     assert np.max(np.abs(z1[:, 7] - total)) <= 1e-13 * np.sum(np.abs(z0), axis=1).max()
     z0[:, 7] = z1[:, 7] = 0
     assert np.max(np.abs(z1 - z0)) <= 1e-15 * np.max(np.abs(z0))
+
+
+# units of 16 observation points per source column, whole and partial; 257
+# segments make them two chunks long
+@pytest.mark.parametrize("n", [2, 7, 16, 17, 33, 257])
+def test_near_ground_fill_at_unit_edges(nb, oracle, engine, n):
+    """Pairs within the table limit of their image, in the reference's order
+    through its interpolation cache: to 1e-12 of max|Z| against the oracle
+    integrating the device's own tables."""
+    ctx = nb.nec_create()
+    length = 4.0 if n > 100 else 1.2
+    assert nb.nec_wire(ctx, 1, n, 0.0, -0.5 * length, 0.05, 0.3, 0.5 * length, 0.35, 1e-3, 1.0, 1.0) == 0
+    assert nb.nec_geometry_complete(ctx, 1) == 0
+    assert nb.nec_gn_card(ctx, 2, 0, 10.0, 0.01, 0, 0, 0, 0) == 0
+    st = nb.structure(ctx, 299.8)
+    nb.nec_delete(ctx)
+    engine.reset_interpolation()
+    engine.set_structure(st)
+    engine.fill()
+    st["somm"] = engine.sommerfeld_tables()
+    Zo, _ = oracle.fill(st)
+    assert np.max(np.abs(engine.copy_z() - Zo)) <= 1e-12 * np.max(np.abs(Zo))
+    engine.reset_interpolation()
