@@ -242,6 +242,11 @@ struct necgpu_engine {
   std::vector<int32_t> h_tptr, h_tbasis, h_ind;
   unsigned* d_sweep_ctr = nullptr;  // progress of the refinement sweeps
   bool inv_sweep = true;
+  // the whole refinement in one launch (refine_kernel): its norms, results
+  // and counters, and the other copy of the solution
+  bool refine_fused = true;
+  double* d_refine = nullptr;
+  double2* d_x2 = nullptr;
   bool use_dmma = true;  // FP64 trailing update on the FP64 tensor cores
   int64_t outer = 256;  // outer block of the block-pivoted mixed LU (multiple of 64)
   // mixed path: block-local pivoting first, full partial pivoting as fallback
@@ -448,6 +453,8 @@ void free_all(necgpu_engine* e) {
   e->tc_kbytes2 = 0;
   dfree(e, e->d_tinv);
   dfree(e, e->d_sweep_ctr);
+  dfree(e, e->d_refine);
+  dfree(e, e->d_x2);
   dfree(e, e->ZT32);
   dfree(e, e->ZT64);
   dfree(e, e->d_tinvT);
@@ -1627,6 +1634,78 @@ int run_trsv_inv(necgpu_engine* e, float2* rhs, float2* sol) {
   return run_trsv_inv_on(e, e->Z32, e->d_tinv, e->d_wnext, rhs, sol);
 }
 
+// Z x = b (or, transposed, Z^T x = b) by refine_kernel; false in *done when
+// this device or engine does not take it (the launches of refine then do).
+template <bool ADJ>
+int refine_fused(necgpu_engine* e, const double2* b, double2* x, double2* r, int* iters, double* rel, bool* done) {
+  *done = false;
+  const int64_t n = e->n;
+  // per-launch timing wants the classes apart
+  if (!e->inv_sweep || !e->sweep_trsv || !e->refine_fused || e->sweep_cluster < kRefineCTAs || n > kRefineMaxN ||
+      e->timing_level >= 2)
+    return 0;
+  if (!e->d_refine) TRY(dalloc(e, e->d_refine, 16));  // norms, results, counters
+  if (!e->d_x2) TRY(dalloc(e, e->d_x2, (size_t)n));
+  RefineArgs a{};
+  a.n = n;
+  a.ld = e->ld;
+  a.M = ADJ ? e->ZT32 : e->Z32;
+  a.tinv = ADJ ? e->d_tinvT : e->d_tinv;
+  a.wnext = ADJ ? e->d_wnextT : e->d_wnext;
+  a.Z = ADJ ? e->ZT64 : e->Z64;
+  a.b = b;
+  a.perm = e->d_perm;
+  a.x = x;
+  a.x2 = e->d_x2;
+  a.r = r;
+  // the FP64-sized work vectors hold two complex64 ones each
+  a.w1 = reinterpret_cast<float2*>(e->d_w1);
+  a.w4 = a.w1 + n;
+  a.w2 = reinterpret_cast<float2*>(e->d_w2);
+  a.w3 = a.w2 + n;
+  a.norms = e->d_refine;
+  a.out = e->d_refine + 4;
+  a.counters = reinterpret_cast<unsigned*>(e->d_refine + 8);
+  a.status = e->d_status;
+  a.tol = e->refine_tol;
+  a.max_iter = e->refine_max;
+  CUDA_TRY(cudaMemsetAsync(e->d_refine, 0, 16 * sizeof(double), e->stream));
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(kRefineCTAs);
+  cfg.blockDim = dim3(kInvSweepThreads);
+  cfg.dynamicSmemBytes = sizeof(RefineShared);
+  cfg.stream = e->stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kRefineCTAs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(refine_kernel<ADJ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(refine_kernel<ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(RefineShared)) != cudaSuccess ||
+      cudaLaunchKernelEx(&cfg, refine_kernel<ADJ>, a) != cudaSuccess) {
+    (void)cudaGetLastError();  // the configuration was refused: the separate launches, from now on
+    e->refine_fused = false;
+    return 0;
+  }
+  e->launches++;
+  double out[2] = {0, 0};
+  int st = 0;
+  CUDA_TRY(cudaMemcpyAsync(out, a.out, sizeof out, cudaMemcpyDeviceToHost, e->stream));
+  CUDA_TRY(cudaMemcpyAsync(&st, e->d_status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+  CUDA_TRY(cudaStreamSynchronize(e->stream));
+  e->stats.d2h_bytes += sizeof out + sizeof st;
+  *done = true;
+  *iters = (int)out[0];
+  *rel = out[1];
+  if (st & (1 << 9)) return fail(e, NECGPU_ERR_CUDA, "refinement: triangular sweep gave up waiting on a block");
+  if (!std::isfinite(*rel))
+    return fail(e, NECGPU_ERR_NONFINITE, ADJ ? "adjoint: non-finite residual" : "refinement: non-finite residual");
+  return 0;
+}
+
 // Mixed-precision factorisation of the FP64 matrix: demote to complex64, then
 // LU with block-local pivoting (blockpiv) or full partial pivoting.
 // Operand format of the next mixed factorisation.  TF32 saves a third of the
@@ -1665,6 +1744,9 @@ int factor_mixed(necgpu_engine* e, bool blockpiv) {
 // x = 0, r = b; repeat d = LU^-1 r, x += d, r = b - Z x (FP64) until the
 // relative residual reaches the tolerance or stops decreasing.
 int refine(necgpu_engine* e, int* iters, double* rel_out) {
+  bool done = false;
+  const int rc = refine_fused<false>(e, e->d_b, e->d_x, e->d_r, iters, rel_out, &done);
+  if (rc || done) return rc;
   const int64_t n = e->n;
   const unsigned g1 = (unsigned)((n + 255) / 256);
   float2* w1 = reinterpret_cast<float2*>(e->d_w1);
@@ -1742,6 +1824,9 @@ int ensure_adjoint(necgpu_engine* e) {
 // Z^T w = phi (device vectors), refined in FP64 against Z^T like the forward
 // solve: w = 0, r = phi; repeat d = P^T L^-T U^-T r, w += d, r = phi - Z^T w.
 int refine_T(necgpu_engine* e, const double2* phi, double2* w, int* iters, double* rel_out) {
+  bool done = false;
+  const int rc = refine_fused<true>(e, phi, w, e->d_adj_r, iters, rel_out, &done);
+  if (rc || done) return rc;
   const int64_t n = e->n;
   const unsigned g1 = (unsigned)((n + 255) / 256);
   float2* w1 = reinterpret_cast<float2*>(e->d_w1);
@@ -2123,6 +2208,7 @@ int necgpu_create(necgpu_engine** out, int device) {
   if (const char* s = std::getenv("NECPP_B200_BLOCKED_TRSV")) e->sweep_trsv = (s[0] == '0');
   if (const char* s = std::getenv("NECPP_B200_PARTIAL_PIVOT")) e->prefer_blockpiv = (s[0] == '0');
   if (const char* s = std::getenv("NECPP_B200_FLAG_SWEEP")) e->inv_sweep = (s[0] == '0');
+  if (const char* s = std::getenv("NECPP_B200_REFINE_FUSED")) e->refine_fused = (s[0] != '0');
   if (const char* s = std::getenv("NECPP_B200_NO_DMMA")) e->use_dmma = (s[0] == '0');
   if (const char* s = std::getenv("NECPP_B200_LOOKAHEAD")) e->env_lookahead = (s[0] != '0');
   if (const char* s = std::getenv("NECPP_B200_TRSM1")) e->trsm8 = (s[0] == '0');

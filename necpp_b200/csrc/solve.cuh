@@ -564,29 +564,52 @@ __device__ __forceinline__ float2 ld_volatile_shared_f2(const float2* p) {
 // without fences.  All CTAs of a cluster
 // meet at a cluster barrier before they exit, so none exits while a peer
 // may still write to it.
-template <bool LOWER, int CS = 0>
-__global__ void __launch_bounds__(kInvSweepThreads, 2) inv_sweep_kernel(const float2* M, int64_t ld, int64_t n,
-                                                                     const float2* tinv, const float2* wnext,
-                                                                     const float2* b, float2* x, unsigned* counter,
-                                                                     int* status) {
+struct SweepShared {
+  float2 part[4][kBlk];
+  float2 part2[4][kBlk];  // the last products' partial sums (part may still be read)
+  float2 sv[kBlk];
+  alignas(16) float2 sx[kInvSweepChunk * kBlk];
+  float2 sinv[kBlk][kBlk + 1];      // inv(T_vv), rows padded against bank conflicts
+  float2 xin[kSweepDepth][kBlk];    // x_{s-d} from cluster peers (CS > 0), unset until written
+  int s_avail;
+};
+
+// Marks the hand-off buffers unset (CS > 0); a barrier of the cluster must
+// follow before a peer may write to them.
+__device__ __forceinline__ void sweep_reset(SweepShared& S) {
+  for (int e = threadIdx.x; e < kSweepDepth * kBlk; e += kInvSweepThreads)
+    S.xin[e / kBlk][e % kBlk] = make_float2(__uint_as_float(kSweepUnset), __uint_as_float(kSweepUnset));
+}
+
+// inv(T_vv) of the CTA's block, 16 loads of each thread in flight at a time
+__device__ __forceinline__ void sweep_load_inverse(float2 (&sinv)[kBlk][kBlk + 1], const float2* tinv) {
+  constexpr int L = kBlk * kBlk / kInvSweepThreads;
+  float2 v[L];
+#pragma unroll
+  for (int k = 0; k < L; k++) v[k] = __ldg(tinv + threadIdx.x + k * kInvSweepThreads);
+#pragma unroll
+  for (int k = 0; k < L; k++) {
+    const int e = threadIdx.x + k * kInvSweepThreads;
+    sinv[e / kBlk][e % kBlk] = v[k];
+  }
+}
+
+// This CTA's positions of one sweep; false when a wait ran out.  LOADED: the
+// inverse of its (one) block is in sinv already.
+template <bool LOWER, int CS, bool LOADED = false>
+__device__ __forceinline__ bool inv_sweep_run(SweepShared& S, float2 (&sinv)[kBlk][kBlk + 1], const float2* M, int64_t ld, int64_t n,
+                                              const float2* tinv, const float2* wnext, const float2* b, float2* x,
+                                              unsigned* counter, int* status, unsigned rank) {
   constexpr int NB = kBlk, QW = NB / 4, KX = kInvSweepChunk, D = kSweepDepth;  // four column quarters of 16
-  __shared__ float2 part[4][NB];
-  __shared__ float2 part2[4][NB];  // the last products' partial sums (part may still be read)
-  __shared__ float2 sv[NB];
-  __shared__ float2 sx[KX * NB];
-  __shared__ float2 sinv[NB][NB + 1];  // inv(T_vv), rows padded against bank conflicts
-  __shared__ float2 xin[D][NB];        // x_{s-d} from cluster peers (CS > 0), unset until written
-  __shared__ int s_avail;
+  auto& part = S.part;
+  auto& part2 = S.part2;
+  auto& sv = S.sv;
+  auto& sx = S.sx;
+  auto& xin = S.xin;
+  int& s_avail = S.s_avail;
   const int t = threadIdx.x;
   const int r = t & (NB - 1), q = t >> 6;  // row in the block, column quarter
   const int nblk = (int)((n + NB - 1) / NB);
-  unsigned rank = 0;
-  if constexpr (CS > 0) {
-    rank = cluster_rank();
-    for (int e = t; e < D * NB; e += kInvSweepThreads)
-      xin[e / NB][e % NB] = make_float2(__uint_as_float(kSweepUnset), __uint_as_float(kSweepUnset));
-    cluster_sync_all();  // no peer writes before every buffer is unset
-  }
   // one position of the sweep order; false when a wait ran out
   auto position = [&](int s) -> bool {
     const int v = LOWER ? s : nblk - 1 - s;
@@ -598,7 +621,7 @@ __global__ void __launch_bounds__(kInvSweepThreads, 2) inv_sweep_kernel(const fl
     const int64_t bbase = ((int64_t)v * 2 + (LOWER ? 0 : 1)) * NB * NB;
     const int64_t wbase = ((int64_t)v * 2 + (LOWER ? 0 : 1)) * D * NB * NB + r * NB + q * QW;
     __syncthreads();  // the previous block's reads of sinv are done
-    for (int e = t; e < NB * NB; e += kInvSweepThreads) sinv[e / NB][e % NB] = tinv[bbase + e];
+    if (!LOADED) sweep_load_inverse(sinv, tinv + bbase);
     // this thread's row quarters of the W_d (128-byte lines) into L2, late
     // enough that the tiles streamed meanwhile do not evict them: at the
     // last pass of the fold-in, or now when there is none
@@ -608,7 +631,7 @@ __global__ void __launch_bounds__(kInvSweepThreads, 2) inv_sweep_kernel(const fl
         if (s >= d) asm volatile("prefetch.global.L2 [%0];" ::"l"(wnext + wbase + (d - 1) * NB * NB));
     };
     if (s - D <= 0) prefetch_w();
-    const float2 bb = t < bs ? b[r0 + t] : make_float2(0.f, 0.f);
+    const float2 bb = t < bs ? __ldcg(b + r0 + t) : make_float2(0.f, 0.f);
     // the quarter row of the tile at sweep position i
     auto load_tile = [&](float2 (&m)[QW], int i) {
       const int u = LOWER ? i : nblk - 1 - i;
@@ -864,12 +887,232 @@ __global__ void __launch_bounds__(kInvSweepThreads, 2) inv_sweep_kernel(const fl
     return true;
   };
   if constexpr (CS > 0) {
-    if ((int)blockIdx.x < nblk) position((int)blockIdx.x);
-    cluster_sync_all();
+    return (int)blockIdx.x >= nblk || position((int)blockIdx.x);
   } else {
     for (int s = blockIdx.x; s < nblk; s += gridDim.x)  // s: position in sweep order
-      if (!position(s)) return;
+      if (!position(s)) return false;
+    return true;
   }
+}
+
+template <bool LOWER, int CS = 0>
+__global__ void __launch_bounds__(kInvSweepThreads, 2) inv_sweep_kernel(const float2* M, int64_t ld, int64_t n,
+                                                                     const float2* tinv, const float2* wnext,
+                                                                     const float2* b, float2* x, unsigned* counter,
+                                                                     int* status) {
+  __shared__ SweepShared S;
+  unsigned rank = 0;
+  if constexpr (CS > 0) {
+    rank = cluster_rank();
+    sweep_reset(S);
+    cluster_sync_all();  // no peer writes before every buffer is unset
+  }
+  inv_sweep_run<LOWER, CS>(S, S.sinv, M, ld, n, tinv, wnext, b, x, counter, status, rank);
+  if constexpr (CS > 0) cluster_sync_all();
+}
+
+// ---------------------------------------------------------------------------
+// The whole iterative refinement of up to 1,024 unknowns in one launch of one
+// cluster of 16 CTAs: x = 0, r = b; repeat d = U^-1 L^-1 P r on the complex64
+// factors, x += d, r = b - Z x in FP64, until ||r|| / ||b|| <= tol or the
+// residual stops halving.  (Adjoint: the transposed factors without the
+// permutation, d scattered through it.)  A step is the two sweeps (a 64-row
+// block per CTA) and the residual (the rows shared by the CTAs), with a
+// cluster barrier between them; every CTA reads the residual norm and takes
+// the same decision, so the host waits once per solve.  The inverted diagonal
+// blocks stay in shared memory from step to step.
+//
+// Latency-bound.  As separate launches (permutation, two memsets and a launch
+// per sweep, copy, update, memset, residual, read-back) a step of a mesh of
+// 480 segments took 105 us, of which the sweeps and the residual were 35;
+// here it takes 34.  The limit is the cluster: beyond 16 blocks a step needs
+// barriers of the whole grid and the residual more SMs than that, and the
+// separate launches, each at its own best grid, were faster (3,280 unknowns:
+// 280 against 395 us a step; 11,520: 1.2 against 2.0 ms).
+constexpr int kRefineCTAs = 16;
+constexpr int64_t kRefineMaxN = (int64_t)kRefineCTAs * kBlk;
+struct RefineArgs {
+  int64_t n, ld;
+  const float2 *M, *tinv, *wnext;  // factors, block inverses, neighbouring products
+  const double2 *Z, *b;
+  const int* perm;
+  double2 *x, *x2, *r;    // solution (x at the end) and its other copy, residual
+  float2 *w1, *w2, *w3;   // permuted residual, L^-1 of it, U^-1 of that
+  float2* w4;             // adjoint: w3 scattered
+  double* norms;          // [0..2] the steps' ||r||^2 in turn, [3] ||b||^2: zero at launch
+  unsigned* counters;     // [0], [1] the sweeps'
+  int* status;
+  double tol;
+  int max_iter;
+  double* out;            // [0] steps, [1] final ||r|| / ||b||
+};
+struct RefineShared {
+  SweepShared S;
+  float2 sinv2[kBlk][kBlk + 1];  // the upper sweep's inverse
+};
+
+// r = b - Z xs for `R` rows per warp of one chunk: 16 loads in flight a lane
+template <int R>
+__device__ __forceinline__ void residual_rows(const double2* z, int64_t ld, int rows, int cnt, const double2* xs,
+                                              double (&sr)[4], double (&si)[4]) {
+  const int lane = threadIdx.x & 31;
+  constexpr int U = R == 1 ? 8 : 16 / R;
+  const double2* zk[R];
+#pragma unroll
+  for (int k = 0; k < R; k++) zk[k] = z + (k < rows ? k : 0) * ld;  // a row too many is computed and dropped
+  for (int e0 = lane; e0 < cnt; e0 += 32 * U) {
+    double2 a[R][U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int e = min(e0 + 32 * u, cnt - 1);  // past the end: the last element, times zero
+#pragma unroll
+      for (int k = 0; k < R; k++) a[k][u] = __ldg(zk[k] + e);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int e = e0 + 32 * u;
+      const double2 v = e < cnt ? xs[e] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int k = 0; k < R; k++) {
+        sr[k] += a[k][u].x * v.x - a[k][u].y * v.y;
+        si[k] += a[k][u].x * v.y + a[k][u].y * v.x;
+      }
+    }
+  }
+}
+
+template <bool ADJOINT>
+__global__ void __launch_bounds__(kInvSweepThreads, 1) refine_kernel(const __grid_constant__ RefineArgs A) {
+  extern __shared__ unsigned char refine_smem[];
+  RefineShared& RS = *reinterpret_cast<RefineShared*>(refine_smem);
+  SweepShared& S = RS.S;
+  constexpr int CS = kRefineCTAs;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int64_t n = A.n, ld = A.ld;
+  const unsigned rank = cluster_rank();
+  const int nblk = (int)((n + kBlk - 1) / kBlk);
+  // this CTA's rows of the vectors and of the residual
+  const int64_t per = (n + CS - 1) / CS;
+  const int64_t c0 = min(n, per * rank), c1 = min(n, c0 + per);
+  const float2 unset = make_float2(__uint_as_float(kSweepUnset), __uint_as_float(kSweepUnset));
+  double2 *x = A.x, *xn = A.x2;
+  double part = 0.0;
+  for (int64_t i = c0 + t; i < c1; i += kInvSweepThreads) {
+    const double2 v = A.b[i];
+    x[i] = make_double2(0.0, 0.0);
+    A.r[i] = v;
+    part += v.x * v.x + v.y * v.y;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) part += __shfl_down_sync(0xffffffffu, part, off);
+  if (lane == 0 && c1 > c0) atomicAdd(A.norms + 3, part);
+  if ((int)rank < nblk) {  // position `rank` of the lower sweep is block rank, of the upper nblk - 1 - rank
+    sweep_load_inverse(S.sinv, A.tinv + (int64_t)rank * 2 * kBlk * kBlk);
+    sweep_load_inverse(RS.sinv2, A.tinv + ((int64_t)(nblk - 1 - (int)rank) * 2 + 1) * kBlk * kBlk);
+  }
+  double prev = 1e300, rel = 1.0;
+  int it = 0;
+  cluster_sync_all();  // r is written
+  for (; it <= A.max_iter; it++) {
+    for (int64_t i = c0 + t; i < c1; i += kInvSweepThreads) {
+      const double2 v = __ldcg(A.r + (ADJOINT ? i : (int64_t)A.perm[i]));
+      A.w1[i] = make_float2((float)v.x, (float)v.y);
+      A.w2[i] = unset;
+      A.w3[i] = unset;
+    }
+    if (rank == 0 && t == 0) {
+      A.counters[0] = A.counters[1] = 0;
+      A.norms[(it + 1) % 3] = 0.0;
+    }
+    sweep_reset(S);
+    cluster_sync_all();
+    bool ok = inv_sweep_run<true, CS, true>(S, S.sinv, A.M, ld, n, A.tinv, A.wnext, A.w1, A.w2, A.counters, A.status,
+                                            rank);
+    // every value that a peer sends in a sweep has been taken by the CTA it
+    // was sent to before that CTA gets here
+    __syncthreads();
+    sweep_reset(S);
+    cluster_sync_all();
+    ok = inv_sweep_run<false, CS, true>(S, RS.sinv2, A.M, ld, n, A.tinv, A.wnext, A.w2, A.w3, A.counters + 1, A.status,
+                                        rank) &&
+         ok;
+    (void)ok;  // a wait that ran out has set the status bit
+    cluster_sync_all();
+    if (*(volatile int*)A.status & (1 << 9)) break;  // the same in every CTA: set before the barrier
+    const float2* d = A.w3;
+    if (ADJOINT) {
+      for (int64_t i = c0 + t; i < c1; i += kInvSweepThreads) A.w4[A.perm[i]] = __ldcg(A.w3 + i);
+      cluster_sync_all();
+      d = A.w4;
+    }
+    // x += d and r = b - Z x for rows [c0, c1): the new x staged in shared
+    // memory a chunk at a time, up to four rows per warp
+    constexpr int KC = kInvSweepChunk * kBlk / 2;
+    double2* xs = reinterpret_cast<double2*>(S.sx);
+    const int rw = (int)min((int64_t)4, (c1 - c0 + 7) / 8);
+    double rn = 0.0;
+    for (int64_t g0 = c0; g0 < c1; g0 += 8 * rw) {
+      const int64_t row0 = g0 + warp * rw;
+      const int rows = (int)max((int64_t)0, min((int64_t)rw, c1 - row0));
+      double sr[4] = {0, 0, 0, 0}, si[4] = {0, 0, 0, 0};
+      for (int64_t q0 = 0; q0 < n; q0 += KC) {
+        const int cnt = (int)min((int64_t)KC, n - q0);
+        __syncthreads();
+        for (int e = t; e < cnt; e += kInvSweepThreads) {
+          double2 v = __ldcg(x + q0 + e);
+          const float2 w = __ldcg(d + q0 + e);
+          v.x += (double)w.x;
+          v.y += (double)w.y;
+          xs[e] = v;
+          if (q0 + e >= c0 && q0 + e < c1 && g0 == c0) xn[q0 + e] = v;
+        }
+        __syncthreads();
+        if (rows > 0) {
+          const double2* z = A.Z + row0 * ld + q0;
+          if (rw == 1)
+            residual_rows<1>(z, ld, rows, cnt, xs, sr, si);
+          else if (rw == 2)
+            residual_rows<2>(z, ld, rows, cnt, xs, sr, si);
+          else
+            residual_rows<4>(z, ld, rows, cnt, xs, sr, si);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (k < rows) {
+#pragma unroll
+          for (int off = 16; off > 0; off >>= 1) {
+            sr[k] += __shfl_down_sync(0xffffffffu, sr[k], off);
+            si[k] += __shfl_down_sync(0xffffffffu, si[k], off);
+          }
+          if (lane == 0) {
+            const double2 bb = A.b[row0 + k];
+            const double2 o = make_double2(bb.x - sr[k], bb.y - si[k]);
+            A.r[row0 + k] = o;
+            rn += o.x * o.x + o.y * o.y;
+          }
+        }
+    }
+    if (lane == 0 && c1 > c0) atomicAdd(A.norms + it % 3, rn);
+    cluster_sync_all();
+    double2* const tmp = x;
+    x = xn;
+    xn = tmp;
+    const double bn = sqrt(__ldcg(A.norms + 3)), rr = sqrt(__ldcg(A.norms + it % 3));
+    rel = bn > 0 ? rr / bn : 0.0;
+    if (!isfinite(rel) || rel <= A.tol || rel > 0.5 * prev) {  // converged, or at the FP64 floor
+      it++;
+      break;
+    }
+    prev = rel;
+  }
+  if (x != A.x)
+    for (int64_t i = c0 + t; i < c1; i += kInvSweepThreads) A.x[i] = x[i];  // rows this CTA wrote
+  if (rank == 0 && t == 0) {
+    A.out[0] = it;
+    A.out[1] = rel;
+  }
+  cluster_sync_all();  // no CTA leaves while a peer may still write to it
 }
 
 // ---------------------------------------------------------------------------
