@@ -11,7 +11,7 @@
 //                         memory, register-tiled trailing updates) and the
 //                         solve refined in FP64 against the FP64 matrix
 //   batch_coeff_kernel    basis amplitudes -> a, b, c and currents
-//   batch_pattern_kernel  far field, one warp per (problem, direction)
+//   batch_pattern_kernel  far field, one warp per problem and few directions
 #pragma once
 #include <cstdint>
 
@@ -462,109 +462,36 @@ struct BatchPatternArgs {
   float* gain;         // nprob x ndir power gain in dB (db10 with the -999.99 floor), or null
 };
 
-__global__ void __launch_bounds__(kPatDirs * 32) batch_pattern_kernel(BatchPatternArgs A) {
+template <int DW>
+__global__ void __launch_bounds__(kPatDirs * 32, 2) batch_pattern_kernel(const __grid_constant__ BatchPatternArgs A) {
   __shared__ SegPat seg[kPatChunk];
   const int p = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int d = blockIdx.x * kPatDirs + warp;
-  const bool active = d < A.ndir;
+  const int d0 = (blockIdx.x * kPatDirs + warp) * DW;
   const int64_t s0 = A.seg_off[p], ns = A.seg_off[p + 1] - s0;
-  const int64_t T = A.nseg_total;
-  double thet = 0, phi = 0;
-  if (active) {
-    thet = A.theta[d];
-    phi = A.phi[d];
-  }
-  double sp, cp, st, ct;
-  sincos(phi, &sp, &cp);
-  sincos(thet, &st, &ct);
-  const double phx = -sp, phy = cp;
-  const double roz0 = ct;
-  const double thx = roz0 * phy, thy = -roz0 * phx, thz = -st;
-  const double rox = -thz * phy, roy = thz * phx;
-  cplx ci[2][3];
-  for (int k = 0; k < A.ksymp; k++) {
-    const double roz = (k == 0) ? roz0 : -roz0;
-    cplx sx = mk(0, 0), sy = mk(0, 0), sz = mk(0, 0);
-    for (int64_t c0 = 0; c0 < ns; c0 += kPatChunk) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < kPatChunk; t += blockDim.x) {
-        const int64_t i = s0 + c0 + t;
-        if (c0 + t < ns) {
-          SegPat g;
-          g.x = A.seg[i];
-          g.y = A.seg[T + i];
-          g.z = A.seg[2 * T + i];
-          g.s = A.seg[3 * T + i];
-          g.cab = A.seg[5 * T + i];
-          g.sab = A.seg[6 * T + i];
-          g.salp = A.seg[7 * T + i];
-          g.air = A.abc[i];
-          g.aii = A.abc[T + i];
-          g.bir = A.abc[2 * T + i];
-          g.bii = A.abc[3 * T + i];
-          g.cir = A.abc[4 * T + i];
-          g.cii = A.abc[5 * T + i];
-          seg_pat_el(g);
-          seg[t] = g;
-        }
-      }
-      __syncthreads();
-      if (active) {
-        const int cnt = (int)min((int64_t)kPatChunk, ns - c0);
-        for (int t = lane; t < cnt; t += 32) {
-          const SegPat& g = seg[t];
-          cplx exa;
-          seg_term(g, rox, roy, roz, &exa);
-          sx += exa * g.cab;
-          sy += exa * g.sab;
-          sz += exa * g.salp;
-        }
-      }
-    }
+  PatDir dir[DW];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      sx.re += __shfl_down_sync(0xffffffffu, sx.re, off);
-      sx.im += __shfl_down_sync(0xffffffffu, sx.im, off);
-      sy.re += __shfl_down_sync(0xffffffffu, sy.re, off);
-      sy.im += __shfl_down_sync(0xffffffffu, sy.im, off);
-      sz.re += __shfl_down_sync(0xffffffffu, sz.re, off);
-      sz.im += __shfl_down_sync(0xffffffffu, sz.im, off);
+  for (int q = 0; q < DW; q++) {
+    const int d = min(d0 + q, A.ndir - 1);
+    dir[q] = pat_dir(A.theta[d], A.phi[d]);
+  }
+  cplx ci[DW][2][3];
+  pattern_sums<DW>(seg, A.seg, A.abc, A.nseg_total, s0, ns, dir, A.ksymp, ci);
+#pragma unroll
+  for (int q = 0; q < DW; q++)
+    if (lane == q && d0 + q < A.ndir) {
+      cplx e_t, e_p;
+      pattern_fields(dir[q], ci[q], A.ksymp, A.perfect, A.zrati, A.eta, &e_t, &e_p);
+      const int64_t o = (int64_t)p * A.ndir + d0 + q;
+      if (A.eth) {
+        A.eth[o] = make_double2(e_t.re, e_t.im);
+        A.eph[o] = make_double2(e_p.re, e_p.im);
+      }
+      if (A.gain) {
+        const double pw = A.gcop[p] * (e_t.re * e_t.re + e_t.im * e_t.im + e_p.re * e_p.re + e_p.im * e_p.im);
+        A.gain[o] = pw < 1.0e-20 ? -999.99f : (float)(10.0 * log10(pw));
+      }
     }
-    ci[k][0] = sx;
-    ci[k][1] = sy;
-    ci[k][2] = sz;
-  }
-  if (!active || lane != 0) return;
-  cplx cix = ci[0][0], ciy = ci[0][1], ciz = ci[0][2];
-  if (A.ksymp == 2) {
-    cplx rrv, rrh;
-    if (A.perfect) {
-      rrv = mk(-1.0, -0.0);
-      rrh = mk(-1.0, -0.0);
-    } else {
-      cplx zrsin = csqrt_(1. - A.zrati * A.zrati * thz * thz);
-      rrv = -(roz0 - A.zrati * zrsin) / (roz0 + A.zrati * zrsin);
-      rrh = (A.zrati * roz0 - zrsin) / (A.zrati * roz0 + zrsin);
-    }
-    cplx ix = ci[1][0], iy = ci[1][1], iz = ci[1][2];
-    cplx cdp = (ix * phx + iy * phy) * (rrh - rrv);
-    cix = cix + ix * rrv + cdp * phx;
-    ciy = ciy + iy * rrv + cdp * phy;
-    ciz = ciz - iz * rrv;
-  }
-  const cplx C3 = mk(0.0, -A.eta / (4.0 * 3.1415926536));
-  cplx e_t = (cix * thx + ciy * thy + ciz * thz) * C3;
-  cplx e_p = (cix * phx + ciy * phy) * C3;
-  const int64_t o = (int64_t)p * A.ndir + d;
-  if (A.eth) {
-    A.eth[o] = make_double2(e_t.re, e_t.im);
-    A.eph[o] = make_double2(e_p.re, e_p.im);
-  }
-  if (A.gain) {
-    const double pw = A.gcop[p] * (e_t.re * e_t.re + e_t.im * e_t.im + e_p.re * e_p.re + e_p.im * e_p.im);
-    A.gain[o] = pw < 1.0e-20 ? -999.99f : (float)(10.0 * log10(pw));
-  }
 }
 
 }  // namespace necb

@@ -1925,12 +1925,6 @@ int run_pattern(necgpu_engine* e, int ndir) {
   a.theta = e->d_theta;
   a.phi = e->d_phi;
   a.x = e->d_seg;
-  a.y = e->d_seg + n;
-  a.z = e->d_seg + 2 * n;
-  a.s = e->d_seg + 3 * n;
-  a.cab = e->d_seg + 5 * n;
-  a.sab = e->d_seg + 6 * n;
-  a.salp = e->d_seg + 7 * n;
   a.abc = e->d_abc;
   a.ksymp = (e->ground == kGroundNone) ? 1 : 2;
   a.perfect = (e->ground == kGroundPerfect) ? 1 : 0;
@@ -1939,8 +1933,13 @@ int run_pattern(necgpu_engine* e, int ndir) {
   a.eth = e->d_eth;
   a.eph = e->d_eph;
   // work units: one per (direction, segment, image) term
-  KLAUNCH(NECGPU_K_PATTERN, (double)ndir * n * a.ksymp,
-          pattern_kernel<<<(unsigned)((ndir + kPatDirs - 1) / kPatDirs), kPatDirs * 32, 0, e->stream>>>(a));
+  const int dw = pattern_width(ndir, 1, e->nsm);
+  const unsigned grid = (unsigned)((ndir + kPatDirs * dw - 1) / (kPatDirs * dw));
+  if (dw == kPatWide)
+    KLAUNCH(NECGPU_K_PATTERN, (double)ndir * n * a.ksymp,
+            pattern_kernel<kPatWide><<<grid, kPatDirs * 32, 0, e->stream>>>(a));
+  else
+    KLAUNCH(NECGPU_K_PATTERN, (double)ndir * n * a.ksymp, pattern_kernel<1><<<grid, kPatDirs * 32, 0, e->stream>>>(a));
   return 0;
 }
 
@@ -3563,9 +3562,14 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
       pa.eph = d_eph;
       pa.gcop = d_gcop;
       pa.gain = d_gain;
-      const dim3 g((unsigned)((ndir + kPatDirs - 1) / kPatDirs), (unsigned)nprob);
-      KLAUNCH(NECGPU_K_PATTERN, (double)ndir * T * pa.ksymp,
-              batch_pattern_kernel<<<g, kPatDirs * 32, 0, e->stream>>>(pa));
+      const int dw = pattern_width(ndir, nprob, e->nsm);
+      const dim3 g((unsigned)((ndir + kPatDirs * dw - 1) / (kPatDirs * dw)), (unsigned)nprob);
+      if (dw == kPatWide)
+        KLAUNCH(NECGPU_K_PATTERN, (double)ndir * T * pa.ksymp,
+                batch_pattern_kernel<kPatWide><<<g, kPatDirs * 32, 0, e->stream>>>(pa));
+      else
+        KLAUNCH(NECGPU_K_PATTERN, (double)ndir * T * pa.ksymp,
+                batch_pattern_kernel<1><<<g, kPatDirs * 32, 0, e->stream>>>(pa));
       if (eth) {
         CUDA_TRY(cudaMemcpyAsync(eth, d_eth, (size_t)nprob * ndir * sizeof(double2), cudaMemcpyDeviceToHost,
                                  e->stream));
