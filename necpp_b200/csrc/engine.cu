@@ -1538,11 +1538,10 @@ int invert_diag_blocks(necgpu_engine* e, bool force = false) {
   if (!e->d_sweep_ctr) TRY(dalloc(e, e->d_sweep_ctr, 4));
   CUDA_TRY(cudaFuncSetAttribute(tri_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_inv_smem()));
   KLAUNCH(NECGPU_K_OTHER, 0.0,
-          tri_inv_kernel<<<(unsigned)nblk, 128, tri_inv_smem(), e->stream>>>(e->Z32, e->ld, e->n, e->d_tinv));
+          tri_inv_kernel<<<dim3((unsigned)nblk, 2), 256, tri_inv_smem(), e->stream>>>(e->Z32, e->ld, e->n, e->d_tinv));
   if (!e->d_wnext) TRY(dalloc(e, e->d_wnext, (size_t)nblk * 2 * kSweepDepth * kBlk * kBlk));
-  CUDA_TRY(cudaFuncSetAttribute(next_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)next_tile_smem()));
   KLAUNCH(NECGPU_K_OTHER, 0.0,
-          next_tile_kernel<<<dim3((unsigned)nblk, 2, kSweepDepth), 256, next_tile_smem(), e->stream>>>(
+          next_tile_kernel<<<dim3((unsigned)nblk, 2, 4 * kSweepDepth), 256, 0, e->stream>>>(
               e->Z32, e->ld, e->n, e->d_tinv, e->d_wnext));
   return 0;
 }
@@ -1813,9 +1812,8 @@ int ensure_adjoint(necgpu_engine* e) {
   KLAUNCH(NECGPU_K_OTHER, 0.0, transpose_kernel<double2><<<g, 256, 0, e->stream>>>(e->Z64, ld, e->ZT64, ld, n));
   KLAUNCH(NECGPU_K_OTHER, 0.0, tinv_transpose_kernel<<<(unsigned)nblk, 256, 0, e->stream>>>(e->d_tinv, e->d_tinvT));
   if (!e->d_wnextT) TRY(dalloc(e, e->d_wnextT, (size_t)nblk * 2 * kSweepDepth * kBlk * kBlk));
-  CUDA_TRY(cudaFuncSetAttribute(next_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)next_tile_smem()));
   KLAUNCH(NECGPU_K_OTHER, 0.0,
-          next_tile_kernel<<<dim3((unsigned)nblk, 2, kSweepDepth), 256, next_tile_smem(), e->stream>>>(
+          next_tile_kernel<<<dim3((unsigned)nblk, 2, 4 * kSweepDepth), 256, 0, e->stream>>>(
               e->ZT32, ld, n, e->d_tinvT, e->d_wnextT));
   e->adj_ready = true;
   return 0;

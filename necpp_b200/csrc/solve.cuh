@@ -360,71 +360,92 @@ __global__ void demote_kernel(const double2* src, float2* dst, int64_t count) {
 // read of x_u and two block reductions.
 
 // tinv[2*blk] = L_bb^-1 (unit lower), tinv[2*blk+1] = U_bb^-1, 64 x 64
-// row-major each, zero outside the kb x kb triangle.  128 threads: threads
-// 0..63 build the columns of L^-1, threads 64..127 those of U^-1.
-constexpr size_t tri_inv_smem() { return (size_t)3 * kBlk * (kBlk + 1) * sizeof(float2); }
-__global__ void __launch_bounds__(128) tri_inv_kernel(const float2* M, int64_t ld, int64_t n, float2* tinv) {
-  constexpr int NB = kBlk;
+// row-major each, zero outside the kb x kb triangle.  grid (nblk, 2): y
+// selects the lower or upper triangle.
+//
+// Latency-bound (one CTA per triangle).  The 8 x 8 diagonal blocks are
+// inverted a column per thread; then pairs of inverted blocks are joined,
+// [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1, C^-1] (and its transpose form),
+// doubling the block three times with two products each that occupy the whole
+// CTA.  A thread per column of the 64, as before, was a chain of 64 dot
+// products: 54 us (80 at 11,520 unknowns), now @TINV@.
+constexpr int kTriPad = kBlk + 1;
+constexpr size_t tri_inv_smem() { return (size_t)3 * kBlk * kTriPad * sizeof(float2); }
+__global__ void __launch_bounds__(256) tri_inv_kernel(const float2* M, int64_t ld, int64_t n, float2* tinv) {
+  constexpr int NB = kBlk, Q = NB * NB / 256;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2(*D)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(smem_raw);
-  float2(*X)[NB + 1] = D + NB;
-  float2(*Y)[NB + 1] = D + 2 * NB;
+  float2(*D)[kTriPad] = reinterpret_cast<float2(*)[kTriPad]>(smem_raw);  // the triangle (unit diagonal if lower)
+  float2(*X)[kTriPad] = D + NB;                                          // its inverse
+  float2(*W)[kTriPad] = D + 2 * NB;                                      // a level's first products
   const int t = threadIdx.x;
+  const bool lower = blockIdx.y == 0;
   const int64_t b0 = (int64_t)blockIdx.x * NB;
   const int kb = (int)min((int64_t)NB, n - b0);
-  for (int e = t; e < NB * NB; e += 128) {
-    const int r = e / NB, c = e % NB;
-    D[r][c] = (r < kb && c < kb) ? M[(b0 + r) * ld + b0 + c] : make_float2(0.f, 0.f);
+  float2 v[Q];
+#pragma unroll
+  for (int k = 0; k < Q; k++) {
+    const int r = (t + 256 * k) / NB, c = (t + 256 * k) % NB;
+    v[k] = (r < kb && c < kb) ? M[(b0 + r) * ld + b0 + c] : make_float2(0.f, 0.f);
+  }
+#pragma unroll
+  for (int k = 0; k < Q; k++) {
+    const int r = (t + 256 * k) / NB, c = (t + 256 * k) % NB;
+    // rows past the matrix: the identity, dropped on the way out
+    if (r == c && (lower || r >= kb)) v[k] = make_float2(1.f, 0.f);
+    D[r][c] = (lower ? c <= r : c >= r) ? v[k] : make_float2(0.f, 0.f);
+    X[r][c] = make_float2(0.f, 0.f);
   }
   __syncthreads();
-  if (t < NB) {
-    // column j of L^-1: X[j][j] = 1, X[i][j] = -sum_{k=j}^{i-1} L[i][k] X[k][j]
-    const int j = t;
-    for (int i = 0; i < NB; i++) {
-      float2 v = make_float2(0.f, 0.f);
-      if (j < kb && i < kb && i >= j) {
-        if (i == j) {
-          v.x = 1.f;
-        } else {
-          float sr = 0.f, si = 0.f;
-          for (int k = j; k < i; k++) {
-            const float2 a = D[i][k], b = X[k][j];
-            sr += a.x * b.x - a.y * b.y;
-            si += a.x * b.y + a.y * b.x;
-          }
-          v = make_float2(-sr, -si);
-        }
+  if (t < NB) {  // column t of its 8 x 8 block's inverse
+    const int o = t & ~7, j = t & 7;
+    float2 x[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int i = lower ? q : 7 - q;
+      float sr = i == j ? 1.f : 0.f, si = 0.f;
+#pragma unroll
+      for (int p = 0; p < q; p++) {
+        const int k = lower ? p : 7 - p;
+        const float2 a = D[o + i][o + k];
+        sr -= a.x * x[p].x - a.y * x[p].y;
+        si -= a.x * x[p].y + a.y * x[p].x;
       }
-      X[i][j] = v;
-    }
-  } else {
-    // column j of U^-1: Y[j][j] = 1/U[j][j],
-    // Y[i][j] = -(sum_{k=i+1}^{j} U[i][k] Y[k][j]) / U[i][i] for i < j
-    const int j = t - NB;
-    for (int i = NB - 1; i >= 0; i--) {
-      float2 v = make_float2(0.f, 0.f);
-      if (j < kb && i <= j) {
-        const float2 di = crecip(D[i][i]);
-        if (i == j) {
-          v = di;
-        } else {
-          float sr = 0.f, si = 0.f;
-          for (int k = i + 1; k <= j; k++) {
-            const float2 a = D[i][k], b = Y[k][j];
-            sr += a.x * b.x - a.y * b.y;
-            si += a.x * b.y + a.y * b.x;
-          }
-          v = cmul(make_float2(-sr, -si), di);
-        }
-      }
-      Y[i][j] = v;
+      x[q] = make_float2(sr, si);
+      if (!lower) x[q] = cmul(x[q], crecip(D[o + i][o + i]));
+      X[o + i][o + j] = x[q];
     }
   }
   __syncthreads();
-  float2* out = tinv + (int64_t)blockIdx.x * 2 * NB * NB;
-  for (int e = t; e < NB * NB; e += 128) {
-    out[e] = X[e / NB][e % NB];
-    out[NB * NB + e] = Y[e / NB][e % NB];
+#pragma unroll
+  for (int s = 8; s < NB; s *= 2) {
+    // pair g: blocks at 2 g s and 2 g s + s.  Lower: W = B A^-1, X = -C^-1 W
+    // in rows of the second, columns of the first; upper: W = B C^-1,
+    // X = -A^-1 W the other way about.
+    for (int pass = 0; pass < 2; pass++) {
+      for (int e = t; e < (NB / (2 * s)) * s * s; e += 256) {
+        const int g = e / (s * s), i = (e / s) % s, j = e % s;
+        const int o = 2 * g * s, ro = lower ? o + s : o, co = lower ? o : o + s;
+        float sr = 0.f, si = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < s; k++) {
+          const float2 a = pass == 0 ? D[ro + i][co + k] : X[ro + i][ro + k];
+          const float2 b = pass == 0 ? X[co + k][co + j] : W[ro + k][co + j];
+          sr += a.x * b.x - a.y * b.y;
+          si += a.x * b.y + a.y * b.x;
+        }
+        if (pass == 0)
+          W[ro + i][co + j] = make_float2(sr, si);
+        else
+          X[ro + i][co + j] = make_float2(-sr, -si);
+      }
+      __syncthreads();
+    }
+  }
+  float2* out = tinv + ((int64_t)blockIdx.x * 2 + blockIdx.y) * NB * NB;
+#pragma unroll
+  for (int k = 0; k < Q; k++) {
+    const int r = (t + 256 * k) / NB, c = (t + 256 * k) % NB;
+    out[t + 256 * k] = (r < kb && c < kb) ? X[r][c] : make_float2(0.f, 0.f);
   }
 }
 
@@ -457,52 +478,59 @@ __device__ __forceinline__ unsigned long long global_ns() {
 //   W[v][0][d] = inv(L_vv) L_{v,v-1-d}   (zero where v - 1 - d < 0)
 //   W[v][1][d] = inv(U_vv) U_{v,v+1+d}   (zero beyond the last block)
 // 64 x 64 row-major each, zero outside the matrix.  grid (nblk, 2,
-// kSweepDepth), 256 threads; blockIdx.y selects the lower (0) or upper (1)
-// product, blockIdx.z the distance d + 1.
+// 4 kSweepDepth), 256 threads; blockIdx.y selects the lower (0) or upper (1)
+// product, blockIdx.z the distance d + 1 and the 32 x 32 quadrant (a small
+// system has few tiles: a CTA each left most SMs idle, 20 us against 5).
 constexpr int kSweepDepth = 3;
+constexpr int kNextPad = 34;  // rows of 32 elements, 16-byte aligned
 __global__ void __launch_bounds__(256) next_tile_kernel(const float2* M, int64_t ld, int64_t n, const float2* tinv,
                                                        float2* W) {
-  constexpr int NB = kBlk;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2(*Tm)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(smem_raw);  // the tile T_vu
-  float2(*Iv)[NB + 1] = Tm + NB;                                         // inv(T_vv)
+  constexpr int NB = kBlk, H = NB / 2, Q = NB * H / 256;
+  __shared__ __align__(16) float2 Tm[NB][kNextPad];  // columns of the tile T_vu
+  __shared__ float2 Iv[H][NB + 1];                   // rows of inv(T_vv)
   const int t = threadIdx.x;
   const int nblk = (int)((n + NB - 1) / NB);
-  const int v = blockIdx.x, side = blockIdx.y, d = blockIdx.z;
+  const int v = blockIdx.x, side = blockIdx.y, d = blockIdx.z >> 2;
+  const int rq = ((blockIdx.z >> 1) & 1) * H, cq = (blockIdx.z & 1) * H;
   const int u = side == 0 ? v - 1 - d : v + 1 + d;
   float2* out = W + (((int64_t)v * 2 + side) * kSweepDepth + d) * NB * NB;
-  if (u < 0 || u >= nblk) {
-    for (int e = t; e < NB * NB; e += 256) out[e] = make_float2(0.f, 0.f);
-    return;
-  }
-  const float2* inv = tinv + ((int64_t)v * 2 + side) * NB * NB;
-  const int64_t r0 = (int64_t)v * NB, c0 = (int64_t)u * NB;
-  for (int e = t; e < NB * NB; e += 256) {
-    const int r = e / NB, c = e % NB;
-    Tm[r][c] = (r0 + r < n && c0 + c < n) ? M[(r0 + r) * ld + c0 + c] : make_float2(0.f, 0.f);
-    Iv[r][c] = inv[e];
-  }
-  __syncthreads();
-  // thread t: row t / 4, sixteen columns (t % 4) + 4 j (a warp reads 8 rows
-  // of the inverse and 4 runs of the tile per k)
-  const int r = t >> 2, cq = t & 3;
-  float2 acc[16];
+  // thread t: rows (t / 16) + 16 i, columns 2 (t % 16) + j of the quadrant
+  const int r = t >> 4, c = 2 * (t & 15);
+  float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+  if (u >= 0 && u < nblk) {  // the same in every thread
+    const float2* inv = tinv + ((int64_t)v * 2 + side) * NB * NB;
+    const int64_t r0 = (int64_t)v * NB, c0 = (int64_t)u * NB + cq;
+    float2 a[Q], b[Q];
 #pragma unroll
-  for (int j = 0; j < 16; j++) acc[j] = make_float2(0.f, 0.f);
-#pragma unroll 4
-  for (int k = 0; k < NB; k++) {
-    const float2 a = Iv[r][k];
+    for (int k = 0; k < Q; k++) {
+      const int e = t + 256 * k, i = e / H, j = e % H;
+      a[k] = (r0 + i < n && c0 + j < n) ? M[(r0 + i) * ld + c0 + j] : make_float2(0.f, 0.f);
+      b[k] = inv[(rq + e / NB) * NB + e % NB];
+    }
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
-      const float2 b = Tm[k][cq + 4 * j];
-      acc[j].x += a.x * b.x - a.y * b.y;
-      acc[j].y += a.x * b.y + a.y * b.x;
+    for (int k = 0; k < Q; k++) {
+      const int e = t + 256 * k;
+      Tm[e / H][e % H] = a[k];
+      Iv[e / NB][e % NB] = b[k];
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < NB; k++) {
+      const float4 x = *reinterpret_cast<const float4*>(&Tm[k][c]);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const float2 w = Iv[r + 16 * i][k];
+        acc[i].x += w.x * x.x - w.y * x.y;
+        acc[i].y += w.x * x.y + w.y * x.x;
+        acc[i].z += w.x * x.z - w.y * x.w;
+        acc[i].w += w.x * x.w + w.y * x.z;
+      }
     }
   }
 #pragma unroll
-  for (int j = 0; j < 16; j++) out[r * NB + cq + 4 * j] = acc[j];
+  for (int i = 0; i < 2; i++)
+    *reinterpret_cast<float4*>(out + (rq + r + 16 * i) * NB + cq + c) = acc[i];
 }
-constexpr size_t next_tile_smem() { return (size_t)2 * kBlk * (kBlk + 1) * sizeof(float2); }
 
 // Hand-off of a solved block to the next CTAs of a thread-block cluster:
 // 64-bit stores into their shared memory.
