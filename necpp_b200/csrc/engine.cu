@@ -248,6 +248,8 @@ struct necgpu_engine {
   double* d_refine = nullptr;
   double2* d_x2 = nullptr;
   bool use_dmma = true;  // FP64 trailing update on the FP64 tensor cores
+  bool panel_cluster = true;  // FP64 panels in one cluster where they fit
+  bool panel_cluster_attr = false;
   int64_t outer = 256;  // outer block of the block-pivoted mixed LU (multiple of 64)
   // mixed path: block-local pivoting first, full partial pivoting as fallback
   bool prefer_blockpiv = true;
@@ -894,6 +896,53 @@ __global__ void max_diff_kernel(const float2* a, const float2* b, int64_t ld, in
 }
 
 // ---------------- LU ----------------
+// The FP64 panel at k0 in one cluster (panel_cluster_kernel); *done stays
+// false when the device refuses the cluster (panel_kernel from then on).
+int launch_panel_cluster(necgpu_engine* e, double2* M, int64_t k0, int kb, bool* done) {
+  const int64_t m = e->n - k0;
+  PanelClusterArgs a{};
+  a.M = M;
+  a.ld = e->ld;
+  a.n = e->n;
+  a.k0 = k0;
+  a.kb = kb;
+  a.rpc = (int)((m + kPcCTAs - 1) / kPcCTAs);
+  a.piv = e->d_piv;
+  a.status = e->d_status;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(kPcCTAs);
+  cfg.blockDim = dim3(kPcThreads);
+  cfg.dynamicSmemBytes = panel_cluster_smem(a.rpc);
+  cfg.stream = e->stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kPcCTAs;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (!e->panel_cluster_attr) {
+    if (cudaFuncSetAttribute(panel_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(panel_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)panel_cluster_smem(kPcRows)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      e->panel_cluster = false;
+      return 0;
+    }
+    e->panel_cluster_attr = true;
+  }
+  const int kt = kbegin(e);
+  if (cudaLaunchKernelEx(&cfg, panel_cluster_kernel, a) != cudaSuccess) {
+    (void)cudaGetLastError();
+    e->panel_cluster = false;
+    return 0;
+  }
+  kend(e, kt, NECGPU_K_PANEL, 4.0 * (double)m * kb * kb, nullptr, "panel_cluster_kernel");
+  e->launches++;
+  *done = true;
+  return 0;
+}
+
 template <typename R, class F = tc::SplitBf16>
 int run_lu(necgpu_engine* e, typename cvec<R>::T* M) {
   using T = typename cvec<R>::T;
@@ -931,6 +980,9 @@ int run_lu(necgpu_engine* e, typename cvec<R>::T* M) {
   for (int64_t k0 = 0; k0 < n; k0 += kNB) {
     const int kb = (int)std::min<int64_t>(kNB, n - k0);
     const int64_t m = n - k0;
+    bool panel_done = false;
+    if constexpr (std::is_same<R, double>::value)
+      if (e->panel_cluster && m <= kPcMaxRows) TRY(launch_panel_cluster(e, M, k0, kb, &panel_done));
     int P = (int)std::min<int64_t>(Pmax, (m + 15) / 16);
     P = std::max(P, 1);
     int rpc = (int)((m + P - 1) / P);
@@ -940,9 +992,9 @@ int run_lu(necgpu_engine* e, typename cvec<R>::T* M) {
     pa.kb = kb;
     pa.rpc = rpc;
     const size_t smem = (size_t)rpc * row_bytes + 2 * row_bytes;
-    CUDA_TRY(cudaMemsetAsync(e->d_counter, 0, sizeof(unsigned), e->stream));
     void* args[] = {&pa};
-    {
+    if (!panel_done) {
+      CUDA_TRY(cudaMemsetAsync(e->d_counter, 0, sizeof(unsigned), e->stream));
       // panel: m x kb unblocked LU, ~8 m kb^2 / 2 real flops
       const int kt = kbegin(e);
       CUDA_TRY(cudaLaunchCooperativeKernel((const void*)panel_kernel<R, kNB>, dim3(P), dim3(kPanelThreads),

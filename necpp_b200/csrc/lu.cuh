@@ -86,6 +86,235 @@ struct PanelArgs {
 constexpr int kPanelThreads = 256;
 constexpr long long kBarrierSpinLimit = 1LL << 26;
 
+// FP64 panel of up to kPcMaxRows rows in one cluster of 16 CTAs: the m x kb
+// panel (partial pivoting over the whole column) in their shared memory.
+//
+// Latency-bound: 64 columns, each a search over all rows and an exchange.
+// Rows stay where they are: a pivot is chosen among the rows not used yet and
+// the rows go to their interchanged places at the end, so a column needs one
+// exchange.  The columns go in blocks of eight, held in registers, a row per
+// thread; each CTA sends its best row of the column (eight values) to every
+// other one and a cluster barrier orders them.  After eight columns the CTAs
+// that own the pivot rows send them whole, every CTA solves the block's U rows
+// and applies them to its rows (a product with inner dimension eight).
+// panel_kernel, one row range per SM with a grid barrier and three global
+// round trips per column, takes @PCOLD@ for 2,880 rows, this @PCNEW@.
+constexpr int kPcCTAs = 16, kPcThreads = 256, kPcSub = 8;
+constexpr int kPcStride = 64 + 1;  // row stride against bank conflicts
+constexpr int kPcRows = 206;       // rows per CTA that fit in 227 KB
+constexpr int64_t kPcMaxRows = (int64_t)kPcCTAs * kPcRows;
+struct PanelClusterArgs {
+  double2* M;
+  int64_t ld, n, k0;
+  int kb, rpc;
+  int* piv;
+  int* status;
+};
+constexpr size_t panel_cluster_smem(int rpc) { return (size_t)rpc * kPcStride * sizeof(double2); }
+
+__device__ __forceinline__ void st_peer_d2(unsigned addr, double2 v) {
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ unsigned pc_peer(const void* p, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+// the larger value, the lower row on ties
+__device__ __forceinline__ void pc_better(double& v, int& r, int& o, double ov, int orow, int oo) {
+  if (ov > v || (ov == v && orow < r)) {
+    v = ov;
+    r = orow;
+    o = oo;
+  }
+}
+
+__global__ void __launch_bounds__(kPcThreads, 1) panel_cluster_kernel(const __grid_constant__ PanelClusterArgs A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* S = reinterpret_cast<double2*>(smem_raw);  // [rpc][kPcStride]
+  __shared__ __align__(16) double2 seg[2][kPcCTAs][kPcSub];  // the CTAs' best rows of a column
+  __shared__ __align__(16) double2 cand[2][kPcCTAs];          // their |pivot|^2 and row number
+  __shared__ __align__(16) double2 prow[kPcSub][64];          // the block's pivot rows, then its U rows
+  __shared__ __align__(16) double2 mine_seg[kPcSub];
+  __shared__ double wv[kPcThreads / 32];
+  __shared__ int wr[kPcThreads / 32];
+  __shared__ int plist[64], pos[64], at[64];  // pivot rows; places of the top rows; rows at the top places
+  __shared__ int sstep[kPcThreads], frow[kPcThreads];
+  unsigned rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kb = A.kb;
+  const int64_t k0 = A.k0, rbeg = k0 + (int64_t)rank * A.rpc;
+  const int nr = (int)max((int64_t)0, min((int64_t)A.rpc, A.n - rbeg));
+  for (int e = tid; e < nr * 64; e += kPcThreads) {
+    const int r = e >> 6, c = e & 63;
+    if (c < kb) S[r * kPcStride + c] = A.M[(rbeg + r) * A.ld + k0 + c];
+  }
+  if (tid < 64) pos[tid] = at[tid] = tid;
+  const bool mine = tid < nr;
+  const int row = (int)(rbeg - k0) + tid;  // this thread's row, counted from k0
+  int step = -1;                           // the column it became the pivot of
+  // the interchange that brings pivot row p to place c (one thread; row p is
+  // where it started unless it was a top row that has been moved away)
+  auto interchange = [&](int c, int p) {
+    const int pp = p < kb ? pos[p] : p, x = at[c];
+    at[c] = p;
+    if (p < kb) pos[p] = c;
+    if (x != p) {
+      pos[x] = pp;
+      if (pp < kb) at[pp] = x;
+    }
+    if (rank == 0) A.piv[k0 + c] = (int)k0 + pp;
+  };
+  // every CTA has started (and staged its rows) before one writes to another
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (int sb = 0; sb < kb; sb += kPcSub) {
+    double2 a[kPcSub];
+#pragma unroll
+    for (int q = 0; q < kPcSub; q++)
+      a[q] = mine && sb + q < kb ? S[tid * kPcStride + sb + q] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int cl = 0; cl < kPcSub; cl++) {
+      const int c = sb + cl, slot = cl & 1;
+      if (c < kb) {  // the same in every thread
+        // this CTA's candidate: a NaN counts below every number
+        double v = -2.0;
+        int r = 0x7fffffff, o = 0;
+        if (mine && step < 0) {
+          v = a[cl].x * a[cl].x + a[cl].y * a[cl].y;
+          if (!(v == v)) v = -1.0;
+          r = row;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+          pc_better(v, r, o, __shfl_xor_sync(0xffffffffu, v, off), __shfl_xor_sync(0xffffffffu, r, off), 0);
+        if (lane == 0) {
+          wv[warp] = v;
+          wr[warp] = r;
+        }
+        __syncthreads();
+        v = wv[lane & 7];
+        r = wr[lane & 7];
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1)
+          pc_better(v, r, o, __shfl_xor_sync(0xffffffffu, v, off), __shfl_xor_sync(0xffffffffu, r, off), 0);
+        if (mine && step < 0 && row == r) {
+#pragma unroll
+          for (int q = 0; q < kPcSub; q++) mine_seg[q] = a[q];
+        }
+        __syncthreads();
+        if (tid < kPcCTAs * kPcSub)
+          st_peer_d2(pc_peer(&seg[slot][rank][tid & 7], tid >> 3), mine_seg[tid & 7]);
+        else if (tid < kPcCTAs * kPcSub + kPcCTAs)
+          st_peer_d2(pc_peer(&cand[slot][rank], tid - kPcCTAs * kPcSub), make_double2(v, (double)r));
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (tid == kPcThreads - 1 && c > 0) interchange(c - 1, plist[c - 1]);
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const double2 cv = cand[slot][lane & 15];
+        v = cv.x;
+        r = (int)cv.y;
+        o = lane & 15;
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1)
+          pc_better(v, r, o, __shfl_xor_sync(0xffffffffu, v, off), __shfl_xor_sync(0xffffffffu, r, off),
+                    __shfl_xor_sync(0xffffffffu, o, off));
+        if (tid == kPcThreads - 1) plist[c] = r;
+        double2 u[kPcSub];
+#pragma unroll
+        for (int q = cl; q < kPcSub; q++) u[q] = seg[slot][o][q];
+        if (!(v > 0.0)) {  // a column of zeros, or of NaNs
+          u[cl] = make_double2(1.0, 0.0);
+          if (rank == 0 && tid == 0) atomicOr(A.status, v == 0.0 ? kLuStatSingular : kLuStatNonFinite);
+        }
+        if (mine && step < 0) {
+          if (row == r) {
+            step = c;
+          } else {
+            const double2 l = cdiv(a[cl], u[cl]);
+            a[cl] = l;
+#pragma unroll
+            for (int q = cl + 1; q < kPcSub; q++) {
+              a[q].x -= l.x * u[q].x - l.y * u[q].y;
+              a[q].y -= l.x * u[q].y + l.y * u[q].x;
+            }
+          }
+        }
+      }
+    }
+    if (mine) {
+#pragma unroll
+      for (int q = 0; q < kPcSub; q++)
+        if (sb + q < kb) S[tid * kPcStride + sb + q] = a[q];
+    }
+    sstep[tid] = step;
+    const int w = kb - sb - kPcSub;
+    __syncthreads();
+    if (w <= 0) break;
+    // the block's pivot rows (from column sb on) to every CTA
+    for (int j = 0; j < kPcSub; j++) {
+      const int64_t r = k0 + plist[sb + j] - rbeg;
+      if (r < 0 || r >= nr) continue;
+      for (int e = tid; e < kPcCTAs * 64; e += kPcThreads) {
+        const int q = e & 63;
+        if (sb + q < kb) st_peer_d2(pc_peer(&prow[j][q], e >> 6), S[r * kPcStride + sb + q]);
+      }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < w) {
+      double2 u[kPcSub];
+#pragma unroll
+      for (int j = 0; j < kPcSub; j++) {
+        u[j] = prow[j][kPcSub + tid];
+#pragma unroll
+        for (int i = 0; i < j; i++) {
+          const double2 l = prow[j][i];
+          u[j].x -= l.x * u[i].x - l.y * u[i].y;
+          u[j].y -= l.x * u[i].y + l.y * u[i].x;
+        }
+      }
+#pragma unroll
+      for (int j = 1; j < kPcSub; j++) prow[j][kPcSub + tid] = u[j];
+    }
+    __syncthreads();
+    {
+      // rows over threads; with few rows the columns are shared out too
+      const int rp = max(32, (nr + 31) / 32 * 32), G = kPcThreads / rp;
+      const int r = tid % rp, g = tid / rp;
+      if (r < nr && g < G) {
+        const int st = sstep[r];
+        double2* s = S + r * kPcStride + sb + kPcSub;
+        if (st < 0) {
+          double2 l[kPcSub];
+#pragma unroll
+          for (int j = 0; j < kPcSub; j++) l[j] = S[r * kPcStride + sb + j];
+#pragma unroll 2
+          for (int q = g; q < w; q += G) {
+            double2 v = s[q];
+#pragma unroll
+            for (int j = 0; j < kPcSub; j++) {
+              const double2 u = prow[j][kPcSub + q];
+              v.x -= l[j].x * u.x - l[j].y * u.y;
+              v.y -= l[j].x * u.y + l[j].y * u.x;
+            }
+            s[q] = v;
+          }
+        } else if (st >= sb) {
+          for (int q = g; q < w; q += G) s[q] = prow[st - sb][kPcSub + q];
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (tid == kPcThreads - 1) interchange(kb - 1, plist[kb - 1]);
+  __syncthreads();
+  if (mine) frow[tid] = step >= 0 ? step : row < kb ? pos[row] : row;
+  __syncthreads();
+  for (int e = tid; e < nr * 64; e += kPcThreads) {
+    const int r = e >> 6, c = e & 63;
+    if (c < kb) A.M[(k0 + frow[r]) * A.ld + k0 + c] = S[r * kPcStride + c];
+  }
+}
+
 template <typename R, int NB>
 __global__ void __launch_bounds__(kPanelThreads) panel_kernel(PanelArgs<R> A) {
   using T = typename cvec<R>::T;
