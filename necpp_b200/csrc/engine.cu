@@ -64,6 +64,13 @@ struct necgpu_engine {
 
   FieldParams P{};
   int ground = 0, use_exk = 0;
+  // structure tables: one device block (d_struct) that the pointers below
+  // divide, filled by one copy from the pinned staging buffer
+  unsigned char* d_struct = nullptr;
+  size_t struct_cap = 0;
+  double* h_pin = nullptr;           // pinned, 16 doubles: status words and small results
+  unsigned char* h_stage = nullptr;  // pinned; read by the copy of the last necgpu_set_structure
+  size_t stage_cap = 0;
   double* d_seg = nullptr;  // 8n: x y z s b cab sab salp
   int32_t* d_ind = nullptr; // 2n
   // the fill's column blocks (FillLists) and its cut into CTAs
@@ -423,16 +430,10 @@ void free_all(necgpu_engine* e) {
   }
   e->lu_seen = LuGraphKey{};
   e->lu_key = LuGraphKey{};
-  dfree(e, e->d_seg);
-  dfree(e, e->d_ind);
-  dfree(e, e->d_blk_ptr);
-  dfree(e, e->d_fsrc);
-  dfree(e, e->d_col_ptr);
-  dfree(e, e->d_eloc);
-  dfree(e, e->d_ecoef);
-  dfree(e, e->d_cptr);
-  dfree(e, e->d_cbasis);
-  dfree(e, e->d_ccoef);
+  dfree(e, e->d_struct);
+  e->struct_cap = 0;
+  e->d_seg = e->d_ecoef = e->d_ccoef = nullptr;
+  e->d_ind = e->d_blk_ptr = e->d_fsrc = e->d_col_ptr = e->d_eloc = e->d_cptr = e->d_cbasis = nullptr;
   dfree(e, e->Z64);
   dfree(e, e->d_dinv);
   dfree(e, e->d_top_cnt);
@@ -516,12 +517,11 @@ void free_all(necgpu_engine* e) {
 void kflush(necgpu_engine* e);
 
 int sync_status(necgpu_engine* e, int* out) {
-  int h[4];
-  CUDA_TRY(cudaMemcpyAsync(h, e->d_status, sizeof(h), cudaMemcpyDeviceToHost, e->stream));
+  CUDA_TRY(cudaMemcpyAsync(e->h_pin, e->d_status, 4 * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
   CUDA_TRY(cudaStreamSynchronize(e->stream));
-  e->stats.d2h_bytes += sizeof(h);
+  e->stats.d2h_bytes += 4 * sizeof(int);
   kflush(e);
-  *out = h[0];
+  *out = *reinterpret_cast<int*>(e->h_pin);
   return 0;
 }
 
@@ -1057,6 +1057,8 @@ int run_lu(necgpu_engine* e, typename cvec<R>::T* M) {
   return 0;
 }
 
+int invert_diag_blocks(necgpu_engine* e, bool force = false);
+
 // FP32 LU with block-local pivoting (mixed path): per 64-column panel, one
 // CTA factors the diagonal block, the exchanges are a per-column gather
 // inside the block, L21 and U12 are row/column-parallel triangular solves,
@@ -1481,19 +1483,15 @@ int run_lu_blockpiv(necgpu_engine* e, float2* M) {
     TRY(issue());
     e->lu_seen = key;
   }
-  std::vector<int> piv(n), perm(n);
-  CUDA_TRY(cudaMemcpyAsync(piv.data(), e->d_piv, n * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-  e->stats.d2h_bytes += n * sizeof(int);
+  // the permutation from the blocks' row orders, and what the sweeps need of
+  // the factors, before the one wait (dropped by the caller when a block had
+  // no usable pivot)
+  if (!e->d_perm) TRY(dalloc(e, e->d_perm, (size_t)n));
+  KLAUNCH(NECGPU_K_OTHER, 0.0,
+          block_perm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, e->stream>>>(e->d_src, e->d_perm, n));
+  TRY(invert_diag_blocks(e));
   int st = 0;
   TRY(sync_status(e, &st));
-  for (int64_t i = 0; i < n; i++) perm[i] = (int)i;
-  for (int64_t k = 0; k < n; k++) {
-    int p = piv[k];
-    if (p < 0 || p >= n) return fail(e, NECGPU_ERR_NONFINITE, "LU: invalid pivot index");
-    std::swap(perm[k], perm[p]);
-  }
-  TRY(upload(e, e->d_perm, perm.data(), perm.size()));
-  CUDA_TRY(cudaStreamSynchronize(e->stream));
   if (st & tc::kStatTimeout) return fail(e, NECGPU_ERR_CUDA, "LU: tensor-core update pipeline timed out");
   if (st & kLuStatNonFinite) return fail(e, NECGPU_ERR_NONFINITE, "LU: NaN/Inf in the matrix");
   if (st & kLuStatSingular) return fail(e, NECGPU_ERR_SINGULAR, "LU: zero pivot in a diagonal block");
@@ -1583,7 +1581,7 @@ int ensure_vectors(necgpu_engine* e) {
 
 // Inverses of the 64 x 64 diagonal blocks of the complex64 factors, for the
 // refinement sweeps (one CTA per block, all blocks at once).
-int invert_diag_blocks(necgpu_engine* e, bool force = false) {
+int invert_diag_blocks(necgpu_engine* e, bool force) {
   if (!e->inv_sweep && !force) return 0;
   const int64_t nblk = (e->n + kBlk - 1) / kBlk;
   if (!e->d_tinv) TRY(dalloc(e, e->d_tinv, (size_t)nblk * 2 * kBlk * kBlk));
@@ -1742,16 +1740,13 @@ int refine_fused(necgpu_engine* e, const double2* b, double2* x, double2* r, int
     return 0;
   }
   e->launches++;
-  double out[2] = {0, 0};
-  int st = 0;
-  CUDA_TRY(cudaMemcpyAsync(out, a.out, sizeof out, cudaMemcpyDeviceToHost, e->stream));
-  CUDA_TRY(cudaMemcpyAsync(&st, e->d_status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+  CUDA_TRY(cudaMemcpyAsync(e->h_pin, a.out, 3 * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
   CUDA_TRY(cudaStreamSynchronize(e->stream));
-  e->stats.d2h_bytes += sizeof out + sizeof st;
+  e->stats.d2h_bytes += 3 * sizeof(double);
   *done = true;
-  *iters = (int)out[0];
-  *rel = out[1];
-  if (st & (1 << 9)) return fail(e, NECGPU_ERR_CUDA, "refinement: triangular sweep gave up waiting on a block");
+  *iters = (int)e->h_pin[0];
+  *rel = e->h_pin[1];
+  if ((int)e->h_pin[2] & (1 << 9)) return fail(e, NECGPU_ERR_CUDA, "refinement: triangular sweep gave up waiting on a block");
   if (!std::isfinite(*rel))
     return fail(e, NECGPU_ERR_NONFINITE, ADJ ? "adjoint: non-finite residual" : "refinement: non-finite residual");
   return 0;
@@ -1782,7 +1777,7 @@ int factor_mixed(necgpu_engine* e, bool blockpiv) {
   e->tc_format_used = fmt;
   if (blockpiv) {
     const int rc = fmt == 2 ? run_lu_blockpiv<tc::Tf32>(e, e->Z32) : run_lu_blockpiv<tc::SplitBf16>(e, e->Z32);
-    if (rc != NECGPU_ERR_SINGULAR && rc != NECGPU_ERR_NONFINITE) return rc ? rc : invert_diag_blocks(e);
+    if (rc != NECGPU_ERR_SINGULAR && rc != NECGPU_ERR_NONFINITE) return rc;
     // a diagonal block without a usable pivot: full partial pivoting
     CUDA_TRY(cudaMemsetAsync(e->d_status, 0, 4 * sizeof(int), e->stream));
     return factor_mixed(e, false);
@@ -2317,6 +2312,7 @@ int necgpu_create(necgpu_engine** out, int device) {
       CUDA_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
     }
   }
+  CUDA_TRY(cudaMallocHost((void**)&e->h_pin, 16 * sizeof(double)));
   TRY(dalloc(e, e->d_status, 4));
   CUDA_TRY(cudaMemsetAsync(e->d_status, 0, 4 * sizeof(int), e->stream));
   return NECGPU_OK;
@@ -2329,6 +2325,8 @@ int necgpu_destroy(necgpu_engine* e) {
     cudaStreamSynchronize(e->stream);
   }
   free_all(e);
+  if (e->h_stage) cudaFreeHost(e->h_stage);
+  if (e->h_pin) cudaFreeHost(e->h_pin);
   dfree(e, e->d_interp_carry);  // the interpolation cache lives as long as the engine
   dfree(e, e->d_status);
   if (e->ev0) cudaEventDestroy(e->ev0);
@@ -2572,18 +2570,49 @@ int necgpu_set_structure(necgpu_engine* e, const necgpu_structure* s) {
   e->h_tbasis.assign(s->trio_basis, s->trio_basis + ntrio);
   e->h_ind = ind;
 
-  TRY(upload(e, e->d_seg, seg.data(), seg.size()));
-  TRY(upload(e, e->d_ind, ind.data(), ind.size()));
-  TRY(upload(e, e->d_blk_ptr, FL.blk_ptr.data(), FL.blk_ptr.size()));
-  TRY(upload(e, e->d_fsrc, FL.src.data(), FL.src.size()));
-  TRY(upload(e, e->d_col_ptr, FL.col_ptr.data(), FL.col_ptr.size()));
-  TRY(upload(e, e->d_eloc, FL.eloc.data(), FL.eloc.size()));
-  TRY(upload(e, e->d_ecoef, FL.ecoef.data(), FL.ecoef.size()));
-  TRY(upload(e, e->d_cptr, cptr.data(), cptr.size()));
-  TRY(upload(e, e->d_cbasis, cbasis.data(), cbasis.size()));
-  TRY(upload(e, e->d_ccoef, ccoef.data(), ccoef.size()));
+  // one staged copy: ten pageable copies cost more host time than a small
+  // structure's fill and factorisation take on the device
+  struct Part {
+    void** p;
+    const void* h;
+    size_t bytes;
+  };
+  const Part parts[] = {{(void**)&e->d_seg, seg.data(), seg.size() * sizeof(double)},
+                        {(void**)&e->d_ecoef, FL.ecoef.data(), FL.ecoef.size() * sizeof(double)},
+                        {(void**)&e->d_ccoef, ccoef.data(), ccoef.size() * sizeof(double)},
+                        {(void**)&e->d_ind, ind.data(), ind.size() * sizeof(int32_t)},
+                        {(void**)&e->d_blk_ptr, FL.blk_ptr.data(), FL.blk_ptr.size() * sizeof(int32_t)},
+                        {(void**)&e->d_fsrc, FL.src.data(), FL.src.size() * sizeof(int32_t)},
+                        {(void**)&e->d_col_ptr, FL.col_ptr.data(), FL.col_ptr.size() * sizeof(int32_t)},
+                        {(void**)&e->d_eloc, FL.eloc.data(), FL.eloc.size() * sizeof(int32_t)},
+                        {(void**)&e->d_cptr, cptr.data(), cptr.size() * sizeof(int32_t)},
+                        {(void**)&e->d_cbasis, cbasis.data(), cbasis.size() * sizeof(int32_t)}};
+  constexpr size_t kAlign = 256;
+  size_t total = 0;
+  for (const Part& q : parts) total += (q.bytes + kAlign - 1) / kAlign * kAlign;
+  if (e->stage_cap < total) {
+    if (e->h_stage) cudaFreeHost(e->h_stage);
+    e->h_stage = nullptr;
+    e->stage_cap = 0;
+    const size_t cap = std::max<size_t>(total, 1 << 18);
+    CUDA_TRY(cudaMallocHost((void**)&e->h_stage, cap));
+    e->stage_cap = cap;
+  }
+  if (e->struct_cap < total) {
+    e->struct_cap = 0;
+    TRY(dalloc(e, e->d_struct, total));
+    e->struct_cap = total;
+  }
+  size_t off = 0;
+  for (const Part& q : parts) {
+    *q.p = e->d_struct + off;
+    if (q.bytes) std::memcpy(e->h_stage + off, q.h, q.bytes);
+    off += (q.bytes + kAlign - 1) / kAlign * kAlign;
+  }
+  CUDA_TRY(cudaMemcpyAsync(e->d_struct, e->h_stage, total, cudaMemcpyHostToDevice, e->stream));
+  e->stats.h2d_bytes += total;
+  // the staging buffer is next written after the next call's wait for the stream
   TRY(ensure_vectors(e));
-  CUDA_TRY(cudaStreamSynchronize(e->stream));  // host staging freed on return
   return NECGPU_OK;
 }
 

@@ -261,6 +261,16 @@ __global__ void permute_kernel(const TI* src, const int* perm, TO* dst, int64_t 
   }
 }
 
+// perm[i]: the row of A that the block-pivoted LU has in row i, from the
+// diagonal blocks' row orders (in range whatever a block without a usable
+// pivot left there).
+__global__ void block_perm_kernel(const int* src, int* perm, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t k0 = i / kBlk * kBlk;
+  perm[i] = (int)(k0 + min((int64_t)max(src[i], 0), min((int64_t)kBlk, n - k0) - 1));
+}
+
 // x += d (d in the factor precision)
 template <typename TD>
 __global__ void axpy_kernel(double2* x, const TD* d, int64_t n) {
@@ -972,7 +982,7 @@ struct RefineArgs {
   int* status;
   double tol;
   int max_iter;
-  double* out;            // [0] steps, [1] final ||r|| / ||b||
+  double* out;            // [0] steps, [1] final ||r|| / ||b||, [2] the status word
 };
 struct RefineShared {
   SweepShared S;
@@ -1139,6 +1149,7 @@ __global__ void __launch_bounds__(kInvSweepThreads, 1) refine_kernel(const __gri
   if (rank == 0 && t == 0) {
     A.out[0] = it;
     A.out[1] = rel;
+    A.out[2] = (double)*(volatile int*)A.status;
   }
   cluster_sync_all();  // no CTA leaves while a peer may still write to it
 }
