@@ -87,16 +87,23 @@ def struct_array(structs):
     global _SDT
     if _SDT is None:
         _SDT = _struct_dtype()
-    out = _np.zeros(len(structs), dtype=_SDT)
     addr = lambda a: a.__array_interface__["data"][0]
-    for k, st in enumerate(structs):
-        n = st["n"]
-        seg, tabc, ind = addr(st["seg"]), addr(st["tabc"]), addr(st["ind"])
-        nt = len(st["tbasis"])
-        p = st["params"]
-        out[k] = (n, seg, seg + 8 * n, seg + 16 * n, seg + 24 * n, seg + 32 * n, seg + 40 * n, seg + 48 * n,
-                  seg + 56 * n, addr(st["tptr"]), addr(st["tbasis"]), tabc, tabc + 8 * nt, tabc + 16 * nt, ind,
-                  ind + 4 * n, p[0], int(p[1]), int(p[2]), p[3], p[4], p[5], p[6], p[7])
+    n = _np.fromiter((st["n"] for st in structs), dtype=_np.uint64, count=len(structs))
+    nt = _np.fromiter((len(st["tbasis"]) for st in structs), dtype=_np.uint64, count=len(structs))
+    at = {k: _np.fromiter((addr(st[k]) for st in structs), dtype=_np.uint64, count=len(structs))
+          for k in ("seg", "tabc", "ind", "tptr", "tbasis")}
+    par = _np.array([st["params"] for st in structs])
+    out = _np.zeros(len(structs), dtype=_SDT)
+    out["n"] = n
+    for k, name in enumerate(("x", "y", "z", "length", "radius", "cab", "sab", "salp")):
+        out[name] = at["seg"] + _np.uint64(8 * k) * n
+    out["trio_ptr"], out["trio_basis"] = at["tptr"], at["tbasis"]
+    for k, name in enumerate(("trio_a", "trio_b", "trio_c")):
+        out[name] = at["tabc"] + _np.uint64(8 * k) * nt
+    out["ek_ind1"], out["ek_ind2"] = at["ind"], at["ind"] + _np.uint64(4) * n
+    for k, name in ((0, "rkh"), (1, "use_exk"), (2, "ground"), (3, "zrati_re"), (4, "zrati_im"), (5, "frati_re"),
+                    (6, "frati_im"), (7, "eta")):
+        out[name] = par[:, k]
     return out
 
 

@@ -3,6 +3,8 @@
 // fill, LU, refined solve, current coefficients and far field are the
 // single-problem path's, but the work of all problems shares each launch:
 //
+//   batch_tables_kernel   basis tables -> the lists of the fill and the
+//                         coefficients, one CTA per problem
 //   batch_fill_kernel     one CTA per few rows of a problem, through the
 //                         single-problem fill_rows
 //   batch_lu_solve_kernel persistent: a CTA takes the next problem (largest
@@ -44,6 +46,122 @@ __global__ void __launch_bounds__(kFillThreads, GROUND == kGroundNone && !EXK ? 
     batch_fill_kernel(const FillArgs* __restrict__ As, const int4* __restrict__ items) {
   const int4 it = items[blockIdx.x];
   fill_rows<GROUND, EXK, false>(As[it.x], ContractArgs{}, it.z >> 16, it.y, it.z & 0xffff, it.w);
+}
+
+// The lists that the fill and the current coefficients read, from each
+// problem's basis tables (the device form of build_fill_lists and
+// build_coef_lists): one CTA per problem.  The host then only gathers the
+// tables: of a sweep of 1,024 problems (n = 33..615) the host's share of the
+// call fell from 35 to 4 ms, for 0.1 ms here, bound by the column scans.
+constexpr int kBatchBlocks = (kBatchMaxN + kFillBlock - 1) / kFillBlock;  // most column blocks of a problem
+struct BatchTables {
+  // in: per problem its entries' offset and, at v + problem, its n + 1 trio
+  // pointers; the entries of all problems one after the other
+  const int64_t* eoff;
+  const int32_t *tptr, *tbasis;
+  const double *ta, *tb, *tc;
+  const int* cols;  // columns per block
+  // out, fill: block pointers (kBatchBlocks + 1 per problem), sources and
+  // entries at the problem's entry offset, column pointers at v + problem
+  int32_t *blk_ptr, *src, *col_ptr, *eloc;
+  double *ea, *eb, *ec;
+  // out, coefficients: per segment its entries by ascending basis (cptr runs
+  // over all problems)
+  int32_t *cptr, *cbasis;
+  double *ca, *cb, *cc;
+};
+constexpr int kBatchTableThreads = 256;
+__global__ void __launch_bounds__(kBatchTableThreads)
+    batch_tables_kernel(const BatchProblem* __restrict__ probs, const __grid_constant__ BatchTables B) {
+  __shared__ int16_t loc[kBatchBlocks][kBatchMaxN];  // a source's place in each block's list
+  __shared__ int count[kBatchMaxN + 1];
+  __shared__ int warps[kBatchTableThreads / 32];
+  const int p = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const BatchProblem pr = probs[p];
+  const int n = pr.n, cols = B.cols[p], nblk = (n + cols - 1) / cols;
+  const int64_t e0 = B.eoff[p], v0 = pr.v + p;
+  const int32_t* tp = B.tptr + v0;
+  const int32_t* basis = B.tbasis + e0;
+  // exclusive scan of one value per thread; the total in *sum
+  auto scan = [&](int x, int* sum) {
+    int y = x;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int z = __shfl_up_sync(0xffffffffu, y, off);
+      if (lane >= off) y += z;
+    }
+    __syncthreads();  // the previous call's sums have been read
+    if (lane == 31) warps[warp] = y;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int w = 0; w < kBatchTableThreads / 32; w++) {
+      before += w < warp ? warps[w] : 0;
+      all += warps[w];
+    }
+    *sum = all;
+    return before + y - x;
+  };
+  // distinct sources of every block, ascending
+  int at = 0;
+  for (int b = 0; b < nblk; b++) {
+    if (t == 0) B.blk_ptr[(int64_t)p * (kBatchBlocks + 1) + b] = at;
+    const int first = at;
+    for (int j0 = 0; j0 < n; j0 += kBatchTableThreads) {
+      const int j = j0 + t;
+      bool has = false;
+      if (j < n)
+        for (int k = tp[j]; k < tp[j + 1]; k++) has = has || basis[k] / cols == b;
+      int sum;
+      const int q = scan(has ? 1 : 0, &sum);
+      if (has) {
+        B.src[e0 + at + q] = j;
+        loc[b][j] = (int16_t)(at + q - first);
+      }
+      at += sum;
+    }
+  }
+  if (t == 0) B.blk_ptr[(int64_t)p * (kBatchBlocks + 1) + nblk] = at;
+  // entries per column, then each column's by ascending source
+  for (int c = t; c <= n; c += kBatchTableThreads) count[c] = 0;
+  __syncthreads();
+  const int ne = tp[n];
+  for (int k = t; k < ne; k += kBatchTableThreads) atomicAdd(&count[basis[k]], 1);
+  __syncthreads();
+  int base = 0;
+  for (int c0 = 0; c0 < n; c0 += kBatchTableThreads) {
+    const int c = c0 + t;
+    int sum;
+    const int q = base + scan(c < n ? count[c] : 0, &sum);
+    base += sum;
+    if (c < n) {
+      B.col_ptr[v0 + c] = q;
+      int w = q;
+      const int b = c / cols;
+      for (int j = 0; j < n; j++)  // the same j and k in every thread
+        for (int k = tp[j]; k < tp[j + 1]; k++)
+          if (basis[k] == c) {
+            B.eloc[e0 + w] = loc[b][j];
+            B.ea[e0 + w] = B.ta[e0 + k];
+            B.eb[e0 + w] = B.tb[e0 + k];
+            B.ec[e0 + w] = B.tc[e0 + k];
+            w++;
+          }
+    }
+  }
+  if (t == 0) B.col_ptr[v0 + n] = ne;
+  // a segment's entries by ascending basis, equal ones in table order
+  for (int j = t; j < n; j += kBatchTableThreads) {
+    const int k0 = tp[j], k1 = tp[j + 1];
+    B.cptr[pr.v + j] = (int32_t)(e0 + k0);
+    for (int k = k0; k < k1; k++) {
+      int q = k0;
+      for (int i = k0; i < k1; i++) q += basis[i] < basis[k] || (basis[i] == basis[k] && i < k);
+      B.cbasis[e0 + q] = basis[k];
+      B.ca[e0 + q] = B.ta[e0 + k];
+      B.cb[e0 + q] = B.tb[e0 + k];
+      B.cc[e0 + q] = B.tc[e0 + k];
+    }
+  }
 }
 
 // CTA-wide argmax of key (>= 0 candidates; -1 none), lowest row on ties.
@@ -449,6 +567,7 @@ __global__ void batch_gain_norm_kernel(int nprob, const int64_t* seg_off, const 
 
 struct BatchPatternArgs {
   int nprob, ndir;
+  int p0;                  // first problem of the launch
   const double *theta, *phi;
   const int64_t* seg_off;  // nprob + 1
   const double* seg;       // 8 x nseg_total (x y z s b cab sab salp)
@@ -465,7 +584,7 @@ struct BatchPatternArgs {
 template <int DW>
 __global__ void __launch_bounds__(kPatDirs * 32, 2) batch_pattern_kernel(const __grid_constant__ BatchPatternArgs A) {
   __shared__ SegPat seg[kPatChunk];
-  const int p = blockIdx.y;
+  const int p = A.p0 + blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int d0 = (blockIdx.x * kPatDirs + warp) * DW;
   const int64_t s0 = A.seg_off[p], ns = A.seg_off[p + 1] - s0;

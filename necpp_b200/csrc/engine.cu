@@ -10,14 +10,15 @@
 #include <cstdlib>
 #include <type_traits>
 #include <cstring>
+#include <limits>
 #include <mutex>
-#include <atomic>
 #include <thread>
 #include <numeric>
 #include <string>
 #include <vector>
 
 #include "../../include/necgpu.h"
+#include "host_parallel.h"
 #include "fill.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_dmma.cuh"
@@ -2223,6 +2224,78 @@ void build_coef_lists(const necgpu_structure* s, int64_t n, CoefLists& C) {
   C.cptr[n] = tp[n];
 }
 
+// Pinned staging buffer of at least `bytes` (its last copy must have finished).
+int ensure_stage(necgpu_engine* e, size_t bytes) {
+  if (e->stage_cap >= bytes) return 0;
+  if (e->h_stage) cudaFreeHost(e->h_stage);
+  e->h_stage = nullptr;
+  e->stage_cap = 0;
+  const size_t cap = std::max<size_t>(bytes, 1 << 18);
+  CUDA_TRY(cudaMallocHost((void**)&e->h_stage, cap));
+  e->stage_cap = cap;
+  return 0;
+}
+
+// The batch's tables (segments as eight arrays over all problems, end flags,
+// trio pointers, basis and a | b | c) gathered by the host cores into the
+// pinned buffer and copied, a range of problems at a time so that the buffer
+// stays within kBatchStage bytes.
+constexpr size_t kBatchStage = (size_t)64 << 20;
+int batch_upload_tables(necgpu_engine* e, int nprob, const necgpu_structure* structs, const std::vector<int64_t>& off,
+                        const std::vector<int64_t>& eoff, double* d_seg, int32_t* d_ind, int32_t* d_tptr,
+                        int32_t* d_tbasis, double* d_tabc, int workers) {
+  const int64_t T = off[nprob], E1 = std::max<int64_t>(eoff[nprob], 1);
+  CUDA_TRY(cudaStreamSynchronize(e->stream));  // the staging buffer's last copy
+  for (int p0 = 0; p0 < nprob;) {
+    auto bytes = [&](int p1) {
+      const int64_t n = off[p1] - off[p0], m = eoff[p1] - eoff[p0];
+      return (size_t)(8 * n + 3 * m) * sizeof(double) + (size_t)(3 * n + (p1 - p0) + m) * sizeof(int32_t);
+    };
+    int p1 = p0 + 1;
+    while (p1 < nprob && bytes(p1 + 1) <= kBatchStage) p1++;
+    TRY(ensure_stage(e, bytes(p1)));
+    const int64_t n = off[p1] - off[p0], m = eoff[p1] - eoff[p0], np = n + (p1 - p0);
+    double* seg = reinterpret_cast<double*>(e->h_stage);
+    double* abc = seg + 8 * n;
+    int32_t* ind = reinterpret_cast<int32_t*>(abc + 3 * m);
+    int32_t* tptr = ind + 2 * n;
+    int32_t* basis = tptr + np;
+    parallel_chunks(p1 - p0, workers, [&](int, int64_t q0, int64_t q1) {
+      for (int64_t q = p0 + q0; q < p0 + q1; q++) {
+        const necgpu_structure& s = structs[q];
+        const int64_t o = off[q] - off[p0], k = eoff[q] - eoff[p0], ns = s.n, ne = eoff[q + 1] - eoff[q];
+        const double* src[8] = {s.x, s.y, s.z, s.length, s.radius, s.cab, s.sab, s.salp};
+        for (int a = 0; a < 8; a++) std::copy(src[a], src[a] + ns, seg + a * n + o);
+        std::copy(s.trio_a, s.trio_a + ne, abc + k);
+        std::copy(s.trio_b, s.trio_b + ne, abc + m + k);
+        std::copy(s.trio_c, s.trio_c + ne, abc + 2 * m + k);
+        if (d_ind) {
+          const bool has = s.ek_ind1 && s.ek_ind2;
+          for (int64_t i = 0; i < ns; i++) {
+            ind[o + i] = has ? s.ek_ind1[i] : 0;
+            ind[n + o + i] = has ? s.ek_ind2[i] : 0;
+          }
+        }
+        std::copy(s.trio_ptr, s.trio_ptr + ns + 1, tptr + o + (q - p0));
+        std::copy(s.trio_basis, s.trio_basis + ne, basis + k);
+      }
+    });
+    auto copy = [&](void* d, const void* h, size_t b) {
+      e->stats.h2d_bytes += b;
+      return b ? cudaMemcpyAsync(d, h, b, cudaMemcpyHostToDevice, e->stream) : cudaSuccess;
+    };
+    for (int a = 0; a < 8; a++) CUDA_TRY(copy(d_seg + a * T + off[p0], seg + a * n, n * sizeof(double)));
+    for (int a = 0; a < 3; a++) CUDA_TRY(copy(d_tabc + a * E1 + eoff[p0], abc + a * m, m * sizeof(double)));
+    if (d_ind)
+      for (int a = 0; a < 2; a++) CUDA_TRY(copy(d_ind + a * T + off[p0], ind + a * n, n * sizeof(int32_t)));
+    CUDA_TRY(copy(d_tptr + off[p0] + p0, tptr, np * sizeof(int32_t)));
+    CUDA_TRY(copy(d_tbasis + eoff[p0], basis, m * sizeof(int32_t)));
+    p0 = p1;
+    if (p0 < nprob) CUDA_TRY(cudaStreamSynchronize(e->stream));  // the next range reuses the buffer
+  }
+  return 0;
+}
+
 }  // namespace
 
 extern "C" {
@@ -2590,14 +2663,7 @@ int necgpu_set_structure(necgpu_engine* e, const necgpu_structure* s) {
   constexpr size_t kAlign = 256;
   size_t total = 0;
   for (const Part& q : parts) total += (q.bytes + kAlign - 1) / kAlign * kAlign;
-  if (e->stage_cap < total) {
-    if (e->h_stage) cudaFreeHost(e->h_stage);
-    e->h_stage = nullptr;
-    e->stage_cap = 0;
-    const size_t cap = std::max<size_t>(total, 1 << 18);
-    CUDA_TRY(cudaMallocHost((void**)&e->h_stage, cap));
-    e->stage_cap = cap;
-  }
+  TRY(ensure_stage(e, total));
   if (e->struct_cap < total) {
     e->struct_cap = 0;
     TRY(dalloc(e, e->d_struct, total));
@@ -3378,82 +3444,35 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     z_off[p + 1] = z_off[p] + s.n * s.n;
   }
   const int64_t T = seg_off[nprob], Zt = z_off[nprob];
-  std::vector<double> seg(8 * T);
-  std::vector<int32_t> ind(2 * T, 0);
-  std::vector<int32_t> bp_pool, src_pool, cp_pool, eloc_pool, cptr_g(T + 1, 0), cbasis_pool;
-  std::vector<double> ecoef_pool, ca_pool, cb_pool, cc_pool;
-  std::vector<int64_t> bp_off(nprob), src_off(nprob), cp_off(nprob), el_off(nprob), ecf_off(nprob), ne_p(nprob);
-  std::vector<int> seg_prob(T);
-  // per-problem fill and coefficient lists on all host cores, then concatenated
-  std::vector<FillLists> FLs(nprob);
-  std::vector<CoefLists> CLs(nprob);
-  std::vector<int> bad(nprob, 0);
-  {
-    const int nth = std::max(1, std::min<int>((int)std::thread::hardware_concurrency(), 64));
-    std::atomic<int> nextp(0);
-    auto work = [&]() {
-      for (int p = nextp++; p < nprob; p = nextp++) {
-        const necgpu_structure& s = structs[p];
-        const int64_t n = s.n;
-        const int32_t* tp = s.trio_ptr;
-        bool ok = tp[0] == 0;
-        for (int64_t j = 0; ok && j < n; j++) ok = tp[j + 1] >= tp[j];
-        for (int64_t k = 0; ok && k < tp[n]; k++) ok = s.trio_basis[k] >= 0 && s.trio_basis[k] < n;
-        if (!ok) {
-          bad[p] = 1;
-          continue;
-        }
-        build_fill_lists(&s, n, fill_block_cols(n, tp[n]), FLs[p]);
-        build_coef_lists(&s, n, CLs[p]);
-      }
-    };
-    std::vector<std::thread> pool;
-    for (int i = 1; i < nth; i++) pool.emplace_back(work);
-    work();
-    for (auto& th : pool) th.join();
-  }
-  for (int p = 0; p < nprob; p++)
-    if (bad[p]) return fail(e, NECGPU_ERR_ARG, "batch_solve: basis tables of problem " + std::to_string(p) + " are malformed");
-  for (int p = 0; p < nprob; p++) {
-    const necgpu_structure& s = structs[p];
-    const int64_t n = s.n, o = seg_off[p];
-    const double* src[8] = {s.x, s.y, s.z, s.length, s.radius, s.cab, s.sab, s.salp};
-    for (int a = 0; a < 8; a++) std::copy(src[a], src[a] + n, seg.begin() + a * T + o);
-    if (s.ek_ind1 && s.ek_ind2) {
-      std::copy(s.ek_ind1, s.ek_ind1 + n, ind.begin() + o);
-      std::copy(s.ek_ind2, s.ek_ind2 + n, ind.begin() + T + o);
+  // basis tables checked and counted on the host cores
+  std::vector<int64_t> eoff(nprob + 1, 0);
+  std::vector<int> seg_prob(T), cols(nprob), bad(nprob, 0);
+  const int workers = std::max(1, std::min<int>({(int)std::thread::hardware_concurrency(), 16, nprob / 16}));
+  parallel_chunks(nprob, workers, [&](int, int64_t p0, int64_t p1) {
+    for (int64_t p = p0; p < p1; p++) {
+      const necgpu_structure& s = structs[p];
+      const int64_t n = s.n;
+      const int32_t* tp = s.trio_ptr;
+      bool ok = tp[0] == 0;
+      for (int64_t j = 0; ok && j < n; j++) ok = tp[j + 1] >= tp[j];
+      for (int64_t k = 0; ok && k < tp[n]; k++) ok = s.trio_basis[k] >= 0 && s.trio_basis[k] < n;
+      bad[p] = !ok;
+      if (!ok) continue;
+      cols[p] = fill_block_cols(n, tp[n]);
+      std::fill(seg_prob.begin() + seg_off[p], seg_prob.begin() + seg_off[p + 1], (int)p);
     }
-    for (int64_t j = 0; j < n; j++) seg_prob[o + j] = p;
-    const int32_t* tp = s.trio_ptr;
-    const FillLists& FL = FLs[p];
-    bp_off[p] = (int64_t)bp_pool.size();
-    src_off[p] = (int64_t)src_pool.size();
-    cp_off[p] = (int64_t)cp_pool.size();
-    el_off[p] = (int64_t)eloc_pool.size();
-    ecf_off[p] = (int64_t)ecoef_pool.size();
-    ne_p[p] = tp[n];
-    bp_pool.insert(bp_pool.end(), FL.blk_ptr.begin(), FL.blk_ptr.end());
-    src_pool.insert(src_pool.end(), FL.src.begin(), FL.src.end());
-    cp_pool.insert(cp_pool.end(), FL.col_ptr.begin(), FL.col_ptr.end());
-    eloc_pool.insert(eloc_pool.end(), FL.eloc.begin(), FL.eloc.end());
-    ecoef_pool.insert(ecoef_pool.end(), FL.ecoef.begin(), FL.ecoef.end());
-    const CoefLists& CL = CLs[p];
-    const int64_t nt = tp[n], cbase = (int64_t)cbasis_pool.size();
-    for (int64_t j = 0; j < n; j++) cptr_g[o + j] = (int32_t)(cbase + CL.cptr[j]);
-    cbasis_pool.insert(cbasis_pool.end(), CL.cbasis.begin(), CL.cbasis.begin() + nt);
-    ca_pool.insert(ca_pool.end(), CL.ccoef.begin(), CL.ccoef.begin() + nt);
-    cb_pool.insert(cb_pool.end(), CL.ccoef.begin() + nt, CL.ccoef.begin() + 2 * nt);
-    cc_pool.insert(cc_pool.end(), CL.ccoef.begin() + 2 * nt, CL.ccoef.begin() + 3 * nt);
+  });
+  for (int p = 0; p < nprob; p++) {
+    if (bad[p]) return fail(e, NECGPU_ERR_ARG, "batch_solve: basis tables of problem " + std::to_string(p) + " are malformed");
+    eoff[p + 1] = eoff[p] + structs[p].trio_ptr[structs[p].n];
   }
-  cptr_g[T] = (int32_t)cbasis_pool.size();
-  if (cbasis_pool.empty()) cbasis_pool.push_back(0);
-  for (auto* v : {&ca_pool, &cb_pool, &cc_pool})
-    if (v->empty()) v->push_back(0.0);
+  const int64_t E = eoff[nprob];
+  if (E > std::numeric_limits<int32_t>::max()) return fail(e, NECGPU_ERR_ARG, "batch_solve: too many basis entries");
   // device pools (stream-ordered; freed at the end of the call)
-  double *d_seg = nullptr, *d_ecoef = nullptr, *d_ca = nullptr, *d_cb = nullptr, *d_cc = nullptr, *d_abc = nullptr,
-         *d_res = nullptr;
-  int32_t *d_ind = nullptr, *d_bp = nullptr, *d_src = nullptr, *d_cp = nullptr, *d_el = nullptr, *d_cptr = nullptr,
-          *d_cbasis = nullptr;
+  double *d_seg = nullptr, *d_tabc = nullptr, *d_eabc = nullptr, *d_cabc = nullptr, *d_abc = nullptr, *d_res = nullptr;
+  int32_t *d_ind = nullptr, *d_tptr = nullptr, *d_tbasis = nullptr, *d_lists = nullptr;
+  int64_t* d_eoff = nullptr;
+  int* d_cols = nullptr;
   double2 *d_Z64 = nullptr, *d_b = nullptr, *d_x = nullptr, *d_cur = nullptr, *d_eth = nullptr, *d_eph = nullptr,
           *d_dirs = nullptr;
   float2* d_Z32 = nullptr;
@@ -3462,35 +3481,40 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
   FillArgs* d_args = nullptr;
   int4* d_items = nullptr;
   auto release = [&]() {
-    dfree(e, d_seg), dfree(e, d_ecoef), dfree(e, d_ca), dfree(e, d_cb), dfree(e, d_cc), dfree(e, d_abc);
-    dfree(e, d_res), dfree(e, d_ind), dfree(e, d_bp), dfree(e, d_src), dfree(e, d_cp), dfree(e, d_cptr);
-    dfree(e, d_cbasis), dfree(e, d_el), dfree(e, d_Z64), dfree(e, d_b), dfree(e, d_x), dfree(e, d_cur);
+    dfree(e, d_seg), dfree(e, d_tabc), dfree(e, d_eabc), dfree(e, d_cabc), dfree(e, d_abc), dfree(e, d_res);
+    dfree(e, d_ind), dfree(e, d_tptr), dfree(e, d_tbasis), dfree(e, d_lists), dfree(e, d_eoff), dfree(e, d_cols);
+    dfree(e, d_Z64), dfree(e, d_b), dfree(e, d_x), dfree(e, d_cur);
     dfree(e, d_eth), dfree(e, d_eph), dfree(e, d_dirs), dfree(e, d_Z32), dfree(e, d_perm), dfree(e, d_segp);
     dfree(e, d_order), dfree(e, d_next), dfree(e, d_st), dfree(e, d_probs), dfree(e, d_args), dfree(e, d_items);
   };
   int rc = 0;
   do {
-    if ((rc = upload(e, d_seg, seg.data(), seg.size()))) break;
-    if ((rc = upload(e, d_ind, ind.data(), ind.size()))) break;
-    if ((rc = upload(e, d_bp, bp_pool.data(), bp_pool.size()))) break;
-    if ((rc = upload(e, d_src, src_pool.data(), src_pool.size()))) break;
-    if ((rc = upload(e, d_cp, cp_pool.data(), cp_pool.size()))) break;
-    if ((rc = upload(e, d_el, eloc_pool.data(), eloc_pool.size()))) break;
-    if ((rc = upload(e, d_ecoef, ecoef_pool.data(), ecoef_pool.size()))) break;
-    if ((rc = upload(e, d_cptr, cptr_g.data(), cptr_g.size()))) break;
-    if ((rc = upload(e, d_cbasis, cbasis_pool.data(), cbasis_pool.size()))) break;
-    if ((rc = upload(e, d_ca, ca_pool.data(), ca_pool.size()))) break;
-    if ((rc = upload(e, d_cb, cb_pool.data(), cb_pool.size()))) break;
-    if ((rc = upload(e, d_cc, cc_pool.data(), cc_pool.size()))) break;
+    const bool xk = s0.use_exk != 0;
+    const int64_t E1 = std::max<int64_t>(E, 1);
+    if ((rc = dalloc(e, d_seg, 8 * (size_t)T))) break;
+    if (xk && (rc = dalloc(e, d_ind, 2 * (size_t)T))) break;
+    if ((rc = dalloc(e, d_tptr, (size_t)(T + nprob)))) break;
+    if ((rc = dalloc(e, d_tbasis, (size_t)E1))) break;
+    if ((rc = dalloc(e, d_tabc, 3 * (size_t)E1))) break;
+    if ((rc = dalloc(e, d_eabc, 3 * (size_t)E1))) break;
+    if ((rc = dalloc(e, d_cabc, 3 * (size_t)E1))) break;
+    // block pointers | column pointers | sources | entries' places | coefficient pointers | basis
+    const int64_t l_col = (int64_t)nprob * (kBatchBlocks + 1), l_src = l_col + T + nprob, l_loc = l_src + E1,
+                  l_cptr = l_loc + E1, l_cbasis = l_cptr + T + 1;
+    if ((rc = dalloc(e, d_lists, (size_t)(l_cbasis + E1)))) break;
+    if ((rc = upload(e, d_eoff, eoff.data(), eoff.size()))) break;
+    if ((rc = upload(e, d_cols, cols.data(), cols.size()))) break;
+    if ((rc = batch_upload_tables(e, nprob, structs, seg_off, eoff, d_seg, d_ind, d_tptr, d_tbasis, d_tabc, workers)))
+      break;
     if ((rc = upload(e, d_segp, seg_prob.data(), seg_prob.size()))) break;
     if ((rc = upload(e, d_b, reinterpret_cast<const double2*>(rhs), (size_t)T))) break;
     if ((rc = dalloc(e, d_Z64, (size_t)Zt))) break;
     if ((rc = dalloc(e, d_Z32, (size_t)Zt))) break;
     if ((rc = dalloc(e, d_x, (size_t)T))) break;
-    if ((rc = dalloc(e, d_perm, (size_t)T))) break;
     if ((rc = dalloc(e, d_cur, (size_t)T))) break;
     if ((rc = dalloc(e, d_abc, 6 * (size_t)T))) break;
     if ((rc = dalloc(e, d_st, (size_t)nprob))) break;
+    if ((rc = dalloc(e, d_perm, (size_t)T))) break;
     if ((rc = dalloc(e, d_res, (size_t)nprob))) break;
     if ((rc = dalloc(e, d_next, 1))) break;
     // per-problem fill arguments
@@ -3512,16 +3536,16 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
       a.cab = d_seg + 5 * T + o;
       a.sab = d_seg + 6 * T + o;
       a.salp = d_seg + 7 * T + o;
-      a.ind1 = d_ind + o;
-      a.ind2 = d_ind + T + o;
-      a.cols = fill_block_cols(n, s.trio_ptr[n]);
-      a.blk_ptr = d_bp + bp_off[p];
-      a.src = d_src + src_off[p];
-      a.col_ptr = d_cp + cp_off[p];
-      a.eloc = d_el + el_off[p];
-      a.ea = d_ecoef + ecf_off[p];
-      a.eb = a.ea + ne_p[p];
-      a.ec = a.ea + 2 * ne_p[p];
+      a.ind1 = xk ? d_ind + o : nullptr;
+      a.ind2 = xk ? d_ind + T + o : nullptr;
+      a.cols = cols[p];
+      a.blk_ptr = d_lists + (int64_t)p * (kBatchBlocks + 1);
+      a.src = d_lists + l_src + eoff[p];
+      a.col_ptr = d_lists + l_col + o + p;
+      a.eloc = d_lists + l_loc + eoff[p];
+      a.ea = d_eabc + eoff[p];
+      a.eb = a.ea + E1;
+      a.ec = a.ea + 2 * E1;
       a.P.rkh = s.rkh;
       a.P.eta = s.eta;
       a.P.zrati = mk(s.zrati_re, s.zrati_im);
@@ -3532,8 +3556,10 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
       a.Z32 = d_Z32 + z_off[p];
       a.status = e->d_status;
       bp[p] = BatchProblem{(int)n, z_off[p], o};
-      const int S = std::max(FLs[p].smax, 1), rows = std::max(1, std::min(kFillMaxRows, kFillPairs / S));
-      const int nblk = (int)FLs[p].blk_ptr.size() - 1;
+      // a block's sources: all segments where it has all columns, else its own
+      // and the neighbours of its ends (more of them are taken in chunks)
+      const int S = (int)std::min<int64_t>(n, cols[p] + 8), rows = std::max(1, std::min(kFillMaxRows, kFillPairs / S));
+      const int nblk = (int)((n + cols[p] - 1) / cols[p]);
       fsmem = std::max(fsmem, fill_smem(rows, S));
       for (int b = 0; b < nblk; b++)
         for (int64_t r = 0; r < n; r += rows) items.push_back(make_int4(p, (int)r, rows | b << 16, S));
@@ -3547,8 +3573,33 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     if ((rc = upload(e, d_order, order.data(), order.size()))) break;
     CUDA_TRY(cudaMemsetAsync(e->d_status, 0, 4 * sizeof(int), e->stream));
     CUDA_TRY(cudaMemsetAsync(d_next, 0, sizeof(int), e->stream));
+    BatchTables bt{};
+    bt.eoff = d_eoff;
+    bt.tptr = d_tptr;
+    bt.tbasis = d_tbasis;
+    bt.ta = d_tabc;
+    bt.tb = d_tabc + E1;
+    bt.tc = d_tabc + 2 * E1;
+    bt.cols = d_cols;
+    bt.blk_ptr = d_lists;
+    bt.col_ptr = d_lists + l_col;
+    bt.src = d_lists + l_src;
+    bt.eloc = d_lists + l_loc;
+    bt.ea = d_eabc;
+    bt.eb = d_eabc + E1;
+    bt.ec = d_eabc + 2 * E1;
+    bt.cptr = d_lists + l_cptr;
+    bt.cbasis = d_lists + l_cbasis;
+    bt.ca = d_cabc;
+    bt.cb = d_cabc + E1;
+    bt.cc = d_cabc + 2 * E1;
+    KLAUNCH(NECGPU_K_OTHER, 0.0,
+            batch_tables_kernel<<<(unsigned)nprob, kBatchTableThreads, 0, e->stream>>>(d_probs, bt));
+    {
+      const int32_t last = (int32_t)E;
+      CUDA_TRY(cudaMemcpyAsync(bt.cptr + T, &last, sizeof last, cudaMemcpyHostToDevice, e->stream));
+    }
     // fill
-    const bool xk = s0.use_exk != 0;
     const double pairs = (double)0 + [&] {
       double q = 0;
       for (int p = 0; p < nprob; p++) q += (double)structs[p].n * structs[p].n;
@@ -3584,7 +3635,7 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
                 nprob, d_order, d_probs, d_Z32, d_Z64, d_perm, d_b, d_x, e->refine_tol, d_next, d_st, d_res));
     KLAUNCH(NECGPU_K_OTHER, 0.0,
             batch_coeff_kernel<<<(unsigned)((T + 255) / 256), 256, 0, e->stream>>>(
-                T, d_segp, d_probs, d_cptr, d_cbasis, d_ca, d_cb, d_cc, d_x, d_abc, d_cur));
+                T, d_segp, d_probs, bt.cptr, bt.cbasis, bt.ca, bt.cb, bt.cc, d_x, d_abc, d_cur));
     double* d_gcop = nullptr;
     float* d_gain = nullptr;
     int64_t* d_so = nullptr;
@@ -3641,23 +3692,39 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
       pa.eph = d_eph;
       pa.gcop = d_gcop;
       pa.gain = d_gain;
+      // In ranges of problems, each copied out while the next ones are
+      // computed: results are usually in pageable memory, whose copy blocks
+      // the host (27 MB of gains: 9 ms).  Ranges of 3 MB and up; one range
+      // below twice that.
+      const size_t per = (size_t)ndir * ((gain ? sizeof(float) : 0) + (eth ? 2 * sizeof(double2) : 0));
+      const int nr = (int)std::max<size_t>(1, std::min<size_t>({8, (size_t)nprob, per * nprob / ((size_t)3 << 20)}));
       const int dw = pattern_width(ndir, nprob, e->nsm);
-      const dim3 g((unsigned)((ndir + kPatDirs * dw - 1) / (kPatDirs * dw)), (unsigned)nprob);
-      if (dw == kPatWide)
-        KLAUNCH(NECGPU_K_PATTERN, (double)ndir * T * pa.ksymp,
-                batch_pattern_kernel<kPatWide><<<g, kPatDirs * 32, 0, e->stream>>>(pa));
-      else
-        KLAUNCH(NECGPU_K_PATTERN, (double)ndir * T * pa.ksymp,
-                batch_pattern_kernel<1><<<g, kPatDirs * 32, 0, e->stream>>>(pa));
-      if (eth) {
-        CUDA_TRY(cudaMemcpyAsync(eth, d_eth, (size_t)nprob * ndir * sizeof(double2), cudaMemcpyDeviceToHost,
-                                 e->stream));
-        CUDA_TRY(cudaMemcpyAsync(eph, d_eph, (size_t)nprob * ndir * sizeof(double2), cudaMemcpyDeviceToHost,
-                                 e->stream));
+      if (!e->stream2) CUDA_TRY(cudaStreamCreateWithFlags(&e->stream2, cudaStreamNonBlocking));
+      std::vector<cudaEvent_t> done(nr, nullptr);
+      for (int r = 0; r < nr; r++) {
+        pa.p0 = (int)((int64_t)nprob * r / nr);
+        const int np = (int)((int64_t)nprob * (r + 1) / nr) - pa.p0;
+        const dim3 g((unsigned)((ndir + kPatDirs * dw - 1) / (kPatDirs * dw)), (unsigned)np);
+        const double terms = (double)ndir * (seg_off[pa.p0 + np] - seg_off[pa.p0]) * pa.ksymp;
+        if (dw == kPatWide)
+          KLAUNCH(NECGPU_K_PATTERN, terms, batch_pattern_kernel<kPatWide><<<g, kPatDirs * 32, 0, e->stream>>>(pa));
+        else
+          KLAUNCH(NECGPU_K_PATTERN, terms, batch_pattern_kernel<1><<<g, kPatDirs * 32, 0, e->stream>>>(pa));
+        CUDA_TRY(cudaEventCreateWithFlags(&done[r], cudaEventDisableTiming));
+        CUDA_TRY(cudaEventRecord(done[r], e->stream));
       }
-      if (gain)
-        CUDA_TRY(cudaMemcpyAsync(gain, d_gain, (size_t)nprob * ndir * sizeof(float), cudaMemcpyDeviceToHost,
-                                 e->stream));
+      for (int r = 0; r < nr; r++) {
+        const size_t o = (size_t)((int64_t)nprob * r / nr) * ndir, m = (size_t)((int64_t)nprob * (r + 1) / nr) * ndir - o;
+        CUDA_TRY(cudaStreamWaitEvent(e->stream2, done[r], 0));
+        CUDA_TRY(cudaEventDestroy(done[r]));
+        if (eth) {
+          CUDA_TRY(cudaMemcpyAsync(eth + 2 * o, d_eth + o, m * sizeof(double2), cudaMemcpyDeviceToHost, e->stream2));
+          CUDA_TRY(cudaMemcpyAsync(eph + 2 * o, d_eph + o, m * sizeof(double2), cudaMemcpyDeviceToHost, e->stream2));
+        }
+        if (gain)
+          CUDA_TRY(cudaMemcpyAsync(gain + o, d_gain + o, m * sizeof(float), cudaMemcpyDeviceToHost, e->stream2));
+      }
+      CUDA_TRY(cudaStreamSynchronize(e->stream2));  // before the buffers are freed in the stream's order
     }
     CUDA_TRY(cudaMemcpyAsync(cur, d_cur, (size_t)T * sizeof(double2), cudaMemcpyDeviceToHost, e->stream));
     CUDA_TRY(cudaMemcpyAsync(status, d_st, (size_t)nprob * sizeof(int), cudaMemcpyDeviceToHost, e->stream));

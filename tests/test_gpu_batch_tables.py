@@ -1,0 +1,73 @@
+"""The batched sweep's lists, made on the device from each problem's basis
+tables, and its factorisation: problems at the edges of the fill's column
+blocks (124) and of the LU's panels, a junction whose sources spread over the
+blocks, and all of them in one call, against the single-problem path."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def wire(nb, n, extended=False):
+    ctx = nb.nec_create()
+    assert nb.nec_wire(ctx, 1, n, 0.0, 0.0, -0.02 * n, 0.0, 0.0, 0.02 * n, 1e-3, 1.0, 1.0) == 0
+    assert nb.nec_geometry_complete(ctx, 0) == 0
+    if extended:
+        assert nb.nec_ek_card(ctx, 0) == 0
+    return ctx
+
+
+def star(nb, arms, segs):
+    """`arms` wires from one point: each end segment lies in the bases of all."""
+    ctx = nb.nec_create()
+    for k in range(arms):
+        a = 2 * np.pi * k / arms
+        assert nb.nec_wire(ctx, k + 1, segs, 0.0, 0.0, 0.0, 2 * np.cos(a), 2 * np.sin(a), 0.1 * k, 1e-3, 1.0, 1.0) == 0
+    assert nb.nec_geometry_complete(ctx, 0) == 0
+    return ctx
+
+
+def tables(nb, ctx, feed):
+    from necpp_b200 import batch as B
+    nb.nec_ex_card(ctx, 0, 1, feed + 1, 0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0)
+    p = B.host_problem(ctx, 150.0, feed)
+    nb.nec_delete(ctx)
+    return p
+
+
+def single(nb, problem):
+    from gpu_helpers import Engine
+    e = Engine(nb.lib)
+    e.set_structure(problem[0])
+    e.fill()
+    e.factor(0)
+    x, _ = e.solve(problem[1])
+    e.close()
+    return np.asarray(x)
+
+
+def check(nb, problems):
+    from necpp_b200 import batch as B
+    r = B.sweep(problems)
+    assert np.all(r["status"] == 0), r["status"]
+    for k, p in enumerate(problems):
+        cur = r["cur"][r["offsets"][k]:r["offsets"][k + 1]] / p[4]
+        ref = single(nb, p)
+        # both refined to the FP64 floor; the two matrices are equal
+        assert np.max(np.abs(cur - ref)) <= 1e-9 * np.max(np.abs(ref)), k
+
+
+def test_sizes_in_one_call(nb):
+    sizes = [3, 15, 16, 17, 31, 33, 63, 65, 123, 124, 125, 127, 247, 249, 373, 639, 640]
+    check(nb, [tables(nb, wire(nb, n), n // 2) for n in sizes])
+
+
+@pytest.mark.parametrize("n", [16, 125, 250])
+def test_extended_kernel(nb, n):
+    check(nb, [tables(nb, wire(nb, n, True), n // 2)])
+
+
+@pytest.mark.parametrize("arms,segs", [(3, 5), (12, 11), (24, 9), (20, 30)])
+def test_junctions(nb, arms, segs):
+    # 24 x 9: the junction alone has more than 4 entries a column, one block
+    check(nb, [tables(nb, star(nb, arms, segs), 0)] + [tables(nb, wire(nb, 40), 20)])
