@@ -9,7 +9,7 @@
 //                         single-problem fill_rows
 //   batch_lu_solve_kernel persistent: a CTA takes the next problem (largest
 //                         first) from a counter and does its complex64 LU
-//                         with partial pivoting (32-wide panels in shared
+//                         with partial pivoting (16-wide panels in shared
 //                         memory, register-tiled trailing updates) and the
 //                         solve refined in FP64 against the FP64 matrix
 //   batch_coeff_kernel    basis amplitudes -> a, b, c and currents
@@ -24,20 +24,21 @@
 namespace necb {
 
 constexpr int kBatchThreads = 256;
-constexpr int kBatchNB = 32;      // LU panel width
+constexpr int kBatchNB = 16;      // LU panel width
+constexpr int kBatchTB = 32;      // block of the triangular solves
 constexpr int kBatchMaxN = 640;   // unknowns per problem on the batched path
 constexpr long long kBatchRefineMax = 20;
 
 struct BatchProblem {
   int n;
   int64_t z;  // element offset of the problem's n x n matrices (Z32, Z64)
-  int64_t v;  // element offset of its vectors (rhs, x, perm)
+  int64_t v;  // element offset of its vectors (rhs, x)
 };
 
 // smem layout of batch_lu_solve_kernel (bytes)
 constexpr size_t kBatchPanelBytes = (size_t)kBatchMaxN * (kBatchNB + 1) * sizeof(float2);
 constexpr size_t kBatchUtBytes = (size_t)kBatchNB * (64 + 1) * sizeof(float2);
-constexpr size_t kBatchSmem = kBatchPanelBytes + kBatchUtBytes + 2 * kBatchMaxN * sizeof(double2) + 256;
+constexpr size_t kBatchSmem = kBatchPanelBytes + kBatchUtBytes;
 
 // One CTA per item: x problem, y first row, z rows and column block (in the
 // low and high halves), w sources staged at once.
@@ -164,52 +165,41 @@ __global__ void __launch_bounds__(kBatchTableThreads)
   }
 }
 
-// CTA-wide argmax of key (>= 0 candidates; -1 none), lowest row on ties.
-__device__ __forceinline__ void cta_argmax(float key, int row, float* s_key, int* s_row, int* out_row,
-                                           float* out_key) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const float ok = __shfl_xor_sync(0xffffffffu, key, off);
-    const int orow = __shfl_xor_sync(0xffffffffu, row, off);
-    if (ok > key || (ok == key && orow < row)) {
-      key = ok;
-      row = orow;
-    }
+// Diagonal block j0 of the factored A (n x n, row-major) into D, each
+// diagonal element of an upper block as its reciprocal.
+template <bool LOWER>
+__device__ __forceinline__ void batch_stage_block(const float2* A, int n, int j0, float2 (*D)[kBatchTB + 1]) {
+  for (int e = threadIdx.x; e < kBatchTB * kBatchTB; e += kBatchThreads) {
+    const int r = e / kBatchTB, c = e % kBatchTB;
+    const bool in = j0 + r < n && j0 + c < n;
+    float2 v = in ? A[(int64_t)(j0 + r) * n + j0 + c] : make_float2(0.f, 0.f);
+    if (!LOWER && r == c && in) v = crecip(v);
+    D[r][c] = v;
   }
-  if (lane == 0) {
-    s_key[warp] = key;
-    s_row[warp] = row;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float k = s_key[0];
-    int r = s_row[0];
-    for (int w = 1; w < kBatchThreads / 32; w++)
-      if (s_key[w] > k || (s_key[w] == k && s_row[w] < r)) {
-        k = s_key[w];
-        r = s_row[w];
-      }
-    *out_row = r;
-    *out_key = k;
-  }
-  __syncthreads();
 }
 
-// y <- (LU)^-1 P... : the two triangular solves of the factored A (n x n,
-// row-major) on the complex64 vector y in shared memory, in place.
-__device__ void batch_trsv(const float2* A, int n, float2* y) {
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  constexpr int B = 32;
-  // forward, unit lower
-  for (int j0 = 0; j0 < n; j0 += B) {
-    const int jb = min(B, n - j0);
+// One triangular solve of the factored A on the complex64 vector y in shared
+// memory, in place, in blocks of 32: a warp solves a diagonal block from
+// shared memory, then four lanes per row subtract it from the remaining rows
+// (32-byte pieces of the row) while the next diagonal block is staged.
+template <bool LOWER>
+__device__ void batch_trsv(const float2* A, int n, float2* y, float2 (*D)[kBatchTB][kBatchTB + 1]) {
+  constexpr int B = kBatchTB;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nblk = (n + B - 1) / B;
+  batch_stage_block<LOWER>(A, n, LOWER ? 0 : (nblk - 1) * B, D[0]);
+  __syncthreads();
+  for (int k = 0; k < nblk; k++) {
+    const int j0 = (LOWER ? k : nblk - 1 - k) * B, jb = min(B, n - j0);
     if (warp == 0) {
+      float2(*d)[B + 1] = D[k & 1];
       float2 v = lane < jb ? y[j0 + lane] : make_float2(0.f, 0.f);
-      for (int c = 0; c < jb - 1; c++) {
+#pragma unroll 8
+      for (int s = 0; s < B; s++) {
+        const int c = LOWER ? s : B - 1 - s;
+        const float2 l = d[lane][c];
+        if (!LOWER && lane == c) v = cmul(v, l);
         const float2 yc = make_float2(__shfl_sync(0xffffffffu, v.x, c), __shfl_sync(0xffffffffu, v.y, c));
-        if (lane > c && lane < jb) {
-          const float2 l = A[(int64_t)(j0 + lane) * n + j0 + c];
+        if (LOWER ? lane > c : lane < c) {
           v.x -= l.x * yc.x - l.y * yc.y;
           v.y -= l.x * yc.y + l.y * yc.x;
         }
@@ -217,46 +207,33 @@ __device__ void batch_trsv(const float2* A, int n, float2* y) {
       if (lane < jb) y[j0 + lane] = v;
     }
     __syncthreads();
-    for (int i = j0 + jb + t; i < n; i += kBatchThreads) {
-      const float2* row = A + (int64_t)i * n + j0;
+    if (k + 1 < nblk) batch_stage_block<LOWER>(A, n, LOWER ? j0 + B : j0 - B, D[(k + 1) & 1]);
+    // lower: rows j0 + B .. n - 1 (jb = B there); upper: rows 0 .. j0 - 1
+    const int first = LOWER ? j0 + B : 0, end = LOWER ? n : j0;
+    for (int i0 = first; i0 < end; i0 += kBatchThreads / 4) {
+      const int i = i0 + (t >> 2), c0 = t & 3;
       float sr = 0.f, si = 0.f;
-      for (int c = 0; c < jb; c++) {
-        const float2 l = row[c], yc = y[j0 + c];
-        sr += l.x * yc.x - l.y * yc.y;
-        si += l.x * yc.y + l.y * yc.x;
-      }
-      y[i].x -= sr;
-      y[i].y -= si;
-    }
-    __syncthreads();
-  }
-  // backward, upper
-  for (int j0 = ((n - 1) / B) * B; j0 >= 0; j0 -= B) {
-    const int jb = min(B, n - j0);
-    if (warp == 0) {
-      float2 v = lane < jb ? y[j0 + lane] : make_float2(0.f, 0.f);
-      for (int c = jb - 1; c >= 0; c--) {
-        if (lane == c) v = cdiv(v, A[(int64_t)(j0 + c) * n + j0 + c]);
-        const float2 xc = make_float2(__shfl_sync(0xffffffffu, v.x, c), __shfl_sync(0xffffffffu, v.y, c));
-        if (lane < c) {
-          const float2 u = A[(int64_t)(j0 + lane) * n + j0 + c];
-          v.x -= u.x * xc.x - u.y * xc.y;
-          v.y -= u.x * xc.y + u.y * xc.x;
+      if (i < end) {
+        const float2* row = A + (int64_t)i * n + j0;
+#pragma unroll
+        for (int m = 0; m < B / 4; m++) {
+          const int c = c0 + 4 * m;
+          if (c < jb) {
+            const float2 l = row[c], yc = y[j0 + c];
+            sr += l.x * yc.x - l.y * yc.y;
+            si += l.x * yc.y + l.y * yc.x;
+          }
         }
       }
-      if (lane < jb) y[j0 + lane] = v;
-    }
-    __syncthreads();
-    for (int i = t; i < j0; i += kBatchThreads) {
-      const float2* row = A + (int64_t)i * n + j0;
-      float sr = 0.f, si = 0.f;
-      for (int c = 0; c < jb; c++) {
-        const float2 u = row[c], xc = y[j0 + c];
-        sr += u.x * xc.x - u.y * xc.y;
-        si += u.x * xc.y + u.y * xc.x;
+#pragma unroll
+      for (int off = 1; off < 4; off <<= 1) {
+        sr += __shfl_xor_sync(0xffffffffu, sr, off);
+        si += __shfl_xor_sync(0xffffffffu, si, off);
       }
-      y[i].x -= sr;
-      y[i].y -= si;
+      if (c0 == 0 && i < end) {
+        y[i].x -= sr;
+        y[i].y -= si;
+      }
     }
     __syncthreads();
   }
@@ -266,20 +243,37 @@ __device__ void batch_trsv(const float2* A, int n, float2* y) {
 // pivoting, then x = Z^-1 b refined in FP64 against Z64 until the relative
 // residual reaches tol or stops halving.  status[p]: 0 ok, 1 singular,
 // 2 non-finite, 3 not converged (>1e-6); resid[p]: final relative residual.
-__global__ void __launch_bounds__(kBatchThreads, 1)
+//
+// Bound by the latency of its chain of short phases, not by arithmetic (the
+// 1,024-problem sweep of n = 33..615 is 32 GF): panels of 16 columns keep the
+// shared memory at 99 KB, so that two CTAs share an SM and fill each other's
+// waits; a pivot search reads the candidates that the previous column's
+// update left, two barriers a column; the panel's exchanges are one gather
+// per column, with the block row solved on the way; the triangular solves
+// work from staged blocks.  That sweep: 16.5 -> 6.5 ms against one CTA an SM
+// with 32-wide panels, serial exchanges and solves from global memory.
+__global__ void __launch_bounds__(kBatchThreads, 2)
     batch_lu_solve_kernel(int nprob, const int* order, const BatchProblem* probs, float2* Z32, const double2* Z64,
-                          int* perm_pool, const double2* b_pool, double2* x_pool, double tol, int* next, int* status,
-                          double* resid) {
+                          const double2* b_pool, double2* x_pool, double tol, int* next, int* status, double* resid) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2(*P)[kBatchNB + 1] = reinterpret_cast<float2(*)[kBatchNB + 1]>(smem_raw);
+  constexpr int NB = kBatchNB, W = kBatchThreads / 32;
+  float2(*P)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(smem_raw);
   float2(*Ut)[64 + 1] = reinterpret_cast<float2(*)[64 + 1]>(smem_raw + kBatchPanelBytes);
-  double2* xv = reinterpret_cast<double2*>(smem_raw + kBatchPanelBytes + kBatchUtBytes);
+  // the solve's vectors and blocks take the panel's place
+  double2* xv = reinterpret_cast<double2*>(smem_raw);
   double2* rv = xv + kBatchMaxN;
-  float* s_key = reinterpret_cast<float*>(rv + kBatchMaxN);
-  int* s_row = reinterpret_cast<int*>(s_key + kBatchThreads / 32);
-  __shared__ int s_prob, s_p, s_bad;
-  __shared__ float s_k;
-  __shared__ double s_red[kBatchThreads / 32][2];
+  float2* y = reinterpret_cast<float2*>(rv + kBatchMaxN);
+  float2(*D)[kBatchTB][kBatchTB + 1] = reinterpret_cast<float2(*)[kBatchTB][kBatchTB + 1]>(y + kBatchMaxN);
+  static_assert(2 * kBatchMaxN * sizeof(double2) + kBatchMaxN * sizeof(float2) +
+                        2 * kBatchTB * (kBatchTB + 1) * sizeof(float2) <= kBatchPanelBytes,
+                "the solve's workspace fits the panel's");
+  __shared__ int16_t pm[kBatchMaxN];  // row i of P b is b[pm[i]]
+  __shared__ int16_t mv[kBatchMaxN];  // panel row r was row mv[r] before the panel's exchanges
+  __shared__ int16_t moved[NB];       // rows below the block row whose content changed
+  __shared__ int nmoved, s_prob, s_bad;
+  __shared__ float s_key[2][W];
+  __shared__ int s_row[2][W];
+  __shared__ double s_red[W][2];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (;;) {
     if (t == 0) {
@@ -293,175 +287,205 @@ __global__ void __launch_bounds__(kBatchThreads, 1)
     const BatchProblem pr = probs[p];
     const int n = pr.n;
     float2* A = Z32 + pr.z;
-    int* piv = perm_pool + pr.v;  // pivots during the LU, then the permutation
+    for (int i = t; i < n; i += kBatchThreads) pm[i] = (int16_t)i;
     // ---------------- LU with partial pivoting ----------------
-    for (int k0 = 0; k0 < n; k0 += kBatchNB) {
-      const int kb = min(kBatchNB, n - k0), rows = n - k0;
-      for (int e = t; e < rows * kBatchNB; e += kBatchThreads) {
-        const int r = e / kBatchNB, c = e % kBatchNB;
+    for (int k0 = 0; k0 < n; k0 += NB) {
+      const int kb = min(NB, n - k0), rows = n - k0;
+      for (int e = t; e < rows * NB; e += kBatchThreads) {
+        const int r = e / NB, c = e % NB;
         P[r][c] = c < kb ? A[(int64_t)(k0 + r) * n + k0 + c] : make_float2(0.f, 0.f);
       }
+      for (int r = t; r < rows; r += kBatchThreads) mv[r] = (int16_t)r;
+      if (t == 0) nmoved = 0;
       __syncthreads();
+      float best = -1.f;
+      int brow = 0x7fffffff;
+      auto candidate = [&](const float2 v, int r) {
+        const float a = v.x * v.x + v.y * v.y;
+        if (a > best) {  // rows ascend: the lowest on ties
+          best = a;
+          brow = r;
+        }
+      };
+      for (int r = t; r < rows; r += kBatchThreads) candidate(P[r][0], r);
       for (int c = 0; c < kb; c++) {
-        float best = -1.f;
-        int brow = c;
-        for (int r = c + t; r < rows; r += kBatchThreads) {
-          const float2 v = P[r][c];
-          const float a = v.x * v.x + v.y * v.y;
-          if (a > best) {
-            best = a;
+        // largest |.|^2 of the column, lowest row on ties
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+          const float k = __shfl_xor_sync(0xffffffffu, best, off);
+          const int r = __shfl_xor_sync(0xffffffffu, brow, off);
+          if (k > best || (k == best && r < brow)) {
+            best = k;
             brow = r;
           }
         }
-        cta_argmax(best, brow, s_key, s_row, &s_p, &s_k);
-        int pc = s_p;
-        if (!(s_k > 0.f)) {
-          if (t == 0) s_bad = s_k == 0.f ? 1 : 2;
+        if (lane == 0) {
+          s_key[c & 1][warp] = best;
+          s_row[c & 1][warp] = brow;
+        }
+        __syncthreads();
+        float key = s_key[c & 1][0];
+        int pc = s_row[c & 1][0];
+#pragma unroll
+        for (int w = 1; w < W; w++) {
+          const float k = s_key[c & 1][w];
+          const int r = s_row[c & 1][w];
+          if (k > key || (k == key && r < pc)) {
+            key = k;
+            pc = r;
+          }
+        }
+        if (!(key > 0.f)) {
+          if (t == 0) s_bad = key == 0.f ? 1 : 2;
           pc = c;
         }
-        if (pc != c && t < kBatchNB) {
-          const float2 a = P[c][t];
-          P[c][t] = P[pc][t];
-          P[pc][t] = a;
+        if (pc != c) {
+          if (t < NB) {
+            const float2 a = P[c][t];
+            P[c][t] = P[pc][t];
+            P[pc][t] = a;
+          } else if (t == 32) {
+            const int16_t a = mv[c], b = pm[k0 + c];
+            mv[c] = mv[pc];
+            mv[pc] = a;
+            pm[k0 + c] = pm[k0 + pc];
+            pm[k0 + pc] = b;
+          }
         }
-        if (t == 0) piv[k0 + c] = k0 + pc;
         __syncthreads();
         const float2 pinv = crecip(P[c][c]);
+        best = -1.f;
+        brow = 0x7fffffff;
         for (int r = c + 1 + t; r < rows; r += kBatchThreads) {
           const float2 l = cmul(P[r][c], pinv);
           P[r][c] = l;
-          for (int q = c + 1; q < kb; q++) {
+          if (c + 1 < kb) {
+            const float2 u = P[c][c + 1];
+            float2 v = P[r][c + 1];
+            v.x -= l.x * u.x - l.y * u.y;
+            v.y -= l.x * u.y + l.y * u.x;
+            P[r][c + 1] = v;
+            candidate(v, r);
+          }
+#pragma unroll 4
+          for (int q = c + 2; q < kb; q++) {
             const float2 u = P[c][q];
             P[r][q].x -= l.x * u.x - l.y * u.y;
             P[r][q].y -= l.x * u.y + l.y * u.x;
           }
         }
-        __syncthreads();
-      }
-      for (int e = t; e < rows * kBatchNB; e += kBatchThreads) {
-        const int r = e / kBatchNB, c = e % kBatchNB;
-        if (c < kb) A[(int64_t)(k0 + r) * n + k0 + c] = P[r][c];
-      }
-      // the panel's exchanges, in order, on every column outside it (one
-      // thread per column: no ordering between threads is needed)
-      for (int col = t; col < n; col += kBatchThreads) {
-        if (col >= k0 && col < k0 + kb) continue;
-        for (int c = 0; c < kb; c++) {
-          const int pr2 = piv[k0 + c];
-          if (pr2 != k0 + c) {
-            const float2 a = A[(int64_t)(k0 + c) * n + col];
-            A[(int64_t)(k0 + c) * n + col] = A[(int64_t)pr2 * n + col];
-            A[(int64_t)pr2 * n + col] = a;
-          }
-        }
       }
       __syncthreads();
-      const int c0 = k0 + kb, rest = n - c0;
-      if (rest > 0) {
-        // U12 = L11^-1 A12, one column per thread (L11 in the panel)
-        for (int col = c0 + t; col < n; col += kBatchThreads) {
-          float2 xcol[kBatchNB];
+      for (int r = kb + t; r < rows; r += kBatchThreads)
+        if (mv[r] != r) moved[atomicAdd(&nmoved, 1)] = (int16_t)r;
+      for (int e = t; e < rows * NB; e += kBatchThreads) {
+        const int r = e / NB, c = e % NB;
+        if (c < kb) A[(int64_t)(k0 + r) * n + k0 + c] = P[r][c];
+      }
+      __syncthreads();
+      const int c0 = k0 + kb, rest = n - c0, nm = nmoved;
+      // the panel's exchanges on every column outside it, a column per thread:
+      // the block row gathers its rows, and at most as many rows below take
+      // what was in the block row (an exchange brings a lower row up or moves
+      // one that was there).  Right of the panel the block row is then solved:
+      // U12 = L11^-1 A12.
+      for (int col = t; col < n; col += kBatchThreads) {
+        if (col >= k0 && col < c0) continue;
+        float2 x[NB], d[NB];
+        float2* Ak = A + (int64_t)k0 * n + col;
 #pragma unroll
-          for (int r = 0; r < kBatchNB; r++) xcol[r] = r < kb ? A[(int64_t)(k0 + r) * n + col] : make_float2(0.f, 0.f);
+        for (int r = 0; r < NB; r++) x[r] = r < kb ? Ak[(int64_t)mv[r] * n] : make_float2(0.f, 0.f);
 #pragma unroll
-          for (int r = 0; r < kBatchNB; r++) {
+        for (int i = 0; i < NB; i++)
+          if (i < nm) d[i] = Ak[(int64_t)mv[moved[i]] * n];
 #pragma unroll
-            for (int q = r + 1; q < kBatchNB; q++) {
-              if (q < kb) {
-                const float2 l = P[q][r];
-                xcol[q].x -= l.x * xcol[r].x - l.y * xcol[r].y;
-                xcol[q].y -= l.x * xcol[r].y + l.y * xcol[r].x;
-              }
+        for (int i = 0; i < NB; i++)
+          if (i < nm) Ak[(int64_t)moved[i] * n] = d[i];
+        if (col >= c0) {  // kb = NB here
+#pragma unroll
+          for (int r = 0; r < NB; r++) {
+#pragma unroll
+            for (int q = r + 1; q < NB; q++) {
+              const float2 l = P[q][r];
+              x[q].x -= l.x * x[r].x - l.y * x[r].y;
+              x[q].y -= l.x * x[r].y + l.y * x[r].x;
             }
           }
+        }
 #pragma unroll
-          for (int r = 0; r < kBatchNB; r++)
-            if (r < kb) A[(int64_t)(k0 + r) * n + col] = xcol[r];
+        for (int r = 0; r < NB; r++)
+          if (r < kb) Ak[(int64_t)r * n] = x[r];
+      }
+      __syncthreads();
+      // A22 -= L21 U12 in 64 x 64 tiles; L21 rows come from the panel
+      const int tx = t & 15, ty = t >> 4;
+      for (int tj = 0; tj < rest; tj += 64) {
+        for (int e = t; e < NB * 64; e += kBatchThreads) {
+          const int q = e / 64, cc = e % 64;
+          Ut[q][cc] = tj + cc < rest ? A[(int64_t)(k0 + q) * n + c0 + tj + cc] : make_float2(0.f, 0.f);
         }
         __syncthreads();
-        // A22 -= L21 U12 in 64 x 64 tiles; L21 rows come from the panel
-        const int tx = t & 15, ty = t >> 4;
-        for (int tj = 0; tj < rest; tj += 64) {
-          for (int e = t; e < kBatchNB * 64; e += kBatchThreads) {
-            const int q = e / 64, cc = e % 64;
-            Ut[q][cc] = (q < kb && tj + cc < rest) ? A[(int64_t)(k0 + q) * n + c0 + tj + cc] : make_float2(0.f, 0.f);
+        for (int ti = 0; ti < rest; ti += 64) {
+          float accr[4][4], acci[4][4];
+          float2 old[4][4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const int r = ti + ty + 16 * i;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const int cc = tj + tx + 16 * j;
+              if (r < rest && cc < rest) old[i][j] = A[(int64_t)(c0 + r) * n + c0 + cc];
+              accr[i][j] = 0.f;
+              acci[i][j] = 0.f;
+            }
           }
-          __syncthreads();
-          for (int ti = 0; ti < rest; ti += 64) {
-            float accr[4][4], acci[4][4];
+#pragma unroll 4
+          for (int q = 0; q < NB; q++) {
+            float2 a[4], bq[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = P[NB + min(ti + ty + 16 * i, rest - 1)][q];
+#pragma unroll
+            for (int j = 0; j < 4; j++) bq[j] = Ut[q][tx + 16 * j];
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
               for (int j = 0; j < 4; j++) {
-                accr[i][j] = 0.f;
-                acci[i][j] = 0.f;
+                accr[i][j] += a[i].x * bq[j].x - a[i].y * bq[j].y;
+                acci[i][j] += a[i].x * bq[j].y + a[i].y * bq[j].x;
               }
-            for (int q = 0; q < kb; q++) {
-              float2 a[4], bq[4];
+          }
 #pragma unroll
-              for (int i = 0; i < 4; i++) {
-                const int r = ti + ty + 16 * i;
-                a[i] = r < rest ? P[kb + r][q] : make_float2(0.f, 0.f);
-              }
+          for (int i = 0; i < 4; i++) {
+            const int r = ti + ty + 16 * i;
 #pragma unroll
-              for (int j = 0; j < 4; j++) bq[j] = Ut[q][tx + 16 * j];
-#pragma unroll
-              for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                  accr[i][j] += a[i].x * bq[j].x - a[i].y * bq[j].y;
-                  acci[i][j] += a[i].x * bq[j].y + a[i].y * bq[j].x;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const int r = ti + ty + 16 * i;
-              if (r >= rest) continue;
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                const int cc = tj + tx + 16 * j;
-                if (cc >= rest) continue;
-                float2* dst = A + (int64_t)(c0 + r) * n + c0 + cc;
-                float2 v = *dst;
-                v.x -= accr[i][j];
-                v.y -= acci[i][j];
-                *dst = v;
-              }
+            for (int j = 0; j < 4; j++) {
+              const int cc = tj + tx + 16 * j;
+              if (r < rest && cc < rest)
+                A[(int64_t)(c0 + r) * n + c0 + cc] = make_float2(old[i][j].x - accr[i][j], old[i][j].y - acci[i][j]);
             }
           }
-          __syncthreads();
         }
+        __syncthreads();
       }
-      __syncthreads();
     }
+    __syncthreads();
     // ---------------- refined solve ----------------
     const double2* b = b_pool + pr.v;
     const double2* Z = Z64 + pr.z;
-    float2* y = reinterpret_cast<float2*>(smem_raw);  // the panel area is free now
-    int* pm = reinterpret_cast<int*>(y + kBatchMaxN);
-    if (t == 0) {  // the pivots -> a permutation (row i of P b is b[pm[i]])
-      for (int i = 0; i < n; i++) pm[i] = i;
-      for (int k = 0; k < n; k++) {
-        const int q = piv[k];
-        const int a = pm[k];
-        pm[k] = pm[q];
-        pm[q] = a;
-      }
-    }
-    for (int i = t; i < n; i += kBatchThreads) {
-      xv[i] = make_double2(0.0, 0.0);
-      rv[i] = b[i];
-    }
-    __syncthreads();
-    // ||b||^2
     double bn2 = 0.0;
-    for (int i = t; i < n; i += kBatchThreads) bn2 += b[i].x * b[i].x + b[i].y * b[i].y;
+    for (int i = t; i < n; i += kBatchThreads) {
+      const double2 v = b[i];
+      xv[i] = make_double2(0.0, 0.0);
+      rv[i] = v;
+      bn2 += v.x * v.x + v.y * v.y;
+    }
+    // ||b||^2
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) bn2 += __shfl_xor_sync(0xffffffffu, bn2, off);
     if (lane == 0) s_red[warp][1] = bn2;
     __syncthreads();
     bn2 = 0.0;
-    for (int w = 0; w < kBatchThreads / 32; w++) bn2 += s_red[w][1];
+    for (int w = 0; w < W; w++) bn2 += s_red[w][1];
     const double bn = sqrt(bn2);
     double prev = 1e300, rel = 1.0;
     for (int it = 0; it < kBatchRefineMax; it++) {
@@ -470,37 +494,49 @@ __global__ void __launch_bounds__(kBatchThreads, 1)
         y[i] = make_float2((float)v.x, (float)v.y);
       }
       __syncthreads();
-      batch_trsv(A, n, y);
+      batch_trsv<true>(A, n, y, D);
+      batch_trsv<false>(A, n, y, D);
       for (int i = t; i < n; i += kBatchThreads) {
         xv[i].x += (double)y[i].x;
         xv[i].y += (double)y[i].y;
       }
       __syncthreads();
-      // r = b - Z x (FP64), ||r||^2
+      // r = b - Z x (FP64), ||r||^2: two rows a warp
       double rn2 = 0.0;
-      for (int i = warp; i < n; i += kBatchThreads / 32) {
+      for (int i = 2 * warp; i < n; i += 2 * W) {
         const double2* row = Z + (int64_t)i * n;
-        double sr = 0.0, si = 0.0;
+        const int64_t two = i + 1 < n ? n : 0;
+        double sr = 0.0, si = 0.0, ur = 0.0, ui = 0.0;
+#pragma unroll 4
         for (int j = lane; j < n; j += 32) {
-          const double2 z = row[j], xx = xv[j];
+          const double2 z = row[j], w = row[two + j], xx = xv[j];
           sr += z.x * xx.x - z.y * xx.y;
           si += z.x * xx.y + z.y * xx.x;
+          ur += w.x * xx.x - w.y * xx.y;
+          ui += w.x * xx.y + w.y * xx.x;
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
           sr += __shfl_xor_sync(0xffffffffu, sr, off);
           si += __shfl_xor_sync(0xffffffffu, si, off);
+          ur += __shfl_xor_sync(0xffffffffu, ur, off);
+          ui += __shfl_xor_sync(0xffffffffu, ui, off);
         }
         if (lane == 0) {
           const double2 r = make_double2(b[i].x - sr, b[i].y - si);
           rv[i] = r;
           rn2 += r.x * r.x + r.y * r.y;
+          if (two) {
+            const double2 u = make_double2(b[i + 1].x - ur, b[i + 1].y - ui);
+            rv[i + 1] = u;
+            rn2 += u.x * u.x + u.y * u.y;
+          }
         }
       }
       if (lane == 0) s_red[warp][0] = rn2;
       __syncthreads();
       rn2 = 0.0;
-      for (int w = 0; w < kBatchThreads / 32; w++) rn2 += s_red[w][0];
+      for (int w = 0; w < W; w++) rn2 += s_red[w][0];
       rel = bn > 0 ? sqrt(rn2) / bn : 0.0;
       __syncthreads();
       if (!(rel == rel) || rel <= tol || rel > 0.5 * prev) break;

@@ -3476,7 +3476,7 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
   double2 *d_Z64 = nullptr, *d_b = nullptr, *d_x = nullptr, *d_cur = nullptr, *d_eth = nullptr, *d_eph = nullptr,
           *d_dirs = nullptr;
   float2* d_Z32 = nullptr;
-  int *d_perm = nullptr, *d_segp = nullptr, *d_order = nullptr, *d_next = nullptr, *d_st = nullptr;
+  int *d_segp = nullptr, *d_order = nullptr, *d_next = nullptr, *d_st = nullptr;
   BatchProblem* d_probs = nullptr;
   FillArgs* d_args = nullptr;
   int4* d_items = nullptr;
@@ -3484,7 +3484,7 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     dfree(e, d_seg), dfree(e, d_tabc), dfree(e, d_eabc), dfree(e, d_cabc), dfree(e, d_abc), dfree(e, d_res);
     dfree(e, d_ind), dfree(e, d_tptr), dfree(e, d_tbasis), dfree(e, d_lists), dfree(e, d_eoff), dfree(e, d_cols);
     dfree(e, d_Z64), dfree(e, d_b), dfree(e, d_x), dfree(e, d_cur);
-    dfree(e, d_eth), dfree(e, d_eph), dfree(e, d_dirs), dfree(e, d_Z32), dfree(e, d_perm), dfree(e, d_segp);
+    dfree(e, d_eth), dfree(e, d_eph), dfree(e, d_dirs), dfree(e, d_Z32), dfree(e, d_segp);
     dfree(e, d_order), dfree(e, d_next), dfree(e, d_st), dfree(e, d_probs), dfree(e, d_args), dfree(e, d_items);
   };
   int rc = 0;
@@ -3514,7 +3514,6 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     if ((rc = dalloc(e, d_cur, (size_t)T))) break;
     if ((rc = dalloc(e, d_abc, 6 * (size_t)T))) break;
     if ((rc = dalloc(e, d_st, (size_t)nprob))) break;
-    if ((rc = dalloc(e, d_perm, (size_t)T))) break;
     if ((rc = dalloc(e, d_res, (size_t)nprob))) break;
     if ((rc = dalloc(e, d_next, 1))) break;
     // per-problem fill arguments
@@ -3631,8 +3630,8 @@ int necgpu_batch_solve(necgpu_engine* e, int nprob, const necgpu_structure* stru
     double lu_flops = 0;
     for (int p = 0; p < nprob; p++) lu_flops += 8.0 * std::pow((double)structs[p].n, 3) / 3.0;
     KLAUNCH(NECGPU_K_PANEL, lu_flops,
-            batch_lu_solve_kernel<<<(unsigned)std::min(nprob, e->nsm), kBatchThreads, kBatchSmem, e->stream>>>(
-                nprob, d_order, d_probs, d_Z32, d_Z64, d_perm, d_b, d_x, e->refine_tol, d_next, d_st, d_res));
+            batch_lu_solve_kernel<<<(unsigned)std::min(nprob, 2 * e->nsm), kBatchThreads, kBatchSmem, e->stream>>>(
+                nprob, d_order, d_probs, d_Z32, d_Z64, d_b, d_x, e->refine_tol, d_next, d_st, d_res));
     KLAUNCH(NECGPU_K_OTHER, 0.0,
             batch_coeff_kernel<<<(unsigned)((T + 255) / 256), 256, 0, e->stream>>>(
                 T, d_segp, d_probs, bt.cptr, bt.cbasis, bt.ca, bt.cb, bt.cc, d_x, d_abc, d_cur));
