@@ -962,9 +962,9 @@ int run_lu(necgpu_engine* e, typename cvec<R>::T* M) {
   const int rpc_max = (int)((kSmemLimit - 2 * row_bytes) / row_bytes);
   CUDA_TRY(cudaFuncSetAttribute(panel_kernel<R, kNB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kSmemLimit));
-  const size_t trsm_smem = (size_t)(kNB * kNB + kNB * 32) * sizeof(T);
-  CUDA_TRY(cudaFuncSetAttribute(trsm_kernel<T, kNB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)trsm_smem));
+  static_assert(kNB == kBlk, "trsm8_panel_kernel solves whole blocks");
+  CUDA_TRY(cudaFuncSetAttribute(trsm8_panel_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)trsm8_smem<T>()));
 
   PanelArgs<R> pa{};
   pa.M = M;
@@ -1009,7 +1009,9 @@ int run_lu(necgpu_engine* e, typename cvec<R>::T* M) {
     const int64_t rest = n - k0 - kb;
     if (rest > 0) {
       KLAUNCH(NECGPU_K_TRSM, 4.0 * (double)kb * kb * rest,
-              trsm_kernel<T, kNB><<<(unsigned)((rest + 31) / 32), 256, trsm_smem, e->stream>>>(M, ld, n, k0, kb));
+              trsm8_panel_kernel<T, true><<<(unsigned)((rest + kTrsm8Vec - 1) / kTrsm8Vec), 256,
+                                            (unsigned)trsm8_smem<T>(), e->stream>>>(M, ld, n, k0, k0 + kb,
+                                                                                    (const T*)nullptr));
       bool done = false;
       if constexpr (std::is_same<R, float>::value) {
         if (e->use_tc) {
