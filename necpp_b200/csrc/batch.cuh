@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kFillThreads, GROUND == kGroundNone && !EXK ? 
 // problem's basis tables (the device form of build_fill_lists and
 // build_coef_lists): one CTA per problem.  The host then only gathers the
 // tables: of a sweep of 1,024 problems (n = 33..615) the host's share of the
-// call fell from 35 to 4 ms, for 0.1 ms here, bound by the column scans.
+// call fell from 35 to 4 ms, for 0.37 ms here, bound by the column scans.
 constexpr int kBatchBlocks = (kBatchMaxN + kFillBlock - 1) / kFillBlock;  // most column blocks of a problem
 struct BatchTables {
   // in: per problem its entries' offset and, at v + problem, its n + 1 trio
