@@ -1198,10 +1198,10 @@ int run_lu_blockpiv(necgpu_engine* e, float2* M) {
   // update has finished, before the next U12 rows are formed.
   const int64_t outer = e->outer;
   const bool la = e->lookahead && e->use_tc && e->nsm > 2 * e->lookahead_sms;
-  if (la && !e->stream2) {
-    CUDA_TRY(cudaStreamCreateWithFlags(&e->stream2, cudaStreamNonBlocking));
-    CUDA_TRY(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
-    CUDA_TRY(cudaEventCreateWithFlags(&e->ev_far, cudaEventDisableTiming));
+  if (la) {  // (a batched sweep may have made stream2 for its copies)
+    if (!e->stream2) CUDA_TRY(cudaStreamCreateWithFlags(&e->stream2, cudaStreamNonBlocking));
+    if (!e->ev_fork) CUDA_TRY(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
+    if (!e->ev_far) CUDA_TRY(cudaEventCreateWithFlags(&e->ev_far, cudaEventDisableTiming));
   }
   // the outer row block's U12 in one launch (u12_rows_kernel) when its
   // finished rows fit in shared memory and its 64-row blocks are whole
