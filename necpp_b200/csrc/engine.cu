@@ -70,7 +70,7 @@ struct necgpu_engine {
   unsigned char* d_struct = nullptr;
   size_t struct_cap = 0;
   double* h_pin = nullptr;           // pinned, 16 doubles: status words and small results
-  unsigned char* h_stage = nullptr;  // pinned; read by the copy of the last necgpu_set_structure
+  unsigned char* h_stage = nullptr;  // pinned; read by the last necgpu_set_structure or sweep
   size_t stage_cap = 0;
   double* d_seg = nullptr;  // 8n: x y z s b cab sab salp
   int32_t* d_ind = nullptr; // 2n
